@@ -20,17 +20,19 @@
 //     (bf16 x bf16 -> f32): |sum| <= K 90^2 < 2^24 for K <= 2048, so the
 //     fp32 accumulator is exact.  A's residues are premultiplied by
 //     y_l = (M_L / p_l)^-1 mod p_l, so the sum is y_l A'B' mod p_l; drain
-//     warps reduce it to z_l in [0, p_l), one byte per element, in a
-//     product-residue tile of the CTA.
-//  5. CRT (reconstruction warps of the same kernel, overlapping the next
-//     tile's MMAs): S = sum_l z_l (M_L / p_l) < L M_L is reduced modulo M_L
-//     and centred into (-M_L/2, M_L/2): that is C' exactly; then
-//     C = C' 2^(E_i + E_j - t_a - t_b) with one rounding to FP64.
+//     warps reduce it to its balanced residue z_l, one byte per element, in
+//     a product-residue tile of the CTA.
+//  5. CRT (the same warps, overlapping the next tile's MMAs): S = sum_l z_l
+//     (M_L / p_l) is reduced modulo M_L and centred into (-M_L/2, M_L/2):
+//     that is C' exactly; then C = C' 2^(E_i + E_j - t_a - t_b) with one
+//     rounding to FP64.
 //
 // Against the digit scheme's 36 digit-pair products for float data, this
 // takes 17 modular products for the same 55-bit operand truncation, and its
 // product of the truncated operands is exact (no dropped digit pairs).
 #include "split_common.cuh"
+
+#include <cmath>
 
 namespace caps {
 
@@ -39,8 +41,11 @@ using namespace split;
 namespace {
 
 // moduli, largest first; any prefix is pairwise coprime
-constexpr int MODULI[LMAX] = {181, 180, 179, 173, 169, 167, 163, 161, 157,
-                              151, 149, 139, 137, 131, 127, 121, 113};
+__host__ __device__ constexpr int modulus(int l) {
+    constexpr int m[LMAX] = {181, 180, 179, 173, 169, 167, 163, 161, 157,
+                             151, 149, 139, 137, 131, 127, 121, 113};
+    return m[l];
+}
 
 constexpr int RSTAGE_K = 4;                       // 16-deep K steps per stage (K = 64)
 constexpr int RNSTAGE = 4;
@@ -49,8 +54,10 @@ constexpr int RB_TILE = RTN * TK * 2;             // 8 KiB: 256 x 16 bf16
 constexpr int RSTAGE_A = RSTAGE_K * RA_TILE;      // 16 KiB
 constexpr int RSTAGE_B = RSTAGE_K * RB_TILE;      // 32 KiB
 constexpr int RSTAGE_BYTES = RSTAGE_A + RSTAGE_B; // 48 KiB
-constexpr int RGEMM_THREADS = 448;                // producer, MMA, 8 drain, 4 reconstruction warps
+constexpr int RGEMM_THREADS = 320;                // producer, MMA, 8 drain warps
 constexpr unsigned RSTATUS = 0x100;               // status bits of this kernel: RSTATUS << code
+
+constexpr int NTRIPLE = (LMAX + 2) / 3;
 
 struct CrtTables {
     // the slicer's constants, each in both lanes of a float2 for the packed
@@ -63,14 +70,53 @@ struct CrtTables {
     float cy[LMAX][LMAX][4];       // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
                                    // y_l = (M_L / p_l)^-1 mod p_l
     int lg[LMAX + 1];              // lg[L] = floor(log2 M_L)
-    uint32_t Ml[LMAX][LMAX][4];    // [L-1][l]: limbs of M_L / p_l, least significant first
+    // reconstruction (crt_reconstruct4), per modulus count L; triple t is the
+    // moduli 3t..3t+2 among the first L, P_t their product
+    uint32_t pc[LMAX][LMAX];       // [L-1][l]: P_t / p_l, t = l / 3
+    uint32_t Mt[LMAX][NTRIPLE][4]; // [L-1][t]: limbs of M_L / P_t, least significant first
     uint32_t M[LMAX][4];           // [L-1]: limbs of M_L
-    float m_inv[LMAX];             // [L-1]: 1 / M_L
+    uint32_t Mn[LMAX][4];          // [L-1]: limbs of 2^(32 W) - M_L, W = crt_words(L)
+    uint32_t Z0[LMAX][4];          // [L-1]: limbs of -ZOFF sum_l M_L / p_l modulo M_L
+    float m_inv[LMAX];             // [L-1]: 2^(32 (W - 2)) / M_L
 };
 
 __constant__ CrtTables c_crt;
 
 typedef unsigned __int128 u128;
+
+__host__ __device__ constexpr u128 moduli_product(int first, int last) {  // of the moduli first..last-1
+    u128 m = 1;
+    for (int l = first; l < last; l++) m *= (u128)modulus(l);
+    return m;
+}
+
+// A product residue is kept balanced (|z| <= p / 2 + 1) and stored as the
+// byte b = z + ZOFF, 5..187.
+constexpr int ZOFF = 96, ZMAX = 187;
+
+// 32-bit words that hold S = sum_l b_l M_L / p_l + Z0, Z0 < M_L: 2 up to 8
+// moduli (M_8 < 2^59.4), 3 up to 12 (M_12 < 2^88.3), 4 up to 17 (M_17 < 2^123.1)
+__host__ __device__ constexpr int crt_words(int L) { return L <= 8 ? 2 : L <= 12 ? 3 : 4; }
+constexpr u128 s_bound(int L) {
+    u128 v = moduli_product(0, L);
+    for (int l = 0; l < L; l++) v += (u128)ZMAX * (moduli_product(0, L) / (u128)modulus(l));
+    return v;
+}
+static_assert(s_bound(8) < ((u128)1 << 64) && s_bound(12) < ((u128)1 << 96), "S in 2 words up to L = 8, 3 up to 12");
+static_assert(s_bound(LMAX) / moduli_product(0, LMAX) < 24 && moduli_product(0, LMAX) < ((u128)1 << 123) / 100 * 108,
+              "S < 24 M_17 < 2^128 in 4 words");
+
+// 32-bit limbs of M_L / P_t
+__host__ __device__ constexpr int triple_limbs(int L, int t) {
+    const int last = 3 * t + 3 < L ? 3 * t + 3 : L;
+    u128 v = moduli_product(0, L) / moduli_product(3 * t, last);
+    int n = 0;
+    while (v) {
+        v >>= 32;
+        n++;
+    }
+    return n;
+}
 
 int mod_inverse(int a, int p) {
     a %= p;
@@ -81,7 +127,7 @@ int mod_inverse(int a, int p) {
 
 void build_tables(CrtTables &t) {
     for (int l = 0; l < LMAX; l++) {
-        const int p = MODULI[l];
+        const int p = modulus(l);
         t.p[l] = (float)p;
         t.invp[l] = 1.0f / (float)p;
         long long v = 1;
@@ -97,30 +143,42 @@ void build_tables(CrtTables &t) {
     t.lg[0] = 0;
     for (int L = 1; L <= LMAX; L++) {
         u128 M = 1;
-        for (int l = 0; l < L; l++) M *= (u128)MODULI[l];
+        for (int l = 0; l < L; l++) M *= (u128)modulus(l);
         int lg = 0;
         while ((M >> (lg + 1)) != 0) lg++;
         t.lg[L] = lg;
-        for (int k = 0; k < 4; k++) t.M[L - 1][k] = (uint32_t)(M >> (32 * k));
-        t.m_inv[L - 1] = (float)(1.0 / (double)M);
+        const int W = crt_words(L);
+        for (int k = 0; k < 4; k++) {
+            t.M[L - 1][k] = (uint32_t)(M >> (32 * k));
+            t.Mn[L - 1][k] = k < W ? (uint32_t)(((u128)0 - M) >> (32 * k)) : 0u;
+        }
+        u128 z0 = 0;
+        for (int l = 0; l < L; l++) z0 = (z0 + (u128)(modulus(l) - ZOFF % modulus(l)) * (M / (u128)modulus(l))) % M;
+        for (int k = 0; k < 4; k++) t.Z0[L - 1][k] = (uint32_t)(z0 >> (32 * k));
+        t.m_inv[L - 1] = (float)(ldexp(1.0, 32 * (W - 2)) / (double)M);
+        for (int i = 0; i < NTRIPLE; i++) {
+            const int first = 3 * i, last = first + 3 < L ? first + 3 : L;
+            const u128 P = first < L ? moduli_product(first, last) : 1;
+            for (int l = first; l < last; l++) t.pc[L - 1][l] = (uint32_t)(P / (u128)modulus(l));
+            for (int k = 0; k < 4; k++) t.Mt[L - 1][i][k] = first < L ? (uint32_t)((M / P) >> (32 * k)) : 0u;
+        }
         for (int l = 0; l < LMAX; l++) {
             if (l >= L) {
+                t.pc[L - 1][l] = 0;
                 for (int k = 0; k < 4; k++) {
-                    t.Ml[L - 1][l][k] = 0;
                     t.cy[L - 1][l][k] = 0;
                     t.cy2[L - 1][l][k] = make_float2(0.f, 0.f);
                 }
                 continue;
             }
-            const u128 Ml = M / (u128)MODULI[l];
-            const int p = MODULI[l], y = mod_inverse((int)(Ml % (u128)p), p);
+            const u128 Ml = M / (u128)modulus(l);
+            const int p = modulus(l), y = mod_inverse((int)(Ml % (u128)p), p);
             long long v = y;
             for (int k = 0; k < 4; k++) {
                 t.cy[L - 1][l][k] = (float)(v > p / 2 ? v - p : v);
                 t.cy2[L - 1][l][k] = make_float2(t.cy[L - 1][l][k], t.cy[L - 1][l][k]);
                 v = (v * 16384) % p;
             }
-            for (int k = 0; k < 4; k++) t.Ml[L - 1][l][k] = (uint32_t)(Ml >> (32 * k));
         }
     }
 }
@@ -255,7 +313,7 @@ int crt_moduli_needed(int bits, int K) {
     const int need = 2 * bits + kb + 1;  // as crt_resolve_kernel: K 2^(ta+tb) < M_L / 2
     u128 M = 1;
     for (int L = 1; L <= LMAX; L++) {
-        M *= (u128)MODULI[L - 1];
+        M *= (u128)modulus(L - 1);
         int lg = 0;
         while ((M >> (lg + 1)) != 0) lg++;
         if (lg >= need) return L;
@@ -464,124 +522,322 @@ __device__ __forceinline__ unsigned long long round_scaled_bits(uint64_t hi, uin
     return sign | (((unsigned long long)(ex + 1074) << 52) + mant);
 }
 
-// The same for the common case, without divergent branches: |v| is shifted
-// so that its top bit is bit 127 (top: bits 127..64, rest: 63..0); a normal
-// result's significand is then top >> 11, its round bit top bit 10 and its
-// sticky bits the rest.  Results below the normal range take the general path.
-__device__ __forceinline__ unsigned long long round_scaled_bits_fast(uint64_t hi, uint64_t lo, bool neg, int e) {
-    if ((hi | lo) == 0) return 0;
-    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
-    const int ex = 128 - lz - 53 + e;  // last place of a normal result
-    if (ex < -1074) return round_scaled_bits(hi, lo, neg, e);
-    uint64_t top, rest;
-    if (lz >= 64) {
-        top = lo << (lz - 64);
-        rest = 0;
-    } else if (lz == 0) {
-        top = hi;
-        rest = lo;
-    } else {
-        top = (hi << lz) | (lo >> (64 - lz));
-        rest = lo << lz;
-    }
-    uint64_t mant = top >> 11;
-    const uint64_t rb = (top >> 10) & 1, st = (top & 0x3FFull) | rest;
-    mant += rb & ((st != 0) | (mant & 1));
-    const unsigned long long sign = neg ? 0x8000000000000000ull : 0ull;
-    if (ex > 971) return sign | 0x7FF0000000000000ull;  // |result| >= 2^1024
-    return sign | (((unsigned long long)(ex + 1074) << 52) + mant);
-}
-
 }  // namespace
 
 namespace {
 
-// C' for 4 consecutive rows of one column from their product-residue bytes:
-// zq[l] holds z_l of the 4 rows (byte q = row q).  S = sum_l z_l M_L / p_l
-// (< L M_L < 2^128) is formed in 32-bit limbs with 64-bit column sums; then
-// qe = S / M_L rounded from an fp32 estimate of S (32-bit conversions: the
-// 64-bit ones run on the FP64 pipe), C' = S - qe M_L in 32-bit limbs with a
-// signed carry, and C' is centred into (-M_L/2, M_L/2] (qe may be one off
-// when S / M_L lies near a half-integer).  out[q] = the FP64 encoding of
-// C'_q 2^e[q], or 0 where zero[q].
-__device__ __forceinline__ void crt_reconstruct4(const uint32_t (&zq)[LMAX], int L, const int (&e)[4],
-                                                 const bool (&zero)[4], unsigned long long (&out)[4]) {
-    uint64_t s[4][4];
+// S += sum over the triples t = T.. of w_t (M_L / P_t), w_t = sum of the
+// triple's b_l (P_t / p_l): w_t < 3 * 187 * 181 * 180 < 2^24.2, so a column sum
+// of up to 6 products w_t limb stays below 2^59 and needs no carries until the end.
+template <int L, int T, int W>
+__device__ __forceinline__ void add_triples(const uint32_t (&z)[L], uint64_t (&s)[W]) {
+    if constexpr (3 * T < L) {
+        uint32_t w = z[3 * T] * c_crt.pc[L - 1][3 * T];
+        if constexpr (3 * T + 1 < L) w += z[3 * T + 1] * c_crt.pc[L - 1][3 * T + 1];
+        if constexpr (3 * T + 2 < L) w += z[3 * T + 2] * c_crt.pc[L - 1][3 * T + 2];
+        constexpr int NL = triple_limbs(L, T);
+        static_assert(NL <= W, "M_L / P_t fits the words of S");
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+        for (int k = 0; k < NL; k++) s[k] += (uint64_t)w * c_crt.Mt[L - 1][T][k];
+        add_triples<L, T + 1, W>(z, s);
+    }
+}
+
+// words of sum_k s[k] 2^(32 k) modulo 2^(32 W)
+template <int W>
+__device__ __forceinline__ void carry_words(const uint64_t (&s)[W], uint32_t (&w)[W]) {
+    uint64_t c = s[0];
+    w[0] = (uint32_t)c;
 #pragma unroll
-        for (int k = 0; k < 4; k++) s[q][k] = 0;
+    for (int k = 1; k < W; k++) {
+        c = s[k] + (c >> 32);
+        w[k] = (uint32_t)c;
+    }
+}
+
+// C' 2^e of one entry from its product residues' bytes b_l = z_l + ZOFF.
+// S = sum_l b_l M_L / p_l + Z0 (< 2^(32 W)), congruent to sum_l z_l M_L / p_l;
+// qe = S / M_L rounded, from an fp32 estimate of S's top two words (32-bit
+// conversions: the 64-bit ones run on the FP64 pipe); C' = S - qe M_L, formed
+// as S + qe (2^(32 W) - M_L) modulo 2^(32 W).  qe may be one off when S / M_L
+// lies near a half-integer: a |C'| whose top word reaches that of M_L / 2 is
+// centred exactly.  Then one rounding at the leading bit, on 32-bit words: the
+// words are moved up until the top one is non-zero (for float data it is at
+// once), shifted so that the top bit is bit 31, and the significand, round
+// and sticky bits read off.
+//
+// Bound by its instructions.  Modulus products in triples and L as a template
+// argument (word counts and limbs of M_L / P_t known, constants read from the
+// constant bank) replace L x 4 wide multiply-adds over all 4 limbs whatever L,
+// 64-bit variable shifts and a 128-bit centring per entry.
+template <int L>
+__device__ __forceinline__ unsigned long long crt_reconstruct(const uint32_t (&z)[L], int e) {
+    constexpr int W = crt_words(L);
+    uint64_t s[W];
 #pragma unroll
-    for (int l = 0; l < LMAX; l++) {
-        if (l < L) {
-            const uint32_t *ml = c_crt.Ml[L - 1][l];
+    for (int k = 0; k < W; k++) s[k] = c_crt.Z0[L - 1][k];
+    add_triples<L, 0, W>(z, s);
+    uint32_t w[W];
+    carry_words<W>(s, w);
+    const float sf = fmaf((float)w[W - 1], 4294967296.0f, (float)w[W - 2]);
+    const uint32_t qe = __float_as_uint(fmaf(sf, c_crt.m_inv[L - 1], MAGIC)) - 0x4B400000u;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const uint32_t z = (zq[l] >> (8 * q)) & 255u;
+    for (int k = 0; k < W; k++) s[k] = (uint64_t)qe * c_crt.Mn[L - 1][k] + w[k];
+    carry_words<W>(s, w);
+    bool neg = (w[W - 1] >> 31) != 0u;
+    if (neg) {
+        uint64_t c = 1;
 #pragma unroll
-                for (int k = 0; k < 4; k++) s[q][k] += (uint64_t)z * ml[k];
-            }
+        for (int k = 0; k < W; k++) {
+            c += (uint32_t)~w[k];
+            w[k] = (uint32_t)c;
+            c >>= 32;
         }
     }
-    uint32_t Mw[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) Mw[k] = c_crt.M[L - 1][k];
-    const u128 Mv = ((u128)(((uint64_t)Mw[3] << 32) | Mw[2]) << 64) | (((uint64_t)Mw[1] << 32) | Mw[0]);
-    const u128 Mhalf = Mv >> 1;
-    const float minv = c_crt.m_inv[L - 1];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        uint32_t w[4];
-        uint64_t c = s[q][0];
-        w[0] = (uint32_t)c;
-        c = s[q][1] + (c >> 32);
-        w[1] = (uint32_t)c;
-        c = s[q][2] + (c >> 32);
-        w[2] = (uint32_t)c;
-        c = s[q][3] + (c >> 32);
-        w[3] = (uint32_t)c;
-        const float sf = fmaf((float)w[3], 7.9228162514264337593543950336e28f,
-                              fmaf((float)w[2], 18446744073709551616.0f, fmaf((float)w[1], 4294967296.0f, (float)w[0])));
-        const long long qe = (long long)__float2int_rn(sf * minv);
-        long long t = 0;
-        uint32_t r[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            t += (long long)w[k] - qe * (long long)Mw[k];
-            r[k] = (uint32_t)t;
-            t >>= 32;
-        }
-        const u128 Cr = ((u128)(((uint64_t)r[3] << 32) | r[2]) << 64) | (((uint64_t)r[1] << 32) | r[0]);
-        bool neg = (r[3] >> 31) != 0;
-        u128 mag = neg ? (u128)0 - Cr : Cr;
-        if (mag > Mhalf) {
-            mag = Mv - mag;  // C' -+ M_L has the other sign
+    if constexpr (W == 2) {
+        const uint64_t mag = ((uint64_t)w[1] << 32) | w[0];
+        const uint64_t Mv = ((uint64_t)c_crt.M[L - 1][1] << 32) | c_crt.M[L - 1][0];
+        if (mag > (Mv >> 1)) {  // C' -+ M_L has the other sign
+            w[0] = (uint32_t)(Mv - mag);
+            w[1] = (uint32_t)((Mv - mag) >> 32);
             neg = !neg;
         }
-        out[q] = zero[q] ? 0ull : round_scaled_bits_fast((uint64_t)(mag >> 64), (uint64_t)mag, neg, e[q]);
+    } else if (w[W - 1] >= (c_crt.M[L - 1][W - 1] >> 1)) {  // |C'| perhaps above M_L / 2
+        u128 mag = 0, Mv = 0;
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            mag |= (u128)w[k] << (32 * k);
+            Mv |= (u128)c_crt.M[L - 1][k] << (32 * k);
+        }
+        if (mag > (Mv >> 1)) {
+            mag = Mv - mag;
+            neg = !neg;
+#pragma unroll
+            for (int k = 0; k < W; k++) w[k] = (uint32_t)(mag >> (32 * k));
+        }
+    }
+    // normalise: leading word in w[W - 1]
+    int up = 0;  // words moved up
+#pragma unroll
+    for (int j = 1; j < W; j++) {
+        if (w[W - 1] == 0u) {
+#pragma unroll
+            for (int k = W - 1; k > 0; k--) w[k] = w[k - 1];
+            w[0] = 0u;
+            up++;
+        }
+    }
+    const int lz = __clz((int)w[W - 1]);
+    const int ex = 32 * (W - up) - lz - 53 + e;  // last place of a normal result
+    if (w[W - 1] == 0u) return 0ull;  // a zero row or column too
+    if ((unsigned)(ex + 1074) > 2045u) {
+        // a result below the normal range or above the largest double
+        uint64_t hi = 0, lo = 0;
+        u128 mag = 0;
+#pragma unroll
+        for (int k = 0; k < W; k++) mag |= (u128)w[k] << (32 * k);
+        mag >>= 32 * up;
+        hi = (uint64_t)(mag >> 64);
+        lo = (uint64_t)mag;
+        return round_scaled_bits(hi, lo, neg, e);
+    }
+    const uint32_t th = __funnelshift_l(w[W - 2], w[W - 1], lz);  // bits 63..32 of the normalised value
+    uint32_t tl, rest = 0u;                                       // bits 31..0, and whether any lie below
+    if constexpr (W == 2) {
+        tl = w[0] << lz;
+    } else {
+        tl = __funnelshift_l(w[W - 3], w[W - 2], lz);
+        if constexpr (W == 3) rest = w[0] << lz;
+        else rest = __funnelshift_l(w[0], w[1], lz) | (w[0] << lz);
+    }
+    const uint32_t ml = __funnelshift_r(tl, th, 11), mh = th >> 11;  // 53-bit significand
+    const uint32_t sticky = (tl & 0x3FFu) | rest | (ml & 1u);
+    const uint32_t inc = ((tl >> 10) & 1u) & (sticky ? 1u : 0u);
+    const uint32_t rl = ml + inc;
+    const uint32_t rh = ((uint32_t)(ex + 1074) << 20) + mh + (rl < inc ? 1u : 0u) + (neg ? 0x80000000u : 0u);
+    // a carry out of the significand at the top exponent gives infinity's encoding
+    return ((unsigned long long)rh << 32) | rl;
+}
+
+// A product-residue tile is eight sections, one per drain warp (its 32 rows x
+// 128 columns of the unit), within each modulus's plane: word [step][lane]
+// holds the bytes of columns 4 step .. 4 step + 3 of row `lane` of the section.
+constexpr int ZPLANE_WORDS = TM * RTN / 4, ZSECTION_WORDS = 32 * 128 / 4, ZSTEPS = 32;
+
+// Where a warp's section of a unit goes in C.
+struct Section {
+    const uint32_t *z;  // word [0][lane] of the section in modulus 0's plane
+    const int *eb;      // column exponents from the section's first column on
+    double *C;          // C at the lane's row and the section's first column
+    int e;              // E_i - ta - tb of the lane's row, less both encodings' offsets
+    int cols;           // columns of the section inside the leaf (0 or less: none)
+    bool row;           // the lane's row is inside the leaf
+};
+
+template <int L>
+__device__ __forceinline__ void load_step(const Section &t, int step, uint32_t (&z)[L]) {
+#pragma unroll
+    for (int l = 0; l < L; l++) z[l] = t.z[l * ZPLANE_WORDS + step * 32];
+}
+
+// C of one step: four columns of the lane's row
+template <int L>
+__device__ __forceinline__ void reconstruct_step(const Section &t, int step, const uint32_t (&zq)[L], int64_t M) {
+    double *dst = t.C + (int64_t)(4 * step) * M;
+    // one entry at a time: unrolled by 2 or 4 it ran no faster (two warps per
+    // scheduler cover the latencies) and spilled registers
+#pragma unroll 1
+    for (int q = 0; q < 4 && 4 * step + q < t.cols; q++) {
+        uint32_t z[L];
+#pragma unroll
+        for (int l = 0; l < L; l++) z[l] = (zq[l] >> (8 * q)) & 255u;
+        // C = C' 2^(E_i + E_j - ta - tb); a zero row / column has C' = 0
+        const unsigned long long v = crt_reconstruct<L>(z, t.e + t.eb[4 * step + q]);
+        if (t.row) dst[q * M] = __longlong_as_double((long long)v);
     }
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------- gemm
-// Persistent, one CTA per SM, 448 threads: warp 0 loads (one lane, bulk
+// Persistent, one CTA per SM, 320 threads: warp 0 loads (one lane, bulk
 // copies of pre-tiled planes), warp 1 issues the MMAs (one lane), warps 2..9
-// drain the accumulators, warps 10..13 reconstruct C.
+// drain the accumulators and reconstruct C.
 //
 // A work unit is (leaf, 128-row tile, 256-column tile).  For each modulus in
 // turn it takes Kp / 16 MMAs of 128 x 256 x 16 into one of two TMEM
 // accumulators of 256 columns; they alternate, so the drain of one modulus
 // overlaps the MMAs of the next.  The drain reduces each exact sum modulo p
-// and stores z = (c mod p) y mod p as a byte into the CTA's product-residue
-// tile: [modulus][column][row], two tiles per CTA used in turn.  When a
-// unit's last modulus is drained, the four reconstruction warps turn that
-// tile into C (CRT, one rounding) while the drain moves on to the next unit's
-// moduli in the other tile; mbarriers hand the tiles back and forth.
+// (two values per packed fp32 instruction) and stores the balanced residue as
+// a byte, four columns to a word, into its section of the CTA's
+// product-residue tile; two tiles per CTA are used in turn.
+//
+// A drain warp also reconstructs the section it drained for the unit before:
+// ceil(32 / L) steps of 32 rows x 4 columns after each modulus's drain.  The
+// words of a step are loaded one modulus ahead, so their way through L2 and
+// DRAM (two tiles per CTA exceed L2) runs beside the wait for the accumulator
+// and the drain.  Four warps of their own, one column ahead, were bound by
+// that latency: 4000 clocks per 128 entries at L = 17 and 2900 at L = 6, that
+// is 256 k clocks a unit beside 278 k (K = 2048, L = 17) or 49 k (K = 1024,
+// L = 6) of MMAs.  A section is written and read by one warp, so no barrier
+// hands tiles over.  Measured against those four warps (us a multiply): the
+// n = 16384 integer case (L = 6, leaves of 1024) 139400 -> 102300, n = 6144
+// (leaves of 1536) 7780 -> 7445, one leaf of 448 294 -> 205; n = 16384 with
+// L = 17, leaves of 2048: 107900 -> 102300 or no change, by the GPU (the wait
+// for planes from L2 bounds it: a third of the issuer's time).
 //
 // Units are ordered leaf, row tile, column tile, and the CTAs go through the
 // moduli in step, so the CTAs running at one time share the A and B planes
 // of one modulus of about one leaf (16 MB at m = 2048) through L2.
+struct DrainArgs {
+    const LeafTask *tasks;
+    char *ws;
+    const Geo *g;
+    unsigned char *ztiles;
+    unsigned *status;
+    uint32_t tmem, tfull0, tempty0, wl;
+    int64_t total;
+    int tab;
+};
+
+template <int L>
+__device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
+    constexpr int NC = (ZSTEPS + L - 1) / L;        // reconstruction steps per modulus
+    constexpr int NB = NC * L <= 40 ? NC : 40 / L;  // steps held in registers at a time
+    const Geo &g = *a.g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quarter = warp & 3;         // TMEM lanes 32*quarter.. (rows of the tile)
+    const int colhalf = (warp - 2) >> 2;  // columns 128*colhalf.. of the tile
+    const int64_t M = g.m, tiles = (int64_t)g.mtiles * g.rtiles;
+    uint32_t uc = 0, tc = 0;
+    Section prev;
+    prev.cols = 0;
+    bool have = false;
+    // one more pass than units: the last unit's reconstruction
+    for (int64_t u = blockIdx.x;; u += gridDim.x, tc++) {
+        const bool live = u < a.total;
+        if (!live && !have) return;
+        uint32_t *zt = reinterpret_cast<uint32_t *>(a.ztiles + (size_t)(tc & 1) * ZTILE_BYTES) +
+                       (warp - 2) * ZSECTION_WORDS + lane;
+        uint32_t zr[NB][L], zn[NB][L];
+        auto load = [&](int first, uint32_t (&z)[NB][L]) {
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+                if (4 * (first + b) < prev.cols) load_step<L>(prev, first + b, z[b]);
+        };
+        load(0, zr);
+#pragma unroll 1
+        for (int l = 0; l < L; l++) {
+            const int s0 = l * NC, s1 = s0 + NC < ZSTEPS ? s0 + NC : ZSTEPS;
+            if (s0 + NC < ZSTEPS) load(s0 + NC, zn);  // for the next modulus
+            if (live) {
+                const uint32_t acc = uc & 1;
+                // warp-uniform: tcgen05.ld below is .sync.aligned
+                const bool got = mbar_wait(a.tfull0 + 8 * acc, (uc >> 1) & 1, a.status, RSTATUS << 5, a.wl);
+                if (!__all_sync(0xffffffffu, got)) return;
+                tc_fence_after();
+                const float2 invp = c_crt.invp2[l], np = c_crt.np2[l];
+                uint32_t *out = zt + (size_t)l * ZPLANE_WORDS;
+#pragma unroll 1
+                for (int c4 = 0; c4 < 4; c4++) {
+                    uint32_t v[32];
+                    tmem_ld32(a.tmem + ((uint32_t)(quarter * 32) << 16) + acc * RTN + colhalf * 128 + c4 * 32, v);
+#pragma unroll
+                    for (int w = 0; w < 8; w++) {
+                        // c = sum rA rB = y A'B' mod p (exact, |c| < 2^24; A's
+                        // residues carry y).  q = c fl(1/p) rounded by MAGIC is
+                        // within 1/2 + |c / p| 2^-24 <= 1/2 + 1/p of c / p, so
+                        // z = c - q p has |z| <= p / 2 + 1 and z = c mod p.
+                        uint32_t b[4];
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const float2 c = make_float2(__uint_as_float(v[4 * w + 2 * h]),
+                                                         __uint_as_float(v[4 * w + 2 * h + 1]));
+                            const float2 q = __fadd2_rn(__ffma2_rn(c, invp, make_float2(MAGIC, MAGIC)),
+                                                        make_float2(-MAGIC, -MAGIC));
+                            const float2 z = __fadd2_rn(__ffma2_rn(q, np, c),
+                                                        make_float2(MAGIC + ZOFF, MAGIC + ZOFF));
+                            b[2 * h] = __float_as_uint(z.x);  // low byte: z + ZOFF
+                            b[2 * h + 1] = __float_as_uint(z.y);
+                        }
+                        out[(c4 * 8 + w) * 32] =
+                            __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a.tempty0 + 8 * acc);
+                uc++;
+            }
+#pragma unroll 1
+            for (int s = s0; s < s1; s += NB) {
+                if (s != s0) load(s, zr);
+#pragma unroll
+                for (int b = 0; b < NB; b++)
+                    if (s + b < s1 && 4 * (s + b) < prev.cols) reconstruct_step<L>(prev, s + b, zr[b], M);
+            }
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+#pragma unroll
+                for (int k = 0; k < L; k++) zr[b][k] = zn[b][k];
+        }
+        if (!live) return;
+        __syncwarp();  // the section's words, written by all lanes, are read from here on
+        const int leafi = (int)(u / tiles);
+        const int64_t tile = u % tiles;
+        const int mt = (int)(tile / g.rtiles), rt = (int)(tile % g.rtiles);
+        const char *sc = leaf_scalars(a.ws, g, leafi);
+        const int64_t i = (int64_t)mt * TM + quarter * 32 + lane, j = (int64_t)rt * RTN + colhalf * 128;
+        prev.row = i < M;
+        prev.e = (prev.row ? reinterpret_cast<const int *>(sc + g.off_ea)[i] : 0) - 8192 - a.tab;
+        prev.eb = reinterpret_cast<const int *>(sc + g.off_eb) + j;
+        prev.z = zt;
+        prev.C = a.tasks[leafi].C + i + j * M;
+        prev.cols = (int)(M - j < 128 ? M - j : 128);
+        have = true;
+    }
+}
+
 __global__ void __launch_bounds__(RGEMM_THREADS, 1)
     crt_gemm_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws, Geo g,
                     unsigned *__restrict__ status, int starve) {
@@ -596,12 +852,11 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
     unsigned char *stA = smem;                        // RNSTAGE x RSTAGE_A
     unsigned char *stB = smem + RNSTAGE * RSTAGE_A;   // RNSTAGE x RSTAGE_B
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + RNSTAGE * RSTAGE_BYTES);
-    // bars: full[RNSTAGE], empty[RNSTAGE], tfull[2], tempty[2], final, zfull[2], zempty[2]
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * RNSTAGE + 9);
+    // bars: full[RNSTAGE], empty[RNSTAGE], tfull[2], tempty[2], final
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * RNSTAGE + 5);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + RNSTAGE);
     const uint32_t tfull0 = smem_u32(bars + 2 * RNSTAGE), tempty0 = smem_u32(bars + 2 * RNSTAGE + 2);
     const uint32_t finalb = smem_u32(bars + 2 * RNSTAGE + 4);
-    const uint32_t zfull0 = smem_u32(bars + 2 * RNSTAGE + 5), zempty0 = smem_u32(bars + 2 * RNSTAGE + 7);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -612,8 +867,6 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
         for (int i = 0; i < 2; i++) {
             mbar_init(tfull0 + 8 * i, 1);
             mbar_init(tempty0 + 8 * i, 8);   // the 8 drain warps
-            mbar_init(zfull0 + 8 * i, 8);    // the 8 drain warps
-            mbar_init(zempty0 + 8 * i, 4);   // the 4 reconstruction warps
         }
         mbar_init(finalb, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -704,124 +957,17 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
             umma_commit(finalb);
             mbar_wait(finalb, 0, status, RSTATUS << 4, wl);
         }
-    } else if (warp < 10) {
-        // ------------------------------------------------ drain (8 warps)
-        const int quarter = warp & 3;          // TMEM lanes 32*quarter.. (rows of the tile)
-        const int colhalf = (warp - 2) >> 2;   // columns 128*colhalf.. of the tile
-        const int row = quarter * 32 + lane;
-        uint32_t uc = 0, tc = 0;
-        bool ok = true;
-        for (int64_t u = blockIdx.x; u < total && ok; u += gridDim.x, tc++) {
-            const uint32_t zb = tc & 1;
-            // the reconstruction warps are done with this residue tile
-            const bool free_ = mbar_wait(zempty0 + 8 * zb, ((tc >> 1) & 1) ^ 1, status, RSTATUS << 6, wl);
-            if (!__all_sync(0xffffffffu, free_)) break;
-            unsigned char *zt = ztiles + (size_t)zb * ZTILE_BYTES + row;
-            for (int l = 0; l < L; l++, uc++) {
-                const uint32_t acc = uc & 1;
-                // warp-uniform: tcgen05.ld below is .sync.aligned
-                const bool got = mbar_wait(tfull0 + 8 * acc, (uc >> 1) & 1, status, RSTATUS << 5, wl);
-                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
-                tc_fence_after();
-                const float p = c_crt.p[l], invp = c_crt.invp[l];
-                unsigned char *out = zt + (size_t)l * RTN * TM;
-#pragma unroll 1
-                for (int c4 = 0; c4 < 4; c4++) {
-                    uint32_t v[32];
-                    const int col0 = colhalf * 128 + c4 * 32;
-                    tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + acc * RTN + col0, v);
-#pragma unroll
-                    for (int e = 0; e < 32; e++) {
-                        // c = sum rA rB = y A'B' mod p (exact, |c| < 2^24; A's
-                        // residues carry y).  q = c / p rounded by MAGIC is floor
-                        // or ceil of c / p (|c / p| 2^-24 < 1/2 away), so c - q p
-                        // lies in [-p, p) and one correction gives z = c mod p.
-                        const float c = __uint_as_float(v[e]);
-                        float z = fmaf(-(fmaf(c, invp, MAGIC) - MAGIC), p, c);
-                        z = z < 0.0f ? z + p : z;
-                        out[(size_t)(col0 + e) * TM] = (unsigned char)__float_as_uint(z + MAGIC);  // low byte: z
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
-            }
-            if (!ok) break;
-            // the tile's residues are complete: hand it to the reconstruction warps
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(zfull0 + 8 * zb);
-        }
     } else {
-        // ------------------------------------------------ reconstruction (4 warps)
-        // one warp = one column of the tile at a time, each lane 4 of its rows
-        const int w = warp - 10;
-        const int64_t M = g.m;
-        uint32_t tc = 0;
-        for (int64_t u = blockIdx.x; u < total; u += gridDim.x, tc++) {
-            const uint32_t zb = tc & 1;
-            const bool got = mbar_wait(zfull0 + 8 * zb, (tc >> 1) & 1, status, RSTATUS << 7, wl);
-            if (!__all_sync(0xffffffffu, got)) break;
-            const int leafi = (int)(u / tiles);
-            const int64_t tile = u % tiles;
-            const int mt = (int)(tile / g.rtiles), rt = (int)(tile % g.rtiles);
-            const char *sc = leaf_scalars(ws, g, leafi);
-            const int *eap = reinterpret_cast<const int *>(sc + g.off_ea);
-            const int *ebp = reinterpret_cast<const int *>(sc + g.off_eb);
-            double *C = tasks[leafi].C;
-            const int64_t i0 = (int64_t)mt * TM + lane * 4;
-            int ei[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) ei[q] = i0 + q < M ? eap[i0 + q] : 0;
-            const unsigned char *zt = ztiles + (size_t)zb * ZTILE_BYTES + lane * 4;
-            // the residue words of column col; the next column's are loaded
-            // before this one is reconstructed (the tiles mostly come from
-            // DRAM: two per CTA exceed L2)
-            uint32_t zq[LMAX], zn[LMAX];
-#pragma unroll
-            for (int l = 0; l < LMAX; l++)
-                zq[l] = l < L ? *reinterpret_cast<const uint32_t *>(zt + ((size_t)l * RTN + w) * TM) : 0u;
-#pragma unroll 1
-            for (int col = w; col < RTN; col += 4) {
-                const int next = col + 4 < RTN ? col + 4 : col;
-#pragma unroll
-                for (int l = 0; l < LMAX; l++)
-                    zn[l] = l < L ? *reinterpret_cast<const uint32_t *>(zt + ((size_t)l * RTN + next) * TM) : 0u;
-                const int64_t j = (int64_t)rt * RTN + col;
-                if (j >= M || i0 >= M) {
-#pragma unroll
-                    for (int l = 0; l < LMAX; l++) zq[l] = zn[l];
-                    continue;
-                }
-                const int ej = ebp[j];
-                int e[4];
-                bool zero[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    // C = C' 2^(E_i + E_j - ta - tb); a zero row / column has C' = 0
-                    zero[q] = ei[q] == 0 || ej == 0;
-                    e[q] = (ei[q] - 4096) + (ej - 4096) - h->ta - h->tb;
-                }
-                unsigned long long out[4];
-                crt_reconstruct4(zq, L, e, zero, out);
-                double *dst = C + i0 + j * M;
-                if (i0 + 3 < M && ((uintptr_t)dst & 15) == 0) {
-                    reinterpret_cast<double2 *>(dst)[0] =
-                        make_double2(__longlong_as_double((long long)out[0]), __longlong_as_double((long long)out[1]));
-                    reinterpret_cast<double2 *>(dst)[1] =
-                        make_double2(__longlong_as_double((long long)out[2]), __longlong_as_double((long long)out[3]));
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (i0 + q < M) dst[q] = __longlong_as_double((long long)out[q]);
-                }
-#pragma unroll
-                for (int l = 0; l < LMAX; l++) zq[l] = zn[l];
-            }
-            // this residue tile may be refilled
-            __syncwarp();
-            if (lane == 0) mbar_arrive(zempty0 + 8 * zb);
+        // ------------------------------------------------ drain and reconstruction (8 warps)
+        const DrainArgs a{tasks, ws, &g, ztiles, status, tmem, tfull0, tempty0, wl, total, h->ta + h->tb};
+        switch (L) {
+#define CAPS_DRAIN(n) case n: drain_and_reconstruct<n>(a); break;
+            CAPS_DRAIN(1) CAPS_DRAIN(2) CAPS_DRAIN(3) CAPS_DRAIN(4) CAPS_DRAIN(5) CAPS_DRAIN(6)
+            CAPS_DRAIN(7) CAPS_DRAIN(8) CAPS_DRAIN(9) CAPS_DRAIN(10) CAPS_DRAIN(11) CAPS_DRAIN(12)
+            CAPS_DRAIN(13) CAPS_DRAIN(14) CAPS_DRAIN(15) CAPS_DRAIN(16) CAPS_DRAIN(17)
+#undef CAPS_DRAIN
         }
+        static_assert(LMAX == 17, "every modulus count is covered");
     }
     tc_fence_before();
     __syncthreads();
