@@ -5,17 +5,19 @@
 // and the rectangular subproject's base case localRectMM (rect-class/
 // rectmm.cpp:47-51): A m x k, B k x n, C m x n, column-major, beta = 0.
 //
-// GB300 runs FP64 (DFMA and DMMA alike) at ~1.05 TFLOP/s for the whole GPU,
+// GB300 runs FP64 (DFMA and DMMA alike) at ~1.1 TFLOP/s for the whole GPU,
 // about 1.8 multiply-adds per clock per SM, so this kernel is bound by the
-// DMMA pipe at any sensible tiling; a 16-deep K slab in shared memory keeps
-// operand traffic far below what that pipe can consume.  Each warp owns a
-// 32 x 32 block of C (4 x 4 m8n8k4 tiles); a CTA is a WM x WN grid of warps,
-// one CTA per (32 WM) x (32 WN) tile of one leaf of the batch (blockIdx.z).
-// Three shapes (caps_dmma_tile): 64 x 64 (2 x 2 warps, the default),
-// 32 x 32 (one warp: four times the CTAs, for small leaves) and 128 x 64
-// (4 x 2 warps: half the B traffic per multiply-add).  The autotuner times
-// them per size.  The epilogue applies the task's fold (DmmaFold) of the
-// lean 'd' step that consumes the product.
+// DMMA pipe at any sensible tiling; a 16-deep K slab in shared memory (the
+// next one already in registers) keeps operand traffic far below what that
+// pipe can consume.  What a launch loses is therefore work for padding and
+// SMs with one tile more than the others.  8 x 8 blocks of C outside the leaf
+// and 4-deep steps beyond K are skipped (a 14 x 14 leaf in a 64 x 64 tile took
+// 29 us, 49 of them 97 % of an n = 56 multiply), and the default tile is
+// chosen per launch (pick_tile).  A CTA is a WM x WN grid of warps, each FM x
+// FN blocks of m8n8k4, one CTA per tile of one leaf of the batch (blockIdx.z).
+// Every tile accumulates each entry over k in the same order, so they agree
+// bit for bit.  The epilogue applies the task's fold (DmmaFold) of the lean
+// 'd' step that consumes the product.
 #include "common.cuh"
 
 namespace caps {
@@ -31,10 +33,11 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
 }
 }  // namespace
 
-template <int WM, int WN>
+template <int WM, int WN, int FM, int FN>
 __global__ void __launch_bounds__(32 * WM * WN) dmma_gemm_kernel(const DmmaTask *__restrict__ tasks, int m, int n,
                                                                  int k) {
-    constexpr int BM = 32 * WM, BN = 32 * WN, NT = 32 * WM * WN;
+    constexpr int BM = 8 * FM * WM, BN = 8 * FN * WN, NT = 32 * WM * WN;
+    constexpr int PA = BM * BK / NT, PB = BN * BK / NT;  // operand entries a thread loads per slab
     constexpr int LDA = BM + 8, LDB = BN + 8;  // padded rows (banks)
     __shared__ double As[BK][LDA];  // As[k][i]
     __shared__ double Bs[BK][LDB];  // Bs[k][j]
@@ -43,52 +46,84 @@ __global__ void __launch_bounds__(32 * WM * WN) dmma_gemm_kernel(const DmmaTask 
     const int wr = warp / WN, wc = warp % WN;
     const int64_t i0 = (int64_t)blockIdx.y * BM, j0 = (int64_t)blockIdx.x * BN;
     const int64_t M = m, N = n, K = k;  // A: M x K, B: K x N, C: M x N
+    // this warp's 8 x 8 blocks inside the leaf
+    const int64_t rows = M - i0 - 8 * FM * wr, cols = N - j0 - 8 * FN * wc;
+    const int fm = rows >= 8 * FM ? FM : rows > 0 ? (int)(rows + 7) / 8 : 0;
+    const int fn = cols >= 8 * FN ? FN : cols > 0 ? (int)(cols + 7) / 8 : 0;
+    const bool whole = fm == FM && fn == FN;
 
-    double acc[4][4][2];
+    double acc[FM][FN][2];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < FM; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
+        for (int b = 0; b < FN; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
 
-    for (int64_t k0 = 0; k0 < K; k0 += BK) {
+    double pa[PA], pb[PB];  // the next slab
+    auto fetch = [&](int64_t k0) {
         // A tile: BM rows x 16 k from a column-major source; consecutive
         // threads read consecutive rows of one column
 #pragma unroll
-        for (int p = 0; p < BM * BK / NT; p++) {
+        for (int p = 0; p < PA; p++) {
             const int e = tid + NT * p, row = e % BM, kk = e / BM;
             const int64_t gi = i0 + row, gk = k0 + kk;
-            As[kk][row] = (gi < M && gk < K) ? t.A[gi + gk * M] : 0.0;
+            pa[p] = (gi < M && gk < K) ? t.A[gi + gk * M] : 0.0;
         }
         // B tile: 16 k x BN columns; consecutive threads read the 16 k of one column
 #pragma unroll
-        for (int p = 0; p < BN * BK / NT; p++) {
+        for (int p = 0; p < PB; p++) {
             const int e = tid + NT * p, kk = e % BK, col = e / BK;
             const int64_t gk = k0 + kk, gj = j0 + col;
-            Bs[kk][col] = (gk < K && gj < N) ? t.B[gk + gj * K] : 0.0;
+            pb[p] = (gk < K && gj < N) ? t.B[gk + gj * K] : 0.0;
         }
+    };
+    fetch(0);
+    for (int64_t k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+        for (int p = 0; p < PA; p++) As[(tid + NT * p) / BM][(tid + NT * p) % BM] = pa[p];
+#pragma unroll
+        for (int p = 0; p < PB; p++) Bs[(tid + NT * p) % BK][(tid + NT * p) / BK] = pb[p];
         __syncthreads();
+        if (k0 + BK < K) fetch(k0 + BK);
+        if (whole && k0 + BK <= K) {
 #pragma unroll
-        for (int ks = 0; ks < BK; ks += 4) {
-            double af[4], bf[4];
+            for (int ks = 0; ks < BK; ks += 4) {
+                double af[FM], bf[FN];
 #pragma unroll
-            for (int a = 0; a < 4; a++) af[a] = As[ks + (lane & 3)][32 * wr + 8 * a + (lane >> 2)];
+                for (int a = 0; a < FM; a++) af[a] = As[ks + (lane & 3)][8 * FM * wr + 8 * a + (lane >> 2)];
 #pragma unroll
-            for (int b = 0; b < 4; b++) bf[b] = Bs[ks + (lane & 3)][32 * wc + 8 * b + (lane >> 2)];
+                for (int b = 0; b < FN; b++) bf[b] = Bs[ks + (lane & 3)][8 * FN * wc + 8 * b + (lane >> 2)];
 #pragma unroll
-            for (int a = 0; a < 4; a++)
+                for (int a = 0; a < FM; a++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) dmma_8x8x4(acc[a][b], af[a], bf[b]);
+                    for (int b = 0; b < FN; b++) dmma_8x8x4(acc[a][b], af[a], bf[b]);
+            }
+        } else {
+            const int kend = K - k0 < BK ? (int)(K - k0) : BK;
+#pragma unroll 1
+            for (int ks = 0; ks < kend; ks += 4) {
+                double bf[FN];
+#pragma unroll
+                for (int b = 0; b < FN; b++) bf[b] = Bs[ks + (lane & 3)][8 * FN * wc + 8 * b + (lane >> 2)];
+#pragma unroll
+                for (int a = 0; a < FM; a++) {
+                    if (a >= fm) break;  // warp-uniform, as below
+                    const double af = As[ks + (lane & 3)][8 * FM * wr + 8 * a + (lane >> 2)];
+#pragma unroll
+                    for (int b = 0; b < FN; b++)
+                        if (b < fn) dmma_8x8x4(acc[a][b], af, bf[b]);
+                }
+            }
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < FM; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++)
+        for (int b = 0; b < FN; b++)
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const int64_t gi = i0 + 32 * wr + 8 * a + (lane >> 2);
-                const int64_t gj = j0 + 32 * wc + 8 * b + 2 * (lane & 3) + e;
+                const int64_t gi = i0 + 8 * FM * wr + 8 * a + (lane >> 2);
+                const int64_t gj = j0 + 8 * FN * wc + 8 * b + 2 * (lane & 3) + e;
                 if (gi >= M || gj >= N) continue;
                 const int64_t x = gi + gj * M;
                 const double p = acc[a][b][e];
@@ -113,16 +148,43 @@ __global__ void __launch_bounds__(32 * WM * WN) dmma_gemm_kernel(const DmmaTask 
             }
 }
 
-template <int WM, int WN>
+template <int WM, int WN, int FM, int FN>
 static cudaError_t launch_dmma_shape(const DmmaTask *tasks_dev, int count, int m, int n, int k, cudaStream_t stream) {
-    const unsigned rows = (unsigned)((m + 32 * WM - 1) / (32 * WM)), cols = (unsigned)((n + 32 * WN - 1) / (32 * WN));
+    constexpr int BM = 8 * FM * WM, BN = 8 * FN * WN;
+    const unsigned rows = (unsigned)((m + BM - 1) / BM), cols = (unsigned)((n + BN - 1) / BN);
     for (int base = 0; base < count; base += 65535) {
         const int c = count - base < 65535 ? count - base : 65535;
         dim3 grid(cols, rows, (unsigned)c);
-        dmma_gemm_kernel<WM, WN><<<grid, 32 * WM * WN, 0, stream>>>(tasks_dev + base, m, n, k);
+        dmma_gemm_kernel<WM, WN, FM, FN><<<grid, 32 * WM * WN, 0, stream>>>(tasks_dev + base, m, n, k);
         count_launch();
     }
     return cudaGetLastError();
+}
+
+// The square tile side whose busiest SM has the least to do.  The CTAs of an
+// SM share its one DMMA pipe, so a launch takes as long as the SM with the
+// most tile area: a leaf of 1024 is 256 tiles of 64 on 152 SMs, 2 on the
+// busiest and 1.7 on average; of 32, 1024 tiles, 7 and 6.7.  Smaller tiles read their
+// operands more often and synchronise more per multiply-add, which costs a
+// little where the SM has few of them to overlap.  us a multiply, 64 always ->
+// picked: n = 4096 'dd' (leaves of 1024) 121390 -> 97350 (93100 at the pipe's
+// rate), 4096 x 2048 x 3072 48910 -> 46980, n = 56 'dd' 1471 -> 437 (with the
+// skipped padding).
+static int pick_tile(int count, int m, int n) {
+    const int sides[3] = {64, 32, 16};
+    const double cost[3] = {1.0, 1.01, 1.04};
+    int best = 64;
+    double best_t = 0.0;
+    for (int i = 0; i < 3; i++) {
+        const int64_t t = sides[i];
+        const int64_t ctas = ((m + t - 1) / t) * ((n + t - 1) / t) * (int64_t)count;
+        const double busiest = (double)((ctas + 151) / 152) * (double)(t * t) * cost[i];
+        if (i == 0 || busiest < best_t) {
+            best = sides[i];
+            best_t = busiest;
+        }
+    }
+    return best;
 }
 
 void dmma_tile_shape(int tile, int *rows, int *cols) {
@@ -137,9 +199,13 @@ cudaError_t launch_dmma_rect(const DmmaTask *tasks_dev, int count, int m, int n,
                              int tile) {
     if (count <= 0 || m <= 0 || n <= 0) return cudaSuccess;
     switch (tile) {
-        case DMMA_TILE_32x32: return launch_dmma_shape<1, 1>(tasks_dev, count, m, n, k, stream);
-        case DMMA_TILE_128x64: return launch_dmma_shape<4, 2>(tasks_dev, count, m, n, k, stream);
-        default: return launch_dmma_shape<2, 2>(tasks_dev, count, m, n, k, stream);
+        case DMMA_TILE_32x32: return launch_dmma_shape<2, 2, 2, 2>(tasks_dev, count, m, n, k, stream);
+        case DMMA_TILE_128x64: return launch_dmma_shape<4, 2, 4, 4>(tasks_dev, count, m, n, k, stream);
+    }
+    switch (pick_tile(count, m, n)) {
+        case 16: return launch_dmma_shape<2, 2, 1, 1>(tasks_dev, count, m, n, k, stream);
+        case 32: return launch_dmma_shape<2, 2, 2, 2>(tasks_dev, count, m, n, k, stream);
+        default: return launch_dmma_shape<2, 2, 4, 4>(tasks_dev, count, m, n, k, stream);
     }
 }
 

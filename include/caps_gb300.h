@@ -96,8 +96,9 @@ typedef struct caps_options {
 
 /* CTA tiles of the plain form's DMMA base case. */
 typedef enum caps_plain_tile {
-    CAPS_TILE_64x64 = 0,   /* default */
-    CAPS_TILE_32x32 = 1,   /* one warp per CTA: four times the CTAs, for small leaves */
+    CAPS_TILE_64x64 = 0,   /* default: 64 x 64, or 32 x 32 or 16 x 16 for launches whose 64 x 64
+                              tiles spread unevenly over the SMs (the same bits) */
+    CAPS_TILE_32x32 = 1,   /* four warps of 16 x 16: four times the CTAs */
     CAPS_TILE_128x64 = 2   /* eight warps: half the B traffic per multiply-add */
 } caps_plain_tile;
 
