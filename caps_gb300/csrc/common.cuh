@@ -136,9 +136,10 @@ cudaError_t launch_dmma_gemm(const DmmaTask *tasks_dev, int count, int m, cudaSt
 cudaError_t launch_dmma_rect(const DmmaTask *tasks_dev, int count, int m, int n, int k, cudaStream_t stream,
                              int tile = DMMA_TILE_64x64);
 
-// Split form.  Two schemes share one launch sequence; the kernels agree on
-// the scheme through the launch group's header, written on the device after
-// the exponent scan (no host round trip):
+// Split form.  Two schemes share one launch sequence (scan, slice, GEMM); the
+// leaf size and the options choose the scheme, and the data the digits or
+// moduli, which the scan leaves in the launch group's header on the device
+// (no host round trip):
 //   digits   -- balanced base-128 digit slices, digit-pair products
 //               (kernels_split.cu);
 //   residues -- residues modulo up to 17 small coprime moduli, one product per
@@ -156,10 +157,11 @@ constexpr int RESIDUE_KMAX = 2048;  // residue scheme: largest leaf K (K 90^2 < 
 // Moduli the residue scheme takes for operands of `bits` bits at inner
 // dimension K (0 if more than it has).
 int crt_moduli_needed(int bits, int K);
-// Computes per-row / per-column scale exponents and the needed digit count.
+int crt_product_bits(int L);  // floor(log2) of the product of the first L moduli
+// Per-row / per-column scale exponents, the digit or modulus count.
 cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
                              cudaStream_t stream);
-// Exponents, the scheme choice, and the operand slices (digit or residue planes).
+// The operand slices (digit or residue planes).
 cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, SplitParams p,
                               void *workspace, cudaStream_t stream);
 // Sets the GEMM kernels' attributes and constant tables (once per device);
@@ -178,7 +180,6 @@ void set_debug_starve(int count);
 
 // kernels_crt.cu, called by the launchers above
 cudaError_t crt_prepare();
-cudaError_t launch_crt_resolve(int count, int m, SplitParams p, void *workspace, cudaStream_t stream);
 cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
                              cudaStream_t stream);
 cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,

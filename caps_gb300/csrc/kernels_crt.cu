@@ -10,9 +10,8 @@
 //     min(bits needed over the launch group, 55, the cap SplitParams.bits);
 //     A'_ik = round(a_ik 2^(t_a - E_i)), B'_kj = round(b_kj 2^(t_b - E_j)),
 //     |A'| <= 2^t_a, |B'| <= 2^t_b, exact when the data needs <= t bits.
-//  2. resolve: the fewest moduli L whose product M_L exceeds
-//     2 * K * 2^(t_a + t_b) (so C' = A'B' is fixed by its residues), and the
-//     scheme: residues wherever they fit (K <= 2048), digits otherwise.
+//  2. at the scan's end: the fewest moduli L whose product M_L exceeds
+//     2 * K * 2^(t_a + t_b) (so C' = A'B' is fixed by its residues).
 //  3. slice:   residues of A', B' modulo the pairwise coprime moduli
 //     p_l in {181, 180, 179, 173, ...} (balanced, |r| <= 90, exact in bf16),
 //     written as pre-tiled UMMA canonical K-major planes like the digits.
@@ -69,7 +68,6 @@ struct CrtTables {
     float c[LMAX][3];              // balanced 2^(14k) mod p_l, k = 1..3
     float cy[LMAX][LMAX][4];       // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
                                    // y_l = (M_L / p_l)^-1 mod p_l
-    int lg[LMAX + 1];              // lg[L] = floor(log2 M_L)
     // reconstruction (crt_reconstruct4), per modulus count L; triple t is the
     // moduli 3t..3t+2 among the first L, P_t their product
     uint32_t pc[LMAX][LMAX];       // [L-1][l]: P_t / p_l, t = l / 3
@@ -140,13 +138,9 @@ void build_tables(CrtTables &t) {
         t.np2[l] = make_float2(-(float)p, -(float)p);
         t.invp2[l] = make_float2(t.invp[l], t.invp[l]);
     }
-    t.lg[0] = 0;
     for (int L = 1; L <= LMAX; L++) {
         u128 M = 1;
         for (int l = 0; l < L; l++) M *= (u128)modulus(l);
-        int lg = 0;
-        while ((M >> (lg + 1)) != 0) lg++;
-        t.lg[L] = lg;
         const int W = crt_words(L);
         for (int k = 0; k < 4; k++) {
             t.M[L - 1][k] = (uint32_t)(M >> (32 * k));
@@ -306,52 +300,20 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 
 }  // namespace
 
+int crt_product_bits(int L) {
+    const u128 M = moduli_product(0, L);
+    int lg = 0;
+    while ((M >> (lg + 1)) != 0) lg++;
+    return lg;
+}
+
 int crt_moduli_needed(int bits, int K) {
     const int Kp = (K + TK - 1) / TK * TK;
     int kb = 0;
     while ((1 << kb) < Kp) kb++;
-    const int need = 2 * bits + kb + 1;  // as crt_resolve_kernel: K 2^(ta+tb) < M_L / 2
-    u128 M = 1;
-    for (int L = 1; L <= LMAX; L++) {
-        M *= (u128)modulus(L - 1);
-        int lg = 0;
-        while ((M >> (lg + 1)) != 0) lg++;
-        if (lg >= need) return L;
-    }
+    for (int L = 1; L <= LMAX; L++)
+        if (crt_product_bits(L) >= 2 * bits + kb + 1) return L;  // as the scan kernel: K 2^(ta+tb) < M_L / 2
     return 0;
-}
-
-// ---------------------------------------------------------------- resolve
-// One thread: picks the scheme for the launch group from the scan's results
-// and writes it into the header, where every later kernel of the group reads it.
-__global__ void crt_resolve_kernel(char *__restrict__ ws, Geo g, SplitParams p) {
-    if (threadIdx.x != 0) return;
-    SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
-    int s, nd;
-    resolve_sd(h, p, s, nd);
-    h->s_used = s;
-    h->nd_used = nd;
-    const bool forced_digits = p.scheme == SCHEME_DIGITS || (p.scheme == SCHEME_AUTO && p.slices > 0);
-    // operand bits: what the data need, at most 55, at most the cap asked for
-    // (a cap only where the residues run: the digit scheme sets its own cut)
-    const int cap = (p.bits > 0 && p.bits < 55 && !forced_digits) ? p.bits : 55;
-    const int ta = h->bitsA < cap ? h->bitsA : cap, tb = h->bitsB < cap ? h->bitsB : cap;
-    int residues = 0, L = 0;
-    if (g.residues_ok && !forced_digits) {
-        int kb = 0;
-        while ((1 << kb) < g.Kp) kb++;
-        const int need = ta + tb + kb + 1;  // K 2^(ta+tb) < M_L / 2
-        L = 1;
-        while (L <= LMAX && c_crt.lg[L] < need) L++;
-        // wherever the residues fit they are the faster cut, integer data
-        // included: the digit GEMM's per-chunk drain of its diagonal
-        // accumulators costs about as much at one digit as at eight
-        if (L <= LMAX) residues = 1;
-    }
-    h->ta = ta;
-    h->tb = tb;
-    h->moduli = residues ? L : 0;
-    h->residues = residues;
 }
 
 // ---------------------------------------------------------------- slice
@@ -464,12 +426,10 @@ __device__ __forceinline__ void crt_slice_tile(const LeafTask *__restrict__ task
     }
 }
 
-// Grid-stride over (leaf, tile), so that the launch is cheap when the digit
-// scheme runs and this kernel returns at once.  blockIdx.y: A (0) or B (1).
+// Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).
 __global__ void __launch_bounds__(256) crt_slice_kernel(const LeafTask *__restrict__ tasks,
                                                         char *__restrict__ ws, Geo g) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
-    if (!h->residues) return;  // the digit scheme runs
     const int L = h->moduli;
     const int64_t atiles = (int64_t)g.mtiles * g.nks, bhalves = (int64_t)g.rtiles * g.nks * 2;
     const int64_t per = atiles > bhalves ? atiles : bhalves;
@@ -842,7 +802,6 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
     crt_gemm_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws, Geo g,
                     unsigned *__restrict__ status, int starve) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
-    if (!h->residues) return;  // the digit scheme runs
     const int L = h->moduli;
     // starve (test hook): no copies are issued, so nothing is ever in flight
     // and every wait may give up after a short spin
@@ -1000,21 +959,13 @@ cudaError_t crt_prepare() {
     return g_crt_error;
 }
 
-cudaError_t launch_crt_resolve(int count, int m, SplitParams p, void *workspace, cudaStream_t stream) {
-    // the resolve reads the moduli tables: they must be on the device before
-    // the first launch group of the process (returns at once afterwards)
+cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
+                             cudaStream_t stream) {
+    // the moduli tables must be on the device before the first launch group
+    // of the process (returns at once afterwards)
     cudaError_t e = crt_prepare();
     if (e != cudaSuccess) return e;
     Geo g = make_geo(m, count, p.scheme);
-    crt_resolve_kernel<<<1, 32, 0, stream>>>((char *)workspace, g, p);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
-                             cudaStream_t stream) {
-    Geo g = make_geo(m, count, p.scheme);
-    if (!g.residues_ok) return cudaSuccess;
     const int64_t atiles = (int64_t)g.mtiles * g.nks, bhalves = (int64_t)g.rtiles * g.nks * 2;
     const int64_t items = (atiles > bhalves ? atiles : bhalves) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
@@ -1026,7 +977,6 @@ cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitP
 cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
                             unsigned int *status_dev, int num_sms, cudaStream_t stream, int starve) {
     Geo g = make_geo(m, count, p.scheme);
-    if (!g.residues_ok) return cudaSuccess;
     cudaError_t e = crt_prepare();
     if (e != cudaSuccess) return e;
     const int64_t units = (int64_t)g.mtiles * g.rtiles * count;

@@ -6,8 +6,8 @@
 //
 //  1. scan:     per row i of A the exponent bound E (|a_ij| < 2^E) and the
 //               lowest set bit; the same per column of B.
-//  2. finalize: f_i = 55 - E_i; digits needed = ceil((E - lsb + 1) / 7),
-//               max over the launch group (exact for integer-like inputs).
+//  2. (end of the scan) f_i = 55 - E_i; digits needed = ceil((E - lsb + 1)
+//               / 7), max over the launch group (exact for integer-like inputs).
 //  3. slice:    X = round(a * 2^f) (|X| <= 2^55) is cut into balanced base-128
 //               digits d_1..d_8 (|d| <= 64), the s most significant kept.
 //               Digits are int8 values carried EXACTLY in bf16, written as
@@ -62,13 +62,49 @@ size_t split_workspace_bytes(int m, int count, int scheme) {
 
 // ---------------------------------------------------------------- scan
 // Per row of A and per column of B: the largest exponent and the lowest set
-// bit over the leaf.  Work units of up to 64K elements each, the same on both
-// sides: grid.y = 0, a block of A rows (512, a thread per two adjacent rows)
-// times a slab of 128 columns; grid.y = 1, a block of 32 B columns (a warp
-// per 4 columns).  16-byte loads when the leaf's element pairs are 16-byte
-// aligned (m even, base aligned), 8-byte loads otherwise.  grid.x strides
-// over (leaf, unit).
-constexpr int SCAN_AROWS = 512, SCAN_KSLAB = 128, SCAN_BCOLS = 32;
+// bit over the leaf.  grid.y = 0, a block of A rows (512, or the next power of
+// two for shorter leaves; a thread per two adjacent rows, the threads left
+// over taking every KT-th column) times a slab of columns; grid.y = 1, a block
+// of B columns (a warp per column, CW columns each in turn).  16-byte loads
+// when the leaf's element pairs are 16-byte aligned (m even, base aligned),
+// 8-byte loads otherwise.  grid.x strides over (leaf, unit).
+//
+// The block that finishes a leaf side turns its exponents into the digit
+// scheme's f and the group's digit and bit counts, and the block that
+// finishes the last side of the group writes the header: no kernels of their
+// own (they took 7 us of a small multiply's 200).  HBM-bound at full size;
+// a few leaves are bound by the longest unit, so the slab and the columns of a
+// warp shrink until a launch has SCAN_UNITS units a side or the unit is 8
+// columns a thread (1200 units were 7 us slower at 7 leaves of 896, 300 were
+// 8 us slower at 7 leaves of 2500).  Scan and counts together, before -> here:
+// one leaf of 448 52 -> 12 us, 7 leaves of 896 57 -> 32, of 2500 147 -> 148.
+constexpr int SCAN_UNITS = 600;
+
+struct ScanShape {
+    int rt, kt;            // A side: row pairs and column groups of a block (rt * kt = 256)
+    int slab;              // A side: columns of a unit
+    int cw;                // B side: columns per warp
+    int64_t rowblocks, aunits, bunits;
+};
+
+static ScanShape scan_shape(int64_t M, int64_t count) {
+    ScanShape s;
+    s.rt = 16;
+    while (s.rt < 256 && 2 * s.rt < M) s.rt *= 2;
+    s.kt = 256 / s.rt;
+    s.rowblocks = (M + 2 * s.rt - 1) / (2 * s.rt);
+    for (s.slab = 128 * s.kt; s.slab > 8 * s.kt; s.slab /= 2)
+        if (s.rowblocks * ((M + s.slab - 1) / s.slab) * count >= SCAN_UNITS) break;
+    s.aunits = s.rowblocks * ((M + s.slab - 1) / s.slab);
+    for (s.cw = 4; s.cw > 1; s.cw /= 2)
+        if ((M + 8 * s.cw - 1) / (8 * s.cw) * count >= SCAN_UNITS) break;
+    s.bunits = (M + 8 * s.cw - 1) / (8 * s.cw);
+    return s;
+}
+
+struct ModuliBits {
+    int lg[LMAX + 1];  // floor(log2) of the product of the first L moduli
+};
 
 __device__ __forceinline__ void scan_value(double x, int &emax, int &lmin) {
     if (nonzero_bits(x)) {
@@ -79,43 +115,66 @@ __device__ __forceinline__ void scan_value(double x, int &emax, int &lmin) {
     }
 }
 
-__device__ __forceinline__ int64_t scan_units(int64_t M) {
-    const int64_t a = ((M + SCAN_AROWS - 1) / SCAN_AROWS) * ((M + SCAN_KSLAB - 1) / SCAN_KSLAB);
-    const int64_t b = (M + SCAN_BCOLS - 1) / SCAN_BCOLS;
-    return a > b ? a : b;
+// The group's header, once every exponent is in (one thread): digits and
+// diagonals, or operand bits and the fewest moduli whose product M_L holds
+// them, K 2^(ta+tb) < M_L / 2.
+__device__ __forceinline__ void resolve_group(SplitHdr *h, const Geo &g, SplitParams p, bool residues,
+                                              const ModuliBits &mb) {
+    SplitHdr v;
+    v.needed = __ldcg(&h->needed);
+    int s, nd;
+    resolve_sd(&v, p, s, nd);
+    h->s_used = s;
+    h->nd_used = nd;
+    // operand bits: what the data need, at most 55, at most the cap asked for
+    const int cap = (p.bits > 0 && p.bits < 55 && residues) ? p.bits : 55;
+    const int ba = __ldcg(&h->bitsA), bb = __ldcg(&h->bitsB);
+    const int ta = ba < cap ? ba : cap, tb = bb < cap ? bb : cap;
+    int L = 0;
+    if (residues) {
+        int kb = 0;
+        while ((1 << kb) < g.Kp) kb++;
+        L = 1;
+        while (L < LMAX && mb.lg[L] < ta + tb + kb + 1) L++;
+    }
+    h->ta = ta;
+    h->tb = tb;
+    h->moduli = L;
 }
 
 __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restrict__ tasks,
-                                                         char *__restrict__ ws, Geo g) {
-    const int64_t M = g.m, per = scan_units(M), total = per * g.count;
-    const int64_t rowblocks = (M + SCAN_AROWS - 1) / SCAN_AROWS;
-    const int64_t aunits = rowblocks * ((M + SCAN_KSLAB - 1) / SCAN_KSLAB);
-    const int64_t bunits = (M + SCAN_BCOLS - 1) / SCAN_BCOLS;
+                                                         char *__restrict__ ws, Geo g, ScanShape sh, SplitParams p,
+                                                         int residues, ModuliBits mb) {
+    const int side = blockIdx.y;
+    const int64_t M = g.m, units = side ? sh.bunits : sh.aunits, total = units * g.count;
+    SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
+    __shared__ int last;
     for (int64_t it = blockIdx.x; it < total; it += gridDim.x) {
-        const int l = (int)(it / per);
-        const int64_t u = it - (int64_t)l * per;
+        const int l = (int)(it / units);
+        const int64_t u = it - (int64_t)l * units;
         const LeafTask t = tasks[l];
         char *sc = leaf_scalars(ws, g, l);
-        if (blockIdx.y == 0) {
-            if (u >= aunits) continue;
-            const int64_t i0 = (u % rowblocks) * SCAN_AROWS + 2 * threadIdx.x;
-            const int64_t k0 = (u / rowblocks) * SCAN_KSLAB;
-            const int64_t k1 = k0 + SCAN_KSLAB < M ? k0 + SCAN_KSLAB : M;
-            if (i0 >= M) continue;
+        if (side == 0) {
+            const int64_t i0 = (u % sh.rowblocks) * 2 * sh.rt + 2 * (threadIdx.x & (sh.rt - 1));
+            const int64_t slab0 = (u / sh.rowblocks) * sh.slab, k0 = slab0 + threadIdx.x / sh.rt;
+            const int64_t k1 = slab0 + sh.slab < M ? slab0 + sh.slab : M;
+            const int n = i0 < M && k0 < k1 ? (int)(k1 - k0 + sh.kt - 1) / sh.kt : 0;  // columns of this thread
+            const int64_t step = M * sh.kt;
+            const double *col = t.A + i0 + k0 * M;
             int e0 = -100000, l0 = 100000, e1 = -100000, l1 = 100000;
             if ((M & 1) == 0 && ((uintptr_t)t.A & 15) == 0) {  // i0 even, M even: the pair is 16-byte aligned
 #pragma unroll 8
-                for (int64_t k = k0; k < k1; k++) {
-                    const double2 v = __ldg(reinterpret_cast<const double2 *>(t.A + i0 + k * M));
+                for (int k = 0; k < n; k++, col += step) {
+                    const double2 v = __ldg(reinterpret_cast<const double2 *>(col));
                     scan_value(v.x, e0, l0);
                     scan_value(v.y, e1, l1);
                 }
             } else {
                 const bool two = i0 + 1 < M;
 #pragma unroll 8
-                for (int64_t k = k0; k < k1; k++) {
-                    scan_value(__ldg(t.A + i0 + k * M), e0, l0);
-                    if (two) scan_value(__ldg(t.A + i0 + 1 + k * M), e1, l1);
+                for (int k = 0; k < n; k++, col += step) {
+                    scan_value(__ldg(col), e0, l0);
+                    if (two) scan_value(__ldg(col + 1), e1, l1);
                 }
             }
             int *ea = reinterpret_cast<int *>(sc + g.off_ea), *la = reinterpret_cast<int *>(sc + g.off_la);
@@ -128,12 +187,11 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
                 atomicMax(la + i0 + 1, 4096 - l1);
             }
         } else {
-            if (u >= bunits) continue;
             const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
             const bool vec = (M & 1) == 0 && ((uintptr_t)t.B & 15) == 0;
 #pragma unroll 1
-            for (int c = 0; c < 4; c++) {
-                const int64_t j = u * SCAN_BCOLS + w * 4 + c;
+            for (int c = 0; c < sh.cw; c++) {
+                const int64_t j = (u * 8 + w) * sh.cw + c;
                 if (j >= M) break;
                 const double *col = t.B + j * M;
                 int emax = -100000, lmin = 100000;
@@ -148,53 +206,52 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
 #pragma unroll 8
                     for (int64_t k = lane; k < M; k += 32) scan_value(__ldg(col + k), emax, lmin);
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-                    lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, o));
-                }
+                emax = __reduce_max_sync(0xffffffffu, emax);
+                lmin = __reduce_min_sync(0xffffffffu, lmin);
                 if (lane == 0 && emax > -100000) {
                     reinterpret_cast<int *>(sc + g.off_eb)[j] = emax + 4096;
                     reinterpret_cast<int *>(sc + g.off_lb)[j] = 4096 - lmin;
                 }
             }
         }
-    }
-}
-
-// f = 55 - E per row / column (digit scheme); digits needed, and the bits
-// E - lsb + 1 per side (max over the group) for the scheme choice
-__global__ void __launch_bounds__(256) split_finalize_kernel(char *__restrict__ ws, Geo g) {
-    char *leaf = leaf_scalars(ws, g, blockIdx.y);
-    SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
-    int idx = blockIdx.x * 256 + threadIdx.x;
-    int need = 0, bits[2] = {0, 0};
-    if (idx < g.m) {
-        for (int side = 0; side < 2; side++) {
-            int ee = reinterpret_cast<int *>(leaf + (side ? g.off_eb : g.off_ea))[idx];
-            int le = reinterpret_cast<int *>(leaf + (side ? g.off_lb : g.off_la))[idx];
-            int f = 0;
-            if (ee != 0) {
-                int E = ee - 4096, lsb = 4096 - le;
-                f = 55 - E;
-                int b = E - lsb + 1;
-                int s = (b + 6) / 7;
-                need = s > need ? s : need;
-                bits[side] = b;
-            }
-            reinterpret_cast<int *>(leaf + (side ? g.off_fb : g.off_fa))[idx] = f;
+        // This leaf side's units done so far, counted where its first f will
+        // be (zero until then); the block's exponents are visible before it
+        // counts, and all the others' once it was the last to.
+        int *f = reinterpret_cast<int *>(sc + (side ? g.off_fb : g.off_fa));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            last = atomicAdd(f, 1) == (int)units - 1;
+            __threadfence();
         }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        need = max(need, __shfl_xor_sync(0xffffffffu, need, o));
-        bits[0] = max(bits[0], __shfl_xor_sync(0xffffffffu, bits[0], o));
-        bits[1] = max(bits[1], __shfl_xor_sync(0xffffffffu, bits[1], o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (need > 0) atomicMax(&h->needed, need);
-        if (bits[0] > 0) atomicMax(&h->bitsA, bits[0]);
-        if (bits[1] > 0) atomicMax(&h->bitsB, bits[1]);
+        __syncthreads();
+        if (!last) continue;
+        const int *ev = reinterpret_cast<const int *>(sc + (side ? g.off_eb : g.off_ea));
+        const int *lv = reinterpret_cast<const int *>(sc + (side ? g.off_lb : g.off_la));
+        int bits = 0;
+#pragma unroll 8
+        for (int idx = threadIdx.x; idx < g.m; idx += 256) {
+            const int ee = __ldcg(ev + idx), le = __ldcg(lv + idx);
+            int fi = 0;
+            if (ee != 0) {
+                const int E = ee - 4096, lsb = 4096 - le;
+                fi = 55 - E;
+                bits = max(bits, E - lsb + 1);
+            }
+            f[idx] = fi;
+        }
+        bits = __reduce_max_sync(0xffffffffu, bits);
+        if ((threadIdx.x & 31) == 0 && bits > 0) {
+            atomicMax(&h->needed, (bits + 6) / 7);
+            atomicMax(side ? &h->bitsB : &h->bitsA, bits);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            const bool all = atomicAdd(&h->finished, 1) == 2 * g.count - 1;
+            __threadfence();
+            if (all) resolve_group(h, g, p, residues != 0, mb);
+        }
     }
 }
 
@@ -294,12 +351,10 @@ __device__ __forceinline__ void split_slice_tile(const LeafTask *__restrict__ ta
     }
 }
 
-// Grid-stride over (leaf, tile), so that the launch is cheap when the residue
-// scheme runs and this kernel returns at once.  blockIdx.y: A (0) or B (1).
+// Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).
 __global__ void __launch_bounds__(256) split_slice_kernel(const LeafTask *__restrict__ tasks, int m,
                                                           char *__restrict__ ws, Geo g, SplitParams p) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
-    if (h->residues) return;  // the residue scheme runs
     int s, nd;
     resolve_sd(h, p, s, nd);
     const int64_t atiles = (int64_t)g.mtiles * g.nks, btiles2 = ((int64_t)g.ntiles * g.nks + 1) / 2;
@@ -369,7 +424,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NSTAGE + 3);
     MmaTable *mtab = reinterpret_cast<MmaTable *>(bars + 16);
 
-    if (reinterpret_cast<const SplitHdr *>(ws)->residues) return;  // the residue scheme runs
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // starve (test hook): no copies are issued, so nothing is ever in flight
     // and every wait may give up after a short spin
@@ -579,15 +633,15 @@ void split_gemm_prepare() {
 
 cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
                               cudaStream_t stream) {
-    Geo g = make_geo(m, count, p.scheme);
+    const Geo g = make_geo(m, count, p.scheme);
     cudaError_t e = cudaMemsetAsync(workspace, 0, g.dg_base, stream);
     if (e != cudaSuccess) return e;
-    const int64_t M = m;
-    const int64_t aunits = ((M + SCAN_AROWS - 1) / SCAN_AROWS) * ((M + SCAN_KSLAB - 1) / SCAN_KSLAB);
-    const int64_t bunits = (M + SCAN_BCOLS - 1) / SCAN_BCOLS;
-    const int64_t items = (aunits > bunits ? aunits : bunits) * count;
+    const ScanShape sh = scan_shape(m, count);
+    ModuliBits mb;
+    for (int L = 0; L <= LMAX; L++) mb.lg[L] = crt_product_bits(L);
+    const int64_t items = (sh.aunits > sh.bunits ? sh.aunits : sh.bunits) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-    split_scan_kernel<<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g);
+    split_scan_kernel<<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, runs_residues(g, p), mb);
     count_launch();
     return cudaGetLastError();
 }
@@ -596,28 +650,13 @@ cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, Split
                               cudaStream_t stream) {
     Geo g = make_geo(m, count, p.scheme);
     char *ws = (char *)workspace;
-    {
-        dim3 grid((unsigned)((m + 255) / 256), (unsigned)count);
-        split_finalize_kernel<<<grid, 256, 0, stream>>>(ws, g);
-        count_launch();
-    }
-    // the scheme, written into the header; of the two slicers below, the one
-    // for the other scheme returns at once
-    cudaError_t e = launch_crt_resolve(count, m, p, ws, stream);
-    if (e != cudaSuccess) return e;
-    e = launch_crt_slice(tasks_dev, count, m, p, ws, stream);
-    if (e != cudaSuccess) return e;
-    // a forced residue scheme always runs when the leaves fit it (L <= 17 for
-    // 55-bit operands and K <= 2048): the digit kernels need no launch
-    if (p.scheme == SCHEME_RESIDUES && g.residues_ok) return cudaSuccess;
-    {
-        int64_t atiles = (int64_t)g.mtiles * g.nks;
-        int64_t btiles2 = ((int64_t)g.ntiles * g.nks + 1) / 2;
-        int64_t items = (atiles > btiles2 ? atiles : btiles2) * count;
-        dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-        split_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, m, ws, g, p);
-        count_launch();
-    }
+    if (runs_residues(g, p)) return launch_crt_slice(tasks_dev, count, m, p, ws, stream);
+    int64_t atiles = (int64_t)g.mtiles * g.nks;
+    int64_t btiles2 = ((int64_t)g.ntiles * g.nks + 1) / 2;
+    int64_t items = (atiles > btiles2 ? atiles : btiles2) * count;
+    dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
+    split_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, m, ws, g, p);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -626,26 +665,20 @@ void set_debug_starve(int count) { g_debug_starve = count > 0 ? count : 0; }
 
 cudaError_t launch_split_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
                               unsigned int *status_dev, cudaStream_t stream) {
-    // one starved call covers both GEMM launches (the one for the scheme not
-    // chosen returns at once)
     const int starve = g_debug_starve > 0 ? 1 : 0;
     if (starve) g_debug_starve--;
     Geo g = make_geo(m, count, p.scheme);
     char *ws = (char *)workspace;
-    cudaError_t e;
     split_gemm_prepare();
-    const size_t smem = (size_t)NSTAGE * STAGE_BYTES + 1024 + 1024;
-    e = g_prepare_error;
+    cudaError_t e = g_prepare_error;
     if (e != cudaSuccess) return e;
-    if (!(p.scheme == SCHEME_RESIDUES && g.residues_ok)) {  // see launch_split_prep
-        int64_t total = (int64_t)g.mtiles * g.ntiles * count;
-        int grid = (int)(total < g_num_sms ? total : g_num_sms);
-        split_gemm_kernel<<<grid, GEMM_THREADS, smem, stream>>>(tasks_dev, count, ws, g, p, status_dev, starve);
-        count_launch();
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    return launch_crt_gemm(tasks_dev, count, m, p, ws, status_dev, g_num_sms, stream, starve);
+    if (runs_residues(g, p)) return launch_crt_gemm(tasks_dev, count, m, p, ws, status_dev, g_num_sms, stream, starve);
+    const size_t smem = (size_t)NSTAGE * STAGE_BYTES + 1024 + 1024;
+    int64_t total = (int64_t)g.mtiles * g.ntiles * count;
+    int grid = (int)(total < g_num_sms ? total : g_num_sms);
+    split_gemm_kernel<<<grid, GEMM_THREADS, smem, stream>>>(tasks_dev, count, ws, g, p, status_dev, starve);
+    count_launch();
+    return cudaGetLastError();
 }
 
 }  // namespace caps

@@ -5,7 +5,7 @@
 // or break its accounting), or a code path where the device-wide
 // synchronisation of cudaMalloc / cudaFree is not acceptable.  For them this
 // entry point runs the same kernels as the split form of caps_leaf_gemm_dev
-// (scan, finalize, slice, tcgen05 digit-pair GEMM) with all of its scratch --
+// (scan, slice, tcgen05 digit-pair GEMM) with all of its scratch --
 // the scale arrays, the digit planes, the one-entry task table and the status
 // word -- in the file-scope device array below.  Nothing is allocated: no
 // cudaMalloc, no cudaFree, no pinned host staging.

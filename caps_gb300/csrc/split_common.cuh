@@ -24,16 +24,16 @@ constexpr uint32_t WAIT_LIMIT_STARVED = 1u << 12;
 
 enum { SCHEME_AUTO = 0, SCHEME_DIGITS = 1, SCHEME_RESIDUES = 2 };
 
-// First 256 bytes of a launch group's workspace.  The host reads the first
-// four fields back after a multiply (counters).
+// First 256 bytes of a launch group's workspace, written by the scan kernel.
+// The host reads the first four fields back after a multiply (counters).
 struct SplitHdr {
-    int needed;    // digits needed, max over the group (finalize)
-    int s_used;    // digit scheme: digits and diagonals (resolve)
+    int needed;    // digits needed, max over the group
+    int s_used;    // digit scheme: digits and diagonals
     int nd_used;
-    int moduli;    // residue scheme: moduli used; 0 when the digit scheme runs (resolve)
-    int bitsA;     // max over rows of A of E - lsb + 1 (finalize)
+    int moduli;    // residue scheme: moduli used; 0 when the digit scheme runs
+    int bitsA;     // max over rows of A of E - lsb + 1
     int bitsB;     // the same over the columns of B
-    int residues;  // 1: the residue scheme runs (resolve)
+    int finished;  // leaf sides whose rows / columns are all scanned
     int ta, tb;    // residue scheme: |A'| <= 2^ta, |B'| <= 2^tb
     int pad[55];
 };
@@ -94,6 +94,16 @@ __host__ __device__ inline Geo make_geo(int m, int count, int scheme) {
     g.z_base = g.dg_base + (size_t)count * g.dg_per_leaf;
     g.total = g.z_base + (g.residues_ok ? (size_t)ZCTA_MAX * 2 * ZTILE_BYTES : 0);
     return g;
+}
+
+// The scheme of a launch group: residues wherever the leaves fit them (they
+// are the faster cut, integer data included: the digit GEMM's per-chunk drain
+// of its diagonal accumulators costs about as much at one digit as at eight),
+// digits for larger leaves, when forced, or when a digit count is asked for.
+// 17 moduli always suffice where they fit: 2 x 55 operand bits, 11 bits of
+// K <= 2048 and the sign need 122, and the product of 17 exceeds 2^123.
+inline bool runs_residues(const Geo &g, const SplitParams &p) {
+    return g.residues_ok && !(p.scheme == SCHEME_AUTO && p.slices > 0);
 }
 
 __device__ __forceinline__ char *leaf_scalars(char *ws, const Geo &g, int l) {
