@@ -33,6 +33,8 @@
 
 #include <cmath>
 
+#include <cuda.h>
+
 namespace caps {
 
 using namespace split;
@@ -47,12 +49,12 @@ __host__ __device__ constexpr int modulus(int l) {
 }
 
 constexpr int RSTAGE_K = 4;                       // 16-deep K steps per stage (K = 64)
-constexpr int RNSTAGE = 4;
-constexpr int RA_TILE = TM * TK * 2;              // 4 KiB: 128 x 16 bf16
-constexpr int RB_TILE = RTN * TK * 2;             // 8 KiB: 256 x 16 bf16
-constexpr int RSTAGE_A = RSTAGE_K * RA_TILE;      // 16 KiB
-constexpr int RSTAGE_B = RSTAGE_K * RB_TILE;      // 32 KiB
-constexpr int RSTAGE_BYTES = RSTAGE_A + RSTAGE_B; // 48 KiB
+constexpr int RNSTAGE = 6;
+constexpr int R_TILE = TM * TK * 2;               // 4 KiB: 128 x 16 bf16, A and B alike
+constexpr int RSTAGE_OP = RSTAGE_K * R_TILE;      // 16 KiB: one operand of a stage
+constexpr int RSTAGE_BYTES = 2 * RSTAGE_OP;       // 32 KiB
+constexpr int MAP_ROW = 512;                      // bytes of a row of the planes' tensor map
+constexpr int MAP_BOX = RSTAGE_OP / MAP_ROW;      // 32 rows: an operand's K steps of a stage
 constexpr int RGEMM_THREADS = 320;                // producer, MMA, 8 drain warps
 constexpr unsigned RSTATUS = 0x100;               // status bits of this kernel: RSTATUS << code
 
@@ -347,54 +349,29 @@ __device__ __forceinline__ void write_residues_unrolled(const Limbs2 (&x)[4], ch
     }
 }
 
-// Residue planes, per modulus l:
-//   A: [l][mt][ks] tiles of 128 x 16 (4 KiB), B: [l][rt][ks] tiles of 256 x 16
-//   (8 KiB), each the UMMA canonical K-major image (8-row x 16-byte core
-//   matrices, K halves side by side: K stride 128 B, row-group stride 256 B).
-// A side: one thread = one row x 8 k, a block = one 128 x 16 tile.  B side:
-// one thread = one column x 8 k, a block = half of a 256 x 16 tile.
+// Residue planes, per modulus l: [l][row tile][ks] for A, [l][column tile][ks]
+// for B, tiles of 128 x 16 (4 KiB), each the UMMA canonical K-major image
+// (8-row x 16-byte core matrices, K halves side by side: K stride 128 B,
+// row-group stride 256 B).  One thread = one row of A or column of B x 8 k, a
+// block = one tile.
 __device__ __forceinline__ void crt_slice_tile(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
                                                const Geo &g, const SplitHdr *h, int L, int leaf, int64_t tile,
                                                int side) {
+    const int tiles = side == 0 ? g.mtiles : 2 * g.rtiles;
+    if (tile >= (int64_t)tiles * g.nks) return;
     const LeafTask t = tasks[leaf];
     const char *sc = leaf_scalars(ws, g, leaf);
-    char *pl = leaf_digits(ws, g, leaf);
     const int64_t M = g.m;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, r = tid & 127;
     const int kg = tid >> 7;  // which 8 of the tile's 16 k
-    int64_t idx, k0, sk;      // row of A / column of B, first k, stride between k
-    const double *src;
-    int ee, tt;
-    char *dst;
-    size_t plane_stride;
-    if (side == 0) {
-        if (tile >= (int64_t)g.mtiles * g.nks) return;
-        const int mt = (int)(tile / g.nks), ks = (int)(tile % g.nks);
-        const int r = tid & 127;
-        idx = (int64_t)mt * TM + r;
-        k0 = (int64_t)ks * TK + kg * 8;
-        src = t.A + idx + k0 * M;
-        sk = M;
-        ee = idx < M ? reinterpret_cast<const int *>(sc + g.off_ea)[idx] : 0;
-        tt = h->ta;
-        dst = pl + g.off_ra + ((size_t)mt * g.nks + ks) * RA_TILE + (size_t)(r >> 3) * 256 + (size_t)kg * 128 +
-              (size_t)(r & 7) * 16;
-        plane_stride = (size_t)g.mtiles * g.nks * RA_TILE;
-    } else {
-        if (tile >= (int64_t)g.rtiles * g.nks * 2) return;
-        const int64_t bt = tile >> 1;
-        const int rt = (int)(bt / g.nks), ks = (int)(bt % g.nks);
-        const int c = (int)(tile & 1) * 128 + (tid & 127);
-        idx = (int64_t)rt * RTN + c;
-        k0 = (int64_t)ks * TK + kg * 8;
-        src = t.B + k0 + idx * M;
-        sk = 1;
-        ee = idx < M ? reinterpret_cast<const int *>(sc + g.off_eb)[idx] : 0;
-        tt = h->tb;
-        dst = pl + g.off_rb + ((size_t)rt * g.nks + ks) * RB_TILE + (size_t)(c >> 3) * 256 + (size_t)kg * 128 +
-              (size_t)(c & 7) * 16;
-        plane_stride = (size_t)g.rtiles * g.nks * RB_TILE;
-    }
+    const int64_t idx = tile / g.nks * TM + r, k0 = tile % g.nks * TK + kg * 8;
+    const int64_t sk = side == 0 ? M : 1;  // stride between k
+    const double *src = side == 0 ? t.A + idx + k0 * M : t.B + k0 + idx * M;
+    const int ee = idx < M ? reinterpret_cast<const int *>(sc + (side == 0 ? g.off_ea : g.off_eb))[idx] : 0;
+    const int tt = side == 0 ? h->ta : h->tb;
+    char *dst = leaf_digits(ws, g, leaf) + (side == 0 ? g.off_ra : g.off_rb) + (size_t)tile * R_TILE +
+                (size_t)(r >> 3) * 256 + (size_t)kg * 128 + (size_t)(r & 7) * 16;
+    const size_t plane_stride = (size_t)tiles * g.nks * R_TILE;
     // f = t - E (ee = E + 4096; 0 for a zero row / column); padding rows,
     // columns and k give zero residues
     const bool live = idx < M && ee != 0;
@@ -431,8 +408,8 @@ __global__ void __launch_bounds__(256) crt_slice_kernel(const LeafTask *__restri
                                                         char *__restrict__ ws, Geo g) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int L = h->moduli;
-    const int64_t atiles = (int64_t)g.mtiles * g.nks, bhalves = (int64_t)g.rtiles * g.nks * 2;
-    const int64_t per = atiles > bhalves ? atiles : bhalves;
+    const int64_t atiles = (int64_t)g.mtiles * g.nks, btiles = (int64_t)g.rtiles * g.nks * 2;
+    const int64_t per = atiles > btiles ? atiles : btiles;
     const int64_t total = per * g.count;
     for (int64_t it = blockIdx.x; it < total; it += gridDim.x)
         crt_slice_tile(tasks, ws, g, h, L, (int)(it / per), it % per, blockIdx.y);
@@ -660,14 +637,22 @@ __device__ __forceinline__ void reconstruct_step(const Section &t, int step, con
 }  // namespace
 
 // ---------------------------------------------------------------- gemm
-// Persistent, one CTA per SM, 320 threads: warp 0 loads (one lane, bulk
-// copies of pre-tiled planes), warp 1 issues the MMAs (one lane), warps 2..9
-// drain the accumulators and reconstruct C.
+// Persistent, one CTA per SM in pairs (clusters of two), 320 threads: warp 0
+// loads (one lane, TMA boxes of pre-tiled planes), warp 1 issues the MMAs (one
+// lane of the pair's first CTA), warps 2..9 drain the accumulators and
+// reconstruct C.
 //
-// A work unit is (leaf, 128-row tile, 256-column tile).  For each modulus in
-// turn it takes Kp / 16 MMAs of 128 x 256 x 16 into one of two TMEM
-// accumulators of 256 columns; they alternate, so the drain of one modulus
-// overlaps the MMAs of the next.  The drain reduces each exact sum modulo p
+// A work unit is (leaf, two 128-row tiles, 256-column tile).  For each modulus
+// in turn it takes Kp / 16 MMAs of 256 x 256 x 16 on both SMs: a CTA loads its
+// own 128 rows of A and half of the columns of B, and its 128 x 256 results
+// fall into one of two TMEM accumulators of its own; they alternate, so the
+// drain of one modulus overlaps the MMAs of the next.  Against one-CTA MMAs of
+// 128 x 256 x 16 an SM loads and reads 8 KiB per MMA instead of 12, and six
+// stages of K = 64 fit instead of four: that kernel's issuer waited for data a
+// third of the time.  49 leaves of 2048 at 17 moduli: 10.2 -> 8.53 ms (1405 ->
+// 1677 TFLOP/s of modular products); 49 leaves of 1536: 4.53 -> 3.80 ms (ncu;
+// the one-CTA kernel with its own reconstruction warps).  A last odd row tile leaves the second CTA's half unused.
+// The drain reduces each exact sum modulo p
 // (two values per packed fp32 instruction) and stores the balanced residue as
 // a byte, four columns to a word, into its section of the CTA's
 // product-residue tile; two tiles per CTA are used in turn.
@@ -682,11 +667,9 @@ __device__ __forceinline__ void reconstruct_step(const Section &t, int step, con
 // L = 6) of MMAs.  A section is written and read by one warp, so no barrier
 // hands tiles over.  Measured against those four warps (us a multiply): the
 // n = 16384 integer case (L = 6, leaves of 1024) 139400 -> 102300, n = 6144
-// (leaves of 1536) 7780 -> 7445, one leaf of 448 294 -> 205; n = 16384 with
-// L = 17, leaves of 2048: 107900 -> 102300 or no change, by the GPU (the wait
-// for planes from L2 bounds it: a third of the issuer's time).
+// (leaves of 1536) 7780 -> 7445, one leaf of 448 294 -> 205 (one-CTA MMAs).
 //
-// Units are ordered leaf, row tile, column tile, and the CTAs go through the
+// Units are ordered leaf, row tiles, column tile, and the CTAs go through the
 // moduli in step, so the CTAs running at one time share the A and B planes
 // of one modulus of about one leaf (16 MB at m = 2048) through L2.
 struct DrainArgs {
@@ -695,7 +678,8 @@ struct DrainArgs {
     const Geo *g;
     unsigned char *ztiles;
     unsigned *status;
-    uint32_t tmem, tfull0, tempty0, wl;
+    uint32_t tmem, tfull0, tempty0, wl;  // tempty0: the leader's, a shared::cluster address
+    uint32_t rank;                       // of this CTA in its pair
     int64_t total;
     int tab;
 };
@@ -708,13 +692,13 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quarter = warp & 3;         // TMEM lanes 32*quarter.. (rows of the tile)
     const int colhalf = (warp - 2) >> 2;  // columns 128*colhalf.. of the tile
-    const int64_t M = g.m, tiles = (int64_t)g.mtiles * g.rtiles;
+    const int64_t M = g.m, tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles;
     uint32_t uc = 0, tc = 0;
     Section prev;
     prev.cols = 0;
     bool have = false;
     // one more pass than units: the last unit's reconstruction
-    for (int64_t u = blockIdx.x;; u += gridDim.x, tc++) {
+    for (int64_t u = blockIdx.x >> 1;; u += gridDim.x >> 1, tc++) {
         const bool live = u < a.total;
         if (!live && !have) return;
         uint32_t *zt = reinterpret_cast<uint32_t *>(a.ztiles + (size_t)(tc & 1) * ZTILE_BYTES) +
@@ -766,7 +750,7 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(a.tempty0 + 8 * acc);
+                if (lane == 0) mbar_arrive_remote(a.tempty0 + 8 * acc);
                 uc++;
             }
 #pragma unroll 1
@@ -785,7 +769,7 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
         __syncwarp();  // the section's words, written by all lanes, are read from here on
         const int leafi = (int)(u / tiles);
         const int64_t tile = u % tiles;
-        const int mt = (int)(tile / g.rtiles), rt = (int)(tile % g.rtiles);
+        const int mt = 2 * (int)(tile / g.rtiles) + (int)a.rank, rt = (int)(tile % g.rtiles);
         const char *sc = leaf_scalars(a.ws, g, leafi);
         const int64_t i = (int64_t)mt * TM + quarter * 32 + lane, j = (int64_t)rt * RTN + colhalf * 128;
         prev.row = i < M;
@@ -793,14 +777,14 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
         prev.eb = reinterpret_cast<const int *>(sc + g.off_eb) + j;
         prev.z = zt;
         prev.C = a.tasks[leafi].C + i + j * M;
-        prev.cols = (int)(M - j < 128 ? M - j : 128);
+        prev.cols = mt >= g.mtiles ? 0 : (int)(M - j < 128 ? M - j : 128);
         have = true;
     }
 }
 
-__global__ void __launch_bounds__(RGEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     crt_gemm_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws, Geo g,
-                    unsigned *__restrict__ status, int starve) {
+                    const __grid_constant__ CUtensorMap planes, unsigned *__restrict__ status, int starve) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int L = h->moduli;
     // starve (test hook): no copies are issued, so nothing is ever in flight
@@ -808,15 +792,18 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
     const uint32_t wl = starve ? WAIT_LIMIT_STARVED : WAIT_LIMIT;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char *stA = smem;                        // RNSTAGE x RSTAGE_A
-    unsigned char *stB = smem + RNSTAGE * RSTAGE_A;   // RNSTAGE x RSTAGE_B
+    unsigned char *stA = smem;                        // RNSTAGE x RSTAGE_OP
+    unsigned char *stB = smem + RNSTAGE * RSTAGE_OP;  // RNSTAGE x RSTAGE_OP
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + RNSTAGE * RSTAGE_BYTES);
-    // bars: full[RNSTAGE], empty[RNSTAGE], tfull[2], tempty[2], final
+    // bars: full[RNSTAGE] (the leader's count both CTAs' copies), empty[RNSTAGE]
+    // and tfull[2] (each CTA's, from the leader's commits), tempty[2] (the
+    // leader's, from both CTAs' drain warps), final
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * RNSTAGE + 5);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + RNSTAGE);
     const uint32_t tfull0 = smem_u32(bars + 2 * RNSTAGE), tempty0 = smem_u32(bars + 2 * RNSTAGE + 2);
     const uint32_t finalb = smem_u32(bars + 2 * RNSTAGE + 4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < RNSTAGE; i++) {
@@ -825,70 +812,79 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(tfull0 + 8 * i, 1);
-            mbar_init(tempty0 + 8 * i, 8);   // the 8 drain warps
+            mbar_init(tempty0 + 8 * i, 16);  // the 8 drain warps of both CTAs
         }
         mbar_init(finalb, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                          smem_u32(tmem_slot))
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    const int64_t tiles = (int64_t)g.mtiles * g.rtiles;
+    const int64_t tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles;
     const int64_t total = tiles * g.count;
     const int nks = g.nks;
     unsigned char *ztiles = (unsigned char *)ws + g.z_base + (size_t)blockIdx.x * 2 * ZTILE_BYTES;
 
     if (warp == 0) {
-        // ------------------------------------------------ producer
+        // ------------------------------------------------ producer (both CTAs)
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            uint32_t armed[RNSTAGE] = {0, 0, 0, 0};  // 1 + phase of the last arm
-            for (int64_t u = blockIdx.x; u < total && ok && !starve; u += gridDim.x) {
+            uint32_t armed[RNSTAGE];  // 1 + phase of the last arm
+            for (int i = 0; i < RNSTAGE; i++) armed[i] = 0;
+            const uint32_t lead_full = map_to_rank(full0, 0);
+            for (int64_t u = blockIdx.x >> 1; u < total && ok && !starve; u += gridDim.x >> 1) {
                 const int leafi = (int)(u / tiles);
                 const int64_t tile = u % tiles;
-                const int mt = (int)(tile / g.rtiles), rt = (int)(tile % g.rtiles);
-                const char *pl = leaf_digits(ws, g, leafi);
+                int mt = 2 * (int)(tile / g.rtiles) + (int)rank;
+                if (mt >= g.mtiles) mt = g.mtiles - 1;  // results unused
+                const int ct = 2 * (int)(tile % g.rtiles) + (int)rank;
+                const size_t pl = (size_t)leafi * g.dg_per_leaf;
                 for (int l = 0; l < L && ok; l++) {
-                    const char *srcA = pl + g.off_ra + (((size_t)l * g.mtiles + mt) * nks) * RA_TILE;
-                    const char *srcB = pl + g.off_rb + (((size_t)l * g.rtiles + rt) * nks) * RB_TILE;
+                    // rows of the tensor map; a box past the tile's last K step
+                    // brings what follows it (zeros at the map's end), unused
+                    const int rowA = (int)((pl + g.off_ra + ((size_t)l * g.mtiles + mt) * nks * R_TILE) / MAP_ROW);
+                    const int rowB = (int)((pl + g.off_rb + ((size_t)l * 2 * g.rtiles + ct) * nks * R_TILE) / MAP_ROW);
                     for (int ks = 0; ks < nks; ks += RSTAGE_K) {
-                        const uint32_t n = ks + RSTAGE_K <= nks ? RSTAGE_K : (uint32_t)(nks - ks);
                         if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, status, RSTATUS << 0, wl)) { ok = false; break; }
-                        mbar_expect_tx(full0 + 8 * stage, n * (RA_TILE + RB_TILE));
-                        bulk_g2s(smem_u32(stA + stage * RSTAGE_A), srcA + (size_t)ks * RA_TILE, n * RA_TILE,
-                                 full0 + 8 * stage);
-                        bulk_g2s(smem_u32(stB + stage * RSTAGE_B), srcB + (size_t)ks * RB_TILE, n * RB_TILE,
-                                 full0 + 8 * stage);
+                        if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * RSTAGE_BYTES);
+                        tma_row_box_pair(smem_u32(stA + stage * RSTAGE_OP), &planes, rowA + ks * (R_TILE / MAP_ROW),
+                                         lead_full + 8 * stage);
+                        tma_row_box_pair(smem_u32(stB + stage * RSTAGE_OP), &planes, rowB + ks * (R_TILE / MAP_ROW),
+                                         lead_full + 8 * stage);
                         armed[stage] = 1 + phase;
                         if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
                     }
                 }
             }
-            // every armed stage's copies land before the CTA exits
+            // every armed stage's copies, both CTAs', land before either exits
             for (int i = 0; i < RNSTAGE; i++)
-                if (armed[i]) mbar_wait(full0 + 8 * i, armed[i] - 1, status, RSTATUS << 1, wl);
+                if (rank == 0 && armed[i]) mbar_wait(full0 + 8 * i, armed[i] - 1, status, RSTATUS << 1, wl);
+            // and so have the leader's commits on this CTA's barriers
+            for (int i = 0; i < RNSTAGE && ok; i++)
+                if (armed[i]) ok = mbar_wait(empty0 + 8 * i, armed[i] - 1, status, RSTATUS << 0, wl);
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // ------------------------------------------------ MMA issuer (the leader)
+        if (rank == 0 && lane == 0) {
             // K-direction core-matrix stride (LBO) 128 B, row-group stride (SBO) 256 B
             const uint64_t a0 = sdesc(smem_u32(stA), 128, 256), b0 = sdesc(smem_u32(stB), 128, 256);
-            const uint32_t idesc = idesc_bf16(TM, RTN);
+            const uint32_t idesc = idesc_bf16(2 * TM, RTN);
             int stage = 0;
             uint32_t phase = 0, uc = 0;
             bool ok = true;
-            for (int64_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
+            for (int64_t u = blockIdx.x >> 1; u < total && ok; u += gridDim.x >> 1) {
                 for (int l = 0; l < L && ok; l++, uc++) {
                     const uint32_t acc = uc & 1;
                     if (!mbar_wait(tempty0 + 8 * acc, ((uc >> 1) & 1) ^ 1, status, RSTATUS << 2, wl)) { ok = false; break; }
@@ -898,27 +894,27 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
                         const int n = ks + RSTAGE_K <= nks ? RSTAGE_K : nks - ks;
                         if (!mbar_wait(full0 + 8 * stage, phase, status, RSTATUS << 3, wl)) { ok = false; break; }
                         tc_fence_after();
-                        const uint64_t sa = (uint64_t)((uint32_t)stage * RSTAGE_A) >> 4;
-                        const uint64_t sb = (uint64_t)((uint32_t)stage * RSTAGE_B) >> 4;
+                        const uint64_t so = (uint64_t)((uint32_t)stage * RSTAGE_OP) >> 4;
 #pragma unroll
                         for (int j = 0; j < RSTAGE_K; j++)
                             if (j < n)
-                                umma(dt, a0 + sa + (uint64_t)(j * RA_TILE >> 4), b0 + sb + (uint64_t)(j * RB_TILE >> 4),
-                                     idesc, (ks + j) > 0 ? 1u : 0u);
-                        umma_commit(empty0 + 8 * stage);
+                                umma_pair(dt, a0 + so + (uint64_t)(j * R_TILE >> 4), b0 + so + (uint64_t)(j * R_TILE >> 4),
+                                          idesc, (ks + j) > 0 ? 1u : 0u);
+                        umma_commit_pair(empty0 + 8 * stage);
                         if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
                     }
                     if (!ok) break;
-                    umma_commit(tfull0 + 8 * acc);
+                    umma_commit_pair(tfull0 + 8 * acc);
                 }
             }
             // every issued MMA completes before TMEM is released
-            umma_commit(finalb);
+            umma_commit_pair_local(finalb);
             mbar_wait(finalb, 0, status, RSTATUS << 4, wl);
         }
     } else {
         // ------------------------------------------------ drain and reconstruction (8 warps)
-        const DrainArgs a{tasks, ws, &g, ztiles, status, tmem, tfull0, tempty0, wl, total, h->ta + h->tb};
+        const DrainArgs a{tasks,  ws,     &g, ztiles, status, tmem, tfull0, map_to_rank(tempty0, 0),
+                          wl,     rank,   total, h->ta + h->tb};
         switch (L) {
 #define CAPS_DRAIN(n) case n: drain_and_reconstruct<n>(a); break;
             CAPS_DRAIN(1) CAPS_DRAIN(2) CAPS_DRAIN(3) CAPS_DRAIN(4) CAPS_DRAIN(5) CAPS_DRAIN(6)
@@ -930,9 +926,10 @@ __global__ void __launch_bounds__(RGEMM_THREADS, 1)
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // neither CTA leaves while the other may read its shared memory or arrive on its barriers
     tc_fence_after();
     if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -941,6 +938,7 @@ static CrtTables g_tables_host;
 static bool g_tables_built = false;
 static int g_crt_device = -1;
 static cudaError_t g_crt_error = cudaSuccess;
+static decltype(&cuTensorMapEncodeTiled) g_encode_tiled = nullptr;
 
 cudaError_t crt_prepare() {
     int dev = 0;
@@ -951,6 +949,13 @@ cudaError_t crt_prepare() {
         g_tables_built = true;
     }
     g_crt_error = cudaMemcpyToSymbol(c_crt, &g_tables_host, sizeof(CrtTables));
+    if (g_crt_error == cudaSuccess) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        g_crt_error = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
+        if (g_crt_error == cudaSuccess && (found != cudaDriverEntryPointSuccess || !fn)) g_crt_error = cudaErrorNotSupported;
+        g_encode_tiled = (decltype(&cuTensorMapEncodeTiled))fn;
+    }
     if (g_crt_error == cudaSuccess) {
         const size_t smem = (size_t)RNSTAGE * RSTAGE_BYTES + 1024 + 1024;
         g_crt_error = cudaFuncSetAttribute(crt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -966,8 +971,8 @@ cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitP
     cudaError_t e = crt_prepare();
     if (e != cudaSuccess) return e;
     Geo g = make_geo(m, count, p.scheme);
-    const int64_t atiles = (int64_t)g.mtiles * g.nks, bhalves = (int64_t)g.rtiles * g.nks * 2;
-    const int64_t items = (atiles > bhalves ? atiles : bhalves) * count;
+    const int64_t atiles = (int64_t)g.mtiles * g.nks, btiles = (int64_t)g.rtiles * g.nks * 2;
+    const int64_t items = (atiles > btiles ? atiles : btiles) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
     crt_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g);
     count_launch();
@@ -979,11 +984,20 @@ cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitPa
     Geo g = make_geo(m, count, p.scheme);
     cudaError_t e = crt_prepare();
     if (e != cudaSuccess) return e;
-    const int64_t units = (int64_t)g.mtiles * g.rtiles * count;
-    int grid = (int)(units < num_sms ? units : num_sms);
-    if (grid > ZCTA_MAX) grid = ZCTA_MAX;  // two product-residue tiles per CTA
+    // the leaves' plane blocks as rows of 512 bytes (every plane starts on one)
+    CUtensorMap planes;
+    const cuuint64_t dims[2] = {MAP_ROW / 2, (cuuint64_t)((size_t)count * g.dg_per_leaf / MAP_ROW)};
+    const cuuint64_t strides[1] = {MAP_ROW};
+    const cuuint32_t box[2] = {MAP_ROW / 2, MAP_BOX}, ones[2] = {1, 1};
+    if (g_encode_tiled(&planes, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (char *)workspace + g.dg_base, dims, strides, box,
+                       ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                       CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    const int64_t units = (int64_t)((g.mtiles + 1) / 2) * g.rtiles * count;
+    int pairs = (int)(units < num_sms / 2 ? units : num_sms / 2);
+    if (pairs > ZCTA_MAX / 2) pairs = ZCTA_MAX / 2;  // two product-residue tiles per CTA
     const size_t smem = (size_t)RNSTAGE * RSTAGE_BYTES + 1024 + 1024;
-    crt_gemm_kernel<<<grid, RGEMM_THREADS, smem, stream>>>(tasks_dev, (char *)workspace, g, status_dev, starve);
+    crt_gemm_kernel<<<2 * pairs, RGEMM_THREADS, smem, stream>>>(tasks_dev, (char *)workspace, g, planes, status_dev, starve);
     count_launch();
     return cudaGetLastError();
 }
