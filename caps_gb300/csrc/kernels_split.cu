@@ -69,16 +69,23 @@ size_t split_workspace_bytes(int m, int count, int scheme) {
 // when the leaf's element pairs are 16-byte aligned (m even, base aligned),
 // 8-byte loads otherwise.  grid.x strides over (leaf, unit).
 //
-// The block that finishes a leaf side turns its exponents into the digit
-// scheme's f and the group's digit and bit counts, and the block that
-// finishes the last side of the group writes the header: no kernels of their
-// own (they took 7 us of a small multiply's 200).  HBM-bound at full size;
-// a few leaves are bound by the longest unit, so the slab and the columns of a
-// warp shrink until a launch has SCAN_UNITS units a side or the unit is 8
-// columns a thread (1200 units were 7 us slower at 7 leaves of 896, 300 were
-// 8 us slower at 7 leaves of 2500).  Scan and counts together, before -> here:
-// one leaf of 448 52 -> 12 us, 7 leaves of 896 57 -> 32, of 2500 147 -> 148.
+// Afterwards each leaf side's exponents become the digit scheme's f and the
+// group's digit and bit counts (finish_side), and the last side of the group
+// writes the header.  A launch whose units all fit the GPU at once does this
+// itself, in the blocks that end a side: a small multiply saves two kernels'
+// 7 us of 200.  In a larger one the wait at each unit's end costs more than
+// the kernel it saves (49 leaves of 2048: 552 us against 507 + 9), so there a
+// second kernel does it.  HBM-bound at full size, with SCAN_BATCH loads of 16
+// bytes a thread issued before the first is used (the unrolled loop kept fewer
+// in flight: 49 leaves of 2048 507 -> 475 us, 7 of 2500 142 -> 119); a few
+// leaves are bound by
+// the longest unit, so the slab and the columns of a warp shrink until a
+// launch has SCAN_UNITS units a side or the unit is 8 columns a thread (1200
+// units were 7 us slower at 7 leaves of 896, 300 were 8 us slower at 7 leaves
+// of 2500).  Scan and counts together, before -> here: one leaf of 448 52 ->
+// 10 us, 7 leaves of 896 56 -> 28.
 constexpr int SCAN_UNITS = 600;
+constexpr int SCAN_BATCH = 4;  // 16-byte loads a thread has in flight
 
 struct ScanShape {
     int rt, kt;            // A side: row pairs and column groups of a block (rt * kt = 256)
@@ -142,12 +149,52 @@ __device__ __forceinline__ void resolve_group(SplitHdr *h, const Geo &g, SplitPa
     h->moduli = L;
 }
 
+// One leaf side, by a block: f = 55 - E per row / column (digit scheme),
+// digits needed, and the bits E - lsb + 1; the last side of the group resolves it.
+__device__ __forceinline__ void finish_side(char *__restrict__ ws, const Geo &g, int leaf, int side, SplitParams p,
+                                            bool residues, const ModuliBits &mb) {
+    SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
+    char *sc = leaf_scalars(ws, g, leaf);
+    const int *ev = reinterpret_cast<const int *>(sc + (side ? g.off_eb : g.off_ea));
+    const int *lv = reinterpret_cast<const int *>(sc + (side ? g.off_lb : g.off_la));
+    int *f = reinterpret_cast<int *>(sc + (side ? g.off_fb : g.off_fa));
+    int bits = 0;
+#pragma unroll 8
+    for (int idx = threadIdx.x; idx < g.m; idx += 256) {
+        const int ee = __ldcg(ev + idx), le = __ldcg(lv + idx);
+        int fi = 0;
+        if (ee != 0) {
+            const int E = ee - 4096, lsb = 4096 - le;
+            fi = 55 - E;
+            bits = max(bits, E - lsb + 1);
+        }
+        f[idx] = fi;
+    }
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    if ((threadIdx.x & 31) == 0 && bits > 0) {
+        atomicMax(&h->needed, (bits + 6) / 7);
+        atomicMax(side ? &h->bitsB : &h->bitsA, bits);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const bool all = atomicAdd(&h->finished, 1) == 2 * g.count - 1;
+        __threadfence();
+        if (all) resolve_group(h, g, p, residues, mb);
+    }
+}
+
+__global__ void __launch_bounds__(256) split_finish_kernel(char *__restrict__ ws, Geo g, SplitParams p, int residues,
+                                                           ModuliBits mb) {
+    finish_side(ws, g, blockIdx.x, blockIdx.y, p, residues != 0, mb);
+}
+
+template <bool FINISH>
 __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restrict__ tasks,
                                                          char *__restrict__ ws, Geo g, ScanShape sh, SplitParams p,
                                                          int residues, ModuliBits mb) {
     const int side = blockIdx.y;
     const int64_t M = g.m, units = side ? sh.bunits : sh.aunits, total = units * g.count;
-    SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
     __shared__ int last;
     for (int64_t it = blockIdx.x; it < total; it += gridDim.x) {
         const int l = (int)(it / units);
@@ -163,8 +210,18 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
             const double *col = t.A + i0 + k0 * M;
             int e0 = -100000, l0 = 100000, e1 = -100000, l1 = 100000;
             if ((M & 1) == 0 && ((uintptr_t)t.A & 15) == 0) {  // i0 even, M even: the pair is 16-byte aligned
-#pragma unroll 8
-                for (int k = 0; k < n; k++, col += step) {
+                int k = 0;
+                for (; k + SCAN_BATCH <= n; k += SCAN_BATCH) {
+                    double2 v[SCAN_BATCH];
+#pragma unroll
+                    for (int b = 0; b < SCAN_BATCH; b++, col += step) v[b] = __ldg(reinterpret_cast<const double2 *>(col));
+#pragma unroll
+                    for (int b = 0; b < SCAN_BATCH; b++) {
+                        scan_value(v[b].x, e0, l0);
+                        scan_value(v[b].y, e1, l1);
+                    }
+                }
+                for (; k < n; k++, col += step) {
                     const double2 v = __ldg(reinterpret_cast<const double2 *>(col));
                     scan_value(v.x, e0, l0);
                     scan_value(v.y, e1, l1);
@@ -196,9 +253,21 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
                 const double *col = t.B + j * M;
                 int emax = -100000, lmin = 100000;
                 if (vec) {
-#pragma unroll 8
-                    for (int64_t k = 2 * lane; k < M; k += 64) {
-                        const double2 v = __ldg(reinterpret_cast<const double2 *>(col + k));
+                    const double2 *p = reinterpret_cast<const double2 *>(col) + lane;
+                    int k = lane;
+                    const int n = (int)(M / 2);
+                    for (; k + 32 * (SCAN_BATCH - 1) < n; k += 32 * SCAN_BATCH, p += 32 * SCAN_BATCH) {
+                        double2 v[SCAN_BATCH];
+#pragma unroll
+                        for (int b = 0; b < SCAN_BATCH; b++) v[b] = __ldg(p + 32 * b);
+#pragma unroll
+                        for (int b = 0; b < SCAN_BATCH; b++) {
+                            scan_value(v[b].x, emax, lmin);
+                            scan_value(v[b].y, emax, lmin);
+                        }
+                    }
+                    for (; k < n; k += 32, p += 32) {
+                        const double2 v = __ldg(p);
                         scan_value(v.x, emax, lmin);
                         scan_value(v.y, emax, lmin);
                     }
@@ -214,6 +283,7 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
                 }
             }
         }
+        if (!FINISH) continue;
         // This leaf side's units done so far, counted where its first f will
         // be (zero until then); the block's exponents are visible before it
         // counts, and all the others' once it was the last to.
@@ -225,33 +295,7 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
             __threadfence();
         }
         __syncthreads();
-        if (!last) continue;
-        const int *ev = reinterpret_cast<const int *>(sc + (side ? g.off_eb : g.off_ea));
-        const int *lv = reinterpret_cast<const int *>(sc + (side ? g.off_lb : g.off_la));
-        int bits = 0;
-#pragma unroll 8
-        for (int idx = threadIdx.x; idx < g.m; idx += 256) {
-            const int ee = __ldcg(ev + idx), le = __ldcg(lv + idx);
-            int fi = 0;
-            if (ee != 0) {
-                const int E = ee - 4096, lsb = 4096 - le;
-                fi = 55 - E;
-                bits = max(bits, E - lsb + 1);
-            }
-            f[idx] = fi;
-        }
-        bits = __reduce_max_sync(0xffffffffu, bits);
-        if ((threadIdx.x & 31) == 0 && bits > 0) {
-            atomicMax(&h->needed, (bits + 6) / 7);
-            atomicMax(side ? &h->bitsB : &h->bitsA, bits);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            const bool all = atomicAdd(&h->finished, 1) == 2 * g.count - 1;
-            __threadfence();
-            if (all) resolve_group(h, g, p, residues != 0, mb);
-        }
+        if (last) finish_side(ws, g, l, side, p, residues != 0, mb);
     }
 }
 
@@ -641,8 +685,16 @@ cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, Split
     for (int L = 0; L <= LMAX; L++) mb.lg[L] = crt_product_bits(L);
     const int64_t items = (sh.aunits > sh.bunits ? sh.aunits : sh.bunits) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-    split_scan_kernel<<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, runs_residues(g, p), mb);
-    count_launch();
+    const int residues = runs_residues(g, p);
+    // 48 registers a thread: 5 blocks of 256 on each of 152 SMs at once
+    if ((sh.aunits + sh.bunits) * count <= 152 * 5) {
+        split_scan_kernel<true><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb);
+        count_launch();
+    } else {
+        split_scan_kernel<false><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb);
+        split_finish_kernel<<<dim3((unsigned)count, 2), 256, 0, stream>>>((char *)workspace, g, p, residues, mb);
+        count_launch(2);
+    }
     return cudaGetLastError();
 }
 
