@@ -1226,12 +1226,16 @@ static caps_status run_plan_direct(BatchPlan &p, cudaStream_t s) {
 // choices are kept per process and in an on-disk cache (tune_cache_*).
 
 // On-disk cache of the tuner's choices: one tab-separated line per choice,
-// keyed by the tuning version, the device's name and SM count, the size,
-// form, slices and asked-for scheme.  The file is CAPS_AUTOTUNE_CACHE if set
+// keyed by the tuning version, the device's name, its SM count and the
+// kernels' generation, the size, form, slices and asked-for scheme.  The file is CAPS_AUTOTUNE_CACHE if set
 // (empty: no disk cache), else $HOME/.cache/caps_gb300/autotune.tsv.  A new
 // tuning version (a change of the kernels or axes the choices were made
 // with) leaves older lines unused; deleting the file forces new timings.
 static const char *kTuneVersion = "caps-tune-4";
+// The device key's last part: kernels of other speeds make other choices
+// (2: items and the combine kernel in the residue GEMM's small launches, where
+// leaves of 448 and 896 had run faster as digits).
+static const char *kTuneKernels = "2";
 
 static std::string tune_cache_path() {
     const char *e = getenv("CAPS_AUTOTUNE_CACHE");
@@ -1251,7 +1255,7 @@ static std::string tune_device_key() {
     std::string name(prop.name);
     for (char &c : name)
         if (c == '\t' || c == ' ') c = '_';
-    return name + "/" + std::to_string(prop.multiProcessorCount);
+    return name + "/" + std::to_string(prop.multiProcessorCount) + "/" + kTuneKernels;
 }
 
 // One line of the on-disk cache (tune_cache_store's format): true if it

@@ -672,6 +672,41 @@ __device__ __forceinline__ void reconstruct_step(const Section &t, int step, con
 // Units are ordered leaf, row tiles, column tile, and the CTAs go through the
 // moduli in step, so the CTAs running at one time share the A and B planes
 // of one modulus of about one leaf (16 MB at m = 2048) through L2.
+//
+// That needs many units a pair.  A launch with few of them (one leaf of 448
+// has 4, for 76 pairs) hands out (unit, modulus) items instead, in turn, all
+// units of a modulus before the next, so that the pairs still share its planes
+// (as runs of one unit's moduli, a leaf of 1792 read every tile's planes from
+// DRAM: 210 us instead of 111).  Each unit then has a residue tile per CTA, and
+// crt_combine_kernel turns the tiles into C with the whole GPU; launch_crt_gemm
+// has the rule.
+struct Items {
+    uint32_t total, pairs, c, L, count;
+    int split;
+
+    __device__ Items(int64_t units, int L_, int split_) : split(split_) {
+        total = (uint32_t)units;
+        L = (uint32_t)L_;
+        c = blockIdx.x >> 1;
+        pairs = gridDim.x >> 1;
+        const uint32_t n = split ? total * L : total;  // items or units handed out in turn
+        count = c < n ? (n - c + pairs - 1) / pairs : 0;
+        if (!split) count *= L;
+    }
+    // this pair's k-th item: unit u, modulus l
+    __device__ void get(uint32_t k, uint32_t &u, uint32_t &l) const {
+        if (split) {
+            const uint32_t i = c + k * pairs;
+            l = i / total;
+            u = i - l * total;
+        } else {
+            const uint32_t i = k / L;
+            l = k - i * L;
+            u = c + i * pairs;
+        }
+    }
+};
+
 struct DrainArgs {
     const LeafTask *tasks;
     char *ws;
@@ -684,6 +719,77 @@ struct DrainArgs {
     int tab;
 };
 
+// One accumulator's residues into a warp's section of modulus l's plane; the
+// accumulator is free afterwards.
+__device__ __forceinline__ void drain_modulus(const DrainArgs &a, int l, uint32_t acc, int quarter, int colhalf,
+                                              uint32_t *out) {
+    tc_fence_after();
+    const float2 invp = c_crt.invp2[l], np = c_crt.np2[l];
+#pragma unroll 1
+    for (int c4 = 0; c4 < 4; c4++) {
+        uint32_t v[32];
+        tmem_ld32(a.tmem + ((uint32_t)(quarter * 32) << 16) + acc * RTN + colhalf * 128 + c4 * 32, v);
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            // c = sum rA rB = y A'B' mod p (exact, |c| < 2^24; A's residues
+            // carry y).  q = c fl(1/p) rounded by MAGIC is within 1/2 +
+            // |c / p| 2^-24 <= 1/2 + 1/p of c / p, so z = c - q p has |z| <=
+            // p / 2 + 1 and z = c mod p.
+            uint32_t b[4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float2 c = make_float2(__uint_as_float(v[4 * w + 2 * h]), __uint_as_float(v[4 * w + 2 * h + 1]));
+                const float2 q =
+                    __fadd2_rn(__ffma2_rn(c, invp, make_float2(MAGIC, MAGIC)), make_float2(-MAGIC, -MAGIC));
+                const float2 z = __fadd2_rn(__ffma2_rn(q, np, c), make_float2(MAGIC + ZOFF, MAGIC + ZOFF));
+                b[2 * h] = __float_as_uint(z.x);  // low byte: z + ZOFF
+                b[2 * h + 1] = __float_as_uint(z.y);
+            }
+            out[(c4 * 8 + w) * 32] =
+                __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive_remote(a.tempty0 + 8 * acc);
+}
+
+// A warp's section of unit u, tile row and column offsets of the section given.
+__device__ __forceinline__ Section unit_section(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
+                                                const Geo &g, int tab, int64_t u, int rank, int section,
+                                                const uint32_t *z) {
+    const int64_t M = g.m, tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles, tile = u % tiles;
+    const int leafi = (int)(u / tiles), lane = threadIdx.x & 31;
+    // sections are numbered by drain warp: warp 2 + section has TMEM quarter (2 + section) % 4
+    const int quarter = (2 + section) & 3, colhalf = section >> 2;
+    const int mt = 2 * (int)(tile / g.rtiles) + rank, rt = (int)(tile % g.rtiles);
+    const char *sc = leaf_scalars(ws, g, leafi);
+    const int64_t i = (int64_t)mt * TM + quarter * 32 + lane, j = (int64_t)rt * RTN + colhalf * 128;
+    Section t;
+    t.row = i < M;
+    t.e = (t.row ? reinterpret_cast<const int *>(sc + g.off_ea)[i] : 0) - 8192 - tab;
+    t.eb = reinterpret_cast<const int *>(sc + g.off_eb) + j;
+    t.z = z;
+    t.C = tasks[leafi].C + i + j * M;
+    t.cols = mt >= g.mtiles ? 0 : (int)(M - j < 128 ? M - j : 128);
+    return t;
+}
+
+// split launches: the residues alone, each unit's into a tile of its own
+__device__ __forceinline__ void drain_only(const DrainArgs &a, const Items &items) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quarter = warp & 3, colhalf = (warp - 2) >> 2;
+    for (uint32_t k = 0; k < items.count; k++) {
+        uint32_t u, l;
+        items.get(k, u, l);
+        const bool got = mbar_wait(a.tfull0 + 8 * (k & 1), (k >> 1) & 1, a.status, RSTATUS << 5, a.wl);
+        if (!__all_sync(0xffffffffu, got)) return;
+        drain_modulus(a, (int)l, k & 1, quarter, colhalf,
+                      reinterpret_cast<uint32_t *>(a.ztiles + (size_t)(2 * u + a.rank) * ZTILE_BYTES) +
+                          (size_t)l * ZPLANE_WORDS + (warp - 2) * ZSECTION_WORDS + lane);
+    }
+}
+
 template <int L>
 __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
     constexpr int NC = (ZSTEPS + L - 1) / L;        // reconstruction steps per modulus
@@ -692,7 +798,7 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quarter = warp & 3;         // TMEM lanes 32*quarter.. (rows of the tile)
     const int colhalf = (warp - 2) >> 2;  // columns 128*colhalf.. of the tile
-    const int64_t M = g.m, tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles;
+    const int64_t M = g.m;
     uint32_t uc = 0, tc = 0;
     Section prev;
     prev.cols = 0;
@@ -719,38 +825,7 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
                 // warp-uniform: tcgen05.ld below is .sync.aligned
                 const bool got = mbar_wait(a.tfull0 + 8 * acc, (uc >> 1) & 1, a.status, RSTATUS << 5, a.wl);
                 if (!__all_sync(0xffffffffu, got)) return;
-                tc_fence_after();
-                const float2 invp = c_crt.invp2[l], np = c_crt.np2[l];
-                uint32_t *out = zt + (size_t)l * ZPLANE_WORDS;
-#pragma unroll 1
-                for (int c4 = 0; c4 < 4; c4++) {
-                    uint32_t v[32];
-                    tmem_ld32(a.tmem + ((uint32_t)(quarter * 32) << 16) + acc * RTN + colhalf * 128 + c4 * 32, v);
-#pragma unroll
-                    for (int w = 0; w < 8; w++) {
-                        // c = sum rA rB = y A'B' mod p (exact, |c| < 2^24; A's
-                        // residues carry y).  q = c fl(1/p) rounded by MAGIC is
-                        // within 1/2 + |c / p| 2^-24 <= 1/2 + 1/p of c / p, so
-                        // z = c - q p has |z| <= p / 2 + 1 and z = c mod p.
-                        uint32_t b[4];
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const float2 c = make_float2(__uint_as_float(v[4 * w + 2 * h]),
-                                                         __uint_as_float(v[4 * w + 2 * h + 1]));
-                            const float2 q = __fadd2_rn(__ffma2_rn(c, invp, make_float2(MAGIC, MAGIC)),
-                                                        make_float2(-MAGIC, -MAGIC));
-                            const float2 z = __fadd2_rn(__ffma2_rn(q, np, c),
-                                                        make_float2(MAGIC + ZOFF, MAGIC + ZOFF));
-                            b[2 * h] = __float_as_uint(z.x);  // low byte: z + ZOFF
-                            b[2 * h + 1] = __float_as_uint(z.y);
-                        }
-                        out[(c4 * 8 + w) * 32] =
-                            __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_remote(a.tempty0 + 8 * acc);
+                drain_modulus(a, l, acc, quarter, colhalf, zt + (size_t)l * ZPLANE_WORDS);
                 uc++;
             }
 #pragma unroll 1
@@ -767,24 +842,15 @@ __device__ __forceinline__ void drain_and_reconstruct(const DrainArgs &a) {
         }
         if (!live) return;
         __syncwarp();  // the section's words, written by all lanes, are read from here on
-        const int leafi = (int)(u / tiles);
-        const int64_t tile = u % tiles;
-        const int mt = 2 * (int)(tile / g.rtiles) + (int)a.rank, rt = (int)(tile % g.rtiles);
-        const char *sc = leaf_scalars(a.ws, g, leafi);
-        const int64_t i = (int64_t)mt * TM + quarter * 32 + lane, j = (int64_t)rt * RTN + colhalf * 128;
-        prev.row = i < M;
-        prev.e = (prev.row ? reinterpret_cast<const int *>(sc + g.off_ea)[i] : 0) - 8192 - a.tab;
-        prev.eb = reinterpret_cast<const int *>(sc + g.off_eb) + j;
-        prev.z = zt;
-        prev.C = a.tasks[leafi].C + i + j * M;
-        prev.cols = mt >= g.mtiles ? 0 : (int)(M - j < 128 ? M - j : 128);
+        prev = unit_section(a.tasks, a.ws, g, a.tab, u, (int)a.rank, warp - 2, zt);
         have = true;
     }
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     crt_gemm_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws, Geo g,
-                    const __grid_constant__ CUtensorMap planes, unsigned *__restrict__ status, int starve) {
+                    const __grid_constant__ CUtensorMap planes, unsigned *__restrict__ status, int split,
+                    int starve) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int L = h->moduli;
     // starve (test hook): no copies are issued, so nothing is ever in flight
@@ -833,7 +899,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     const int64_t tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles;
     const int64_t total = tiles * g.count;
     const int nks = g.nks;
-    unsigned char *ztiles = (unsigned char *)ws + g.z_base + (size_t)blockIdx.x * 2 * ZTILE_BYTES;
+    const Items items(total, L, split);
+    unsigned char *ztiles = (unsigned char *)ws + g.z_base + (split ? 0 : (size_t)blockIdx.x * 2 * ZTILE_BYTES);
 
     if (warp == 0) {
         // ------------------------------------------------ producer (both CTAs)
@@ -844,28 +911,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
             uint32_t armed[RNSTAGE];  // 1 + phase of the last arm
             for (int i = 0; i < RNSTAGE; i++) armed[i] = 0;
             const uint32_t lead_full = map_to_rank(full0, 0);
-            for (int64_t u = blockIdx.x >> 1; u < total && ok && !starve; u += gridDim.x >> 1) {
-                const int leafi = (int)(u / tiles);
-                const int64_t tile = u % tiles;
+            for (uint32_t k = 0; k < items.count && ok && !starve; k++) {
+                uint32_t u, l;
+                items.get(k, u, l);
+                const uint32_t leafi = u / (uint32_t)tiles, tile = u - leafi * (uint32_t)tiles;
                 int mt = 2 * (int)(tile / g.rtiles) + (int)rank;
                 if (mt >= g.mtiles) mt = g.mtiles - 1;  // results unused
                 const int ct = 2 * (int)(tile % g.rtiles) + (int)rank;
                 const size_t pl = (size_t)leafi * g.dg_per_leaf;
-                for (int l = 0; l < L && ok; l++) {
-                    // rows of the tensor map; a box past the tile's last K step
-                    // brings what follows it (zeros at the map's end), unused
-                    const int rowA = (int)((pl + g.off_ra + ((size_t)l * g.mtiles + mt) * nks * R_TILE) / MAP_ROW);
-                    const int rowB = (int)((pl + g.off_rb + ((size_t)l * 2 * g.rtiles + ct) * nks * R_TILE) / MAP_ROW);
-                    for (int ks = 0; ks < nks; ks += RSTAGE_K) {
-                        if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, status, RSTATUS << 0, wl)) { ok = false; break; }
-                        if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * RSTAGE_BYTES);
-                        tma_row_box_pair(smem_u32(stA + stage * RSTAGE_OP), &planes, rowA + ks * (R_TILE / MAP_ROW),
-                                         lead_full + 8 * stage);
-                        tma_row_box_pair(smem_u32(stB + stage * RSTAGE_OP), &planes, rowB + ks * (R_TILE / MAP_ROW),
-                                         lead_full + 8 * stage);
-                        armed[stage] = 1 + phase;
-                        if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
-                    }
+                // rows of the tensor map; a box past the tile's last K step
+                // brings what follows it (zeros at the map's end), unused
+                const int rowA = (int)((pl + g.off_ra + ((size_t)l * g.mtiles + mt) * nks * R_TILE) / MAP_ROW);
+                const int rowB = (int)((pl + g.off_rb + ((size_t)l * 2 * g.rtiles + ct) * nks * R_TILE) / MAP_ROW);
+                for (int ks = 0; ks < nks; ks += RSTAGE_K) {
+                    if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, status, RSTATUS << 0, wl)) { ok = false; break; }
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * RSTAGE_BYTES);
+                    tma_row_box_pair(smem_u32(stA + stage * RSTAGE_OP), &planes, rowA + ks * (R_TILE / MAP_ROW),
+                                     lead_full + 8 * stage);
+                    tma_row_box_pair(smem_u32(stB + stage * RSTAGE_OP), &planes, rowB + ks * (R_TILE / MAP_ROW),
+                                     lead_full + 8 * stage);
+                    armed[stage] = 1 + phase;
+                    if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
                 }
             }
             // every armed stage's copies, both CTAs', land before either exits
@@ -882,30 +948,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
             const uint64_t a0 = sdesc(smem_u32(stA), 128, 256), b0 = sdesc(smem_u32(stB), 128, 256);
             const uint32_t idesc = idesc_bf16(2 * TM, RTN);
             int stage = 0;
-            uint32_t phase = 0, uc = 0;
+            uint32_t phase = 0;
             bool ok = true;
-            for (int64_t u = blockIdx.x >> 1; u < total && ok; u += gridDim.x >> 1) {
-                for (int l = 0; l < L && ok; l++, uc++) {
-                    const uint32_t acc = uc & 1;
-                    if (!mbar_wait(tempty0 + 8 * acc, ((uc >> 1) & 1) ^ 1, status, RSTATUS << 2, wl)) { ok = false; break; }
+            for (uint32_t k = 0; k < items.count && ok; k++) {
+                const uint32_t acc = k & 1;
+                if (!mbar_wait(tempty0 + 8 * acc, ((k >> 1) & 1) ^ 1, status, RSTATUS << 2, wl)) break;
+                tc_fence_after();
+                const uint32_t dt = tmem + acc * RTN;
+                for (int ks = 0; ks < nks; ks += RSTAGE_K) {
+                    const int n = ks + RSTAGE_K <= nks ? RSTAGE_K : nks - ks;
+                    if (!mbar_wait(full0 + 8 * stage, phase, status, RSTATUS << 3, wl)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t dt = tmem + acc * RTN;
-                    for (int ks = 0; ks < nks; ks += RSTAGE_K) {
-                        const int n = ks + RSTAGE_K <= nks ? RSTAGE_K : nks - ks;
-                        if (!mbar_wait(full0 + 8 * stage, phase, status, RSTATUS << 3, wl)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint64_t so = (uint64_t)((uint32_t)stage * RSTAGE_OP) >> 4;
+                    const uint64_t so = (uint64_t)((uint32_t)stage * RSTAGE_OP) >> 4;
 #pragma unroll
-                        for (int j = 0; j < RSTAGE_K; j++)
-                            if (j < n)
-                                umma_pair(dt, a0 + so + (uint64_t)(j * R_TILE >> 4), b0 + so + (uint64_t)(j * R_TILE >> 4),
-                                          idesc, (ks + j) > 0 ? 1u : 0u);
-                        umma_commit_pair(empty0 + 8 * stage);
-                        if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
-                    }
-                    if (!ok) break;
-                    umma_commit_pair(tfull0 + 8 * acc);
+                    for (int j = 0; j < RSTAGE_K; j++)
+                        if (j < n)
+                            umma_pair(dt, a0 + so + (uint64_t)(j * R_TILE >> 4), b0 + so + (uint64_t)(j * R_TILE >> 4),
+                                      idesc, (ks + j) > 0 ? 1u : 0u);
+                    umma_commit_pair(empty0 + 8 * stage);
+                    if (++stage == RNSTAGE) { stage = 0; phase ^= 1; }
                 }
+                if (ok) umma_commit_pair(tfull0 + 8 * acc);
             }
             // every issued MMA completes before TMEM is released
             umma_commit_pair_local(finalb);
@@ -915,7 +978,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
         // ------------------------------------------------ drain and reconstruction (8 warps)
         const DrainArgs a{tasks,  ws,     &g, ztiles, status, tmem, tfull0, map_to_rank(tempty0, 0),
                           wl,     rank,   total, h->ta + h->tb};
-        switch (L) {
+        if (split) drain_only(a, items);
+        else switch (L) {
 #define CAPS_DRAIN(n) case n: drain_and_reconstruct<n>(a); break;
             CAPS_DRAIN(1) CAPS_DRAIN(2) CAPS_DRAIN(3) CAPS_DRAIN(4) CAPS_DRAIN(5) CAPS_DRAIN(6)
             CAPS_DRAIN(7) CAPS_DRAIN(8) CAPS_DRAIN(9) CAPS_DRAIN(10) CAPS_DRAIN(11) CAPS_DRAIN(12)
@@ -930,6 +994,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     tc_fence_after();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------- combine
+// C from the residue tiles of a split launch: a warp per step of a section
+// (32 rows x 4 columns), blockIdx.x over (tile, section, four steps).  Its
+// loads are independent and its arithmetic is that of the drain warps; with
+// every SM at it one leaf of 448 takes 8 us and one of 2048 41; the GEMM kernel
+// of the leaf of 448 took 111 us with its 4 pairs reconstructing, and takes 11.
+template <int L>
+__device__ __forceinline__ void combine_step(const Section &t, int step, int64_t M) {
+    uint32_t z[L];
+    load_step<L>(t, step, z);
+    reconstruct_step<L>(t, step, z, M);
+}
+
+__global__ void __launch_bounds__(128) crt_combine_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
+                                                          Geo g) {
+    const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
+    const int section = (blockIdx.x >> 3) & 7, step = (blockIdx.x & 7) * 4 + (threadIdx.x >> 5);
+    const int64_t tile = blockIdx.x >> 6;
+    const uint32_t *z = reinterpret_cast<const uint32_t *>(ws + g.z_base + (size_t)tile * ZTILE_BYTES) +
+                        section * ZSECTION_WORDS + (threadIdx.x & 31);
+    const Section t = unit_section(tasks, ws, g, h->ta + h->tb, tile >> 1, (int)(tile & 1), section, z);
+    if (4 * step >= t.cols) return;
+    switch (h->moduli) {
+#define CAPS_COMBINE(n) case n: combine_step<n>(t, step, g.m); break;
+        CAPS_COMBINE(1) CAPS_COMBINE(2) CAPS_COMBINE(3) CAPS_COMBINE(4) CAPS_COMBINE(5) CAPS_COMBINE(6)
+        CAPS_COMBINE(7) CAPS_COMBINE(8) CAPS_COMBINE(9) CAPS_COMBINE(10) CAPS_COMBINE(11) CAPS_COMBINE(12)
+        CAPS_COMBINE(13) CAPS_COMBINE(14) CAPS_COMBINE(15) CAPS_COMBINE(16) CAPS_COMBINE(17)
+#undef CAPS_COMBINE
     }
 }
 
@@ -994,11 +1089,27 @@ cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitPa
                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     const int64_t units = (int64_t)((g.mtiles + 1) / 2) * g.rtiles * count;
-    int pairs = (int)(units < num_sms / 2 ? units : num_sms / 2);
+    int pairs = num_sms / 2;
     if (pairs > ZCTA_MAX / 2) pairs = ZCTA_MAX / 2;  // two product-residue tiles per CTA
+    // Whole units to a pair, or (unit, modulus) items and the combine kernel:
+    // items as long as every unit's residues fit the product-residue tiles.
+    // They fill the pairs evenly, and the combine kernel has the whole GPU
+    // where the drain warps of a few pairs end with 50000 clocks of
+    // reconstruction.  us a call at 17 moduli, units -> items: leaf of 448 (4
+    // units) 172 -> 76, of 1000 (16) 244 -> 125, of 2048 (64) 386 -> 339; 7
+    // leaves of 896 (112) 458 -> 394; 3 of 1792 (147, two full rounds of 76
+    // pairs) 1063 -> 1051.
+    const int split = units <= ZCTA_MAX;
     const size_t smem = (size_t)RNSTAGE * RSTAGE_BYTES + 1024 + 1024;
-    crt_gemm_kernel<<<2 * pairs, RGEMM_THREADS, smem, stream>>>(tasks_dev, (char *)workspace, g, planes, status_dev, starve);
+    const int64_t want = split ? units * LMAX : units;
+    if (want < pairs) pairs = (int)want;
+    crt_gemm_kernel<<<2 * pairs, RGEMM_THREADS, smem, stream>>>(tasks_dev, (char *)workspace, g, planes, status_dev, split,
+                                                                starve);
     count_launch();
+    if (split) {
+        crt_combine_kernel<<<(unsigned)(units * 2 * 64), 128, 0, stream>>>(tasks_dev, (char *)workspace, g);
+        count_launch();
+    }
     return cudaGetLastError();
 }
 

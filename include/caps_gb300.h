@@ -259,8 +259,8 @@ caps_status caps_autotune_entry(int index, int *n, int *form, int *nrec, char *p
  * as the leaves allow), the top step's b/d pattern and, for the split form
  * with an automatic scheme, residues against digits.  Its choices are kept
  * in CAPS_AUTOTUNE_CACHE (a file; empty: no cache) or by default in
- * $HOME/.cache/caps_gb300/autotune.tsv, keyed by the device's name and SM
- * count, the size, form, slices and asked-for scheme.  Any pointer may be
+ * $HOME/.cache/caps_gb300/autotune.tsv, keyed by the device's name, SM
+ * count and the library's kernels, the size, form, slices and asked-for scheme.  Any pointer may be
  * NULL.  caps_autotune_info gives every axis. */
 caps_status caps_autotune_entry_ex(int index, int *n, int *form, int *nrec, char *pattern, int *scheme,
                                    int *from_cache, double *seconds);
@@ -318,7 +318,8 @@ void caps_debug_starve_split_gemm(int count);
 /* Test hook for the autotuner's on-disk cache (host only, no device call):
  * 1 if `line`, one line of the cache file, holds a usable choice for size n
  * under (form, slices, split_scheme) on the device whose key is
- * `device_key` (the device name with blanks as '_', '/', its SM count), and
+ * `device_key` (the device name with blanks as '_', '/', its SM count, '/',
+ * the kernels' generation), and
  * then fills *out (if not NULL) as caps_autotune_info would; 0 for a line
  * of another version, device or size, or a damaged one (a field missing or
  * out of range, a pattern that is not nrec steps of 'b' / 'd'). */
