@@ -181,6 +181,7 @@ struct Builder {
     int overlap_stage = 0;      // 0: top step not built yet; 1: building its Q1; 2: no more waits
     bool overlap_extras = true; // the overlapped top step's one-pass sums and early Q5 (about
                                 // 10 quarter buffers more; dropped when the budget is short)
+    bool merge_small = false;   // run small 'd' steps as 'b' steps (see merges)
     int hybrid = 1;             // subproducts an 'h' step runs at once (desc.nproc_summa)
 
     size_t mark() const { return top; }
@@ -341,6 +342,21 @@ static void build_leaf(Builder &b, const std::vector<Prob> &P, int64_t m) {
     b.release(mk);
 }
 
+// A 'd' step runs its seven subproducts in sequence to hold 3 quarter buffers
+// a node instead of 11.  Where those are small the sequence only leaves the
+// GPU idle, launch after launch, and a 'b' step gives the same bits (per
+// element the same operations in the same order): with no budget in the way,
+// steps whose batch takes at most 128 MiB as 'b' steps run as such: one node of
+// quarters up to 1234 (split form, us a call, in sequence -> merged: n = 392
+// 'bd' 377 -> 143, n = 2048 'd' 750 -> 450, n = 2400 'd' 966 -> 735; at n = 4096 a
+// product of its own takes 85 % of the pairs).  Plain form: quarters up to 154
+// (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger leaves fill the FP64
+// pipe one at a time.
+static bool merges(const Builder &b, size_t nodes, int64_t h) {
+    if (!b.merge_small || (b.opt.form == CAPS_FORM_PLAIN && h > 154)) return false;
+    return (int64_t)nodes * 11 * h * h * (int64_t)sizeof(double) <= (int64_t)128 << 20;
+}
+
 static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, const char *pat) {
     if (nrec == 0) {
         build_leaf(b, P, n);
@@ -352,7 +368,10 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
     size_t mk = b.mark();
     std::vector<EwTask> st(P.size());
     const bool hyb = (c == 'h' || c == 'H') && b.hybrid >= 2;
-    if (c == 'b' || c == 'B' || hyb) {
+    // steps that overlap host copies (below) stay in sequence
+    const bool overlaps = b.host_overlap && P.size() == 1 &&
+                          ((b.overlap_stage == 0 && b.ops.empty()) || b.overlap_stage == 1);
+    if (c == 'b' || c == 'B' || hyb || (!overlaps && merges(b, P.size(), h))) {
         // strassenBFS (multiply.cpp:212-310) on one GPU: 7 subproducts as one
         // batch.  Q1..Q4 are written straight into the C quadrants (calcCij
         // reads all seven products of an element before writing any of its
@@ -478,11 +497,7 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
         // With a level below, Q1 runs the same way one level down (stage 1,
         // input events EV_INNER..+2 on the sub-quadrants of A11 and B11), so
         // the first products start after a quarter of A11 and B11 is in.
-        int stage = -1;
-        if (b.host_overlap && P.size() == 1) {
-            if (b.overlap_stage == 0 && b.ops.empty()) stage = 0;
-            else if (b.overlap_stage == 1) stage = 1;
-        }
+        const int stage = overlaps ? b.overlap_stage : -1;
         const bool top = stage == 0, lead = stage >= 0;
         const int ev = stage == 1 ? EV_INNER : 0;
         double *Q2top = lead ? b.alloc(q) : nullptr;
@@ -707,10 +722,11 @@ struct Planned {
 
 static caps_status plan(const double *A, const double *B, double *C, const caps_desc &d,
                         const char *pat, const caps_options &o, char *ws_base, Planned &pl,
-                        bool host_overlap = false, bool overlap_extras = true) {
+                        bool host_overlap = false, bool overlap_extras = true, bool merge_small = false) {
     pl.b = Builder();
     pl.b.host_overlap = host_overlap;
     pl.b.overlap_extras = overlap_extras;
+    pl.b.merge_small = merge_small;
     pl.b.ws_base = ws_base;
     pl.b.bs = d.bs;
     pl.b.hybrid = d.nproc_summa;
@@ -947,11 +963,15 @@ static caps_status multiply_dev_locked(const double *A, const double *B, double 
         auto_pattern(d, o, pat);
     }
     Planned pl;
-    bool extras = true;
-    CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras));
+    bool extras = true, merge = true;
+    CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras, merge));
+    if (o.workspace_limit > 0 && (long long)pl.ws_bytes > o.workspace_limit) {
+        merge = false;  // every step as the pattern has it
+        CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras, merge));
+    }
     if (host_overlap && o.workspace_limit > 0 && (long long)pl.ws_bytes > o.workspace_limit) {
         extras = false;  // the overlapped top step without its extra buffers
-        CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras));
+        CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras, merge));
     }
     if (o.workspace_limit > 0 && (long long)pl.ws_bytes > o.workspace_limit) {
         g_last_err = "workspace of the pattern exceeds the budget";
@@ -959,7 +979,7 @@ static caps_status multiply_dev_locked(const double *A, const double *B, double 
     }
     if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(status_buffer());
     CAPS_TRY(ensure(g_arena, pl.total));
-    CAPS_TRY(plan(A, B, C, d, pat, o, g_arena.ptr, pl, host_overlap, extras));
+    CAPS_TRY(plan(A, B, C, d, pat, o, g_arena.ptr, pl, host_overlap, extras, merge));
     double pt[3] = {0, 0, 0};
     long long l0 = g_launches;
     KernelTiming kt;
