@@ -186,100 +186,102 @@ void build_tables(CrtTables &t) {
 // conversion on the FMA pipe instead of the conversion unit.
 constexpr float MAGIC = 12582912.0f;
 
-__device__ __forceinline__ float small_int_to_float(int a) {  // |a| < 2^22
-    return __int_as_float(0x4B400000 + a) - MAGIC;
-}
-
 // Residues of X = round(x 2^f) modulo the first L moduli, balanced
 // (|r| <= 90).  X (|X| <= 2^55) is cut into four balanced 14-bit limbs a_k
 // (X + 8192 (1 + 2^14 + 2^28 + 2^42) has ordinary base-16384 digits
-// a_k + 8192; |a_k| <= 8192); then y = sum_k a_k (2^(14k) mod p), balanced,
-// has |y| < 2^21.1 and is exact in fp32, and r = y - p q with q = y * fl(1/p)
-// rounded to an integer by one fused multiply-add with MAGIC.  That product
-// is within |y / p| 2^-24 <= 2^-9.7 of y / p, while y / p lies at least
-// 1/(2p) >= 2^-8.5 from a half-integer (or exactly on one for p = 180, where
-// either neighbour gives |r| = 90), so q is a nearest integer and |r| <= p/2.
+// a_k + 8192; |a_k| <= 8192), or two where |X| <= 2^27; then y = sum_k a_k
+// (2^(14k) mod p), balanced, has |y| < 2^21.1 and is exact in fp32, and r = y -
+// p q with q = y * fl(1/p) rounded to an integer by one fused multiply-add with
+// MAGIC.  That product is within |y / p| 2^-24 <= 2^-9.7 of y / p, while y / p
+// lies at least 1/(2p) >= 2^-8.5 from a half-integer (or exactly on one for p =
+// 180, where either neighbour gives |r| = 90), so q is a nearest integer and
+// |r| <= p/2.
+template <int NL>
 struct Limbs {
-    float a[4];
+    float a[NL];
 };
 
+// a digit 0..16384 as the float digit - 8192
+__device__ __forceinline__ float balanced_digit(uint32_t d) {
+    return __uint_as_float(0x4B400000u | d) - (MAGIC + 8192.0f);
+}
+
 // The limbs of X = round(x 2^f) (ties to even; scaled_round in
-// split_common.cuh computes the same X), on 32-bit operations: from the two
-// halves of x's encoding (M 2^e, M below 2^53), q = M shifted by e + f, then
-// the base-16384 digits of X + 8192 (1 + 2^14 + 2^28 + 2^42) less 8192.  For
-// the slicer's f (t - E with E the row's exponent bound, t <= 55) the shift
-// e + f is at most 3.  Rounding right by r: q = M >> r, plus one when the bit
-// below q is set and a lower bit is set or q is odd.  Checked equal to the
-// 64-bit formulation on 40 million doubles and shifts, ties, subnormals and
-// zeros included; it takes fewer integer instructions.
-__device__ __forceinline__ Limbs scaled_limbs14(double x, int f) {
+// split_common.cuh computes the same X), on 32-bit operations and without
+// branches: for the slicer's f (t - E with E the row's exponent bound, t <=
+// 55) the shift of the significand M (M < 2^53, x = +-M 2^e) left by e + f is
+// at most 3, so M 2^3 is shifted right by 3 - e - f >= 0: first by a whole word
+// where that is 32 or more, then by the rest.  What falls out decides the
+// rounding: its top word, with the lowest bit set if any lower bit is.  Shifts
+// of 63 and more leave less than 2^-7 of a unit: 63.  Checked equal to
+// scaled_round on 60 million doubles and shifts, ties, carries, subnormals and
+// zeros included.
+template <int NL>
+__device__ __forceinline__ Limbs<NL> scaled_limbs14(double x, int f) {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
     const int field = (int)((hi >> 20) & 0x7FFu);
     const uint32_t mh = (hi & 0xFFFFFu) | (field ? 0x100000u : 0u);
-    const int sh = (field ? field - 1075 : -1074) + f;
-    uint32_t ql, qh;
-    if (sh >= 0) {  // at most 3
-        ql = lo << sh;
-        qh = __funnelshift_l(lo, mh, sh);
-    } else if (sh >= -53) {
-        const int r1 = -sh - 1;  // 0..52: M >> r1 ends in the round bit
-        uint32_t tl, th;
-        bool sticky;             // any bit below the round bit
-        if (r1 < 32) {
-            tl = __funnelshift_r(lo, mh, r1);
-            th = mh >> r1;
-            sticky = ((lo << (31 - r1)) << 1) != 0u;
-        } else {
-            tl = mh >> (r1 - 32);
-            th = 0u;
-            sticky = lo != 0u || ((mh << (63 - r1)) << 1) != 0u;
-        }
-        ql = __funnelshift_r(tl, th, 1);
-        qh = th >> 1;
-        const uint32_t up = tl & ((sticky ? 1u : 0u) | ql) & 1u;
-        ql += up;
-        qh += ql < up ? 1u : 0u;
-    } else {        // |x 2^f| < 1/2
-        ql = qh = 0u;
+    uint32_t vh = __funnelshift_l(lo, mh, 3), vl = lo << 3;  // M 2^3 < 2^56
+    const int r = min(1078 - max(field, 1) - f, 63);
+    const bool word = r >= 32;
+    const uint32_t out = word ? vl : 0u;  // the word shifted out whole
+    vl = word ? vh : vl;
+    vh = word ? 0u : vh;
+    // shift counts are modulo 32
+    const uint32_t rem = __funnelshift_r(out, vl, r) | (__funnelshift_r(0u, out, r) != 0u ? 1u : 0u);
+    uint32_t ql = __funnelshift_r(vl, vh, r), qh = vh >> (r & 31);
+    const uint32_t up = rem > 0x80000000u - (ql & 1u) ? 1u : 0u;
+    ql += up;
+    qh += ql < up ? 1u : 0u;
+    Limbs<NL> l;
+    const uint32_t s = (uint32_t)((int)hi >> 31);  // all ones for x < 0
+    if constexpr (NL == 2) {
+        const uint32_t u = (ql ^ s) - s + 0x08002000u;  // + 8192 (1 + 2^14)
+        l.a[0] = balanced_digit(u & 16383u);
+        l.a[1] = balanced_digit(u >> 14);
+    } else {
+        const uint64_t q = ((uint64_t)qh << 32) | ql, s64 = ((uint64_t)s << 32) | s;
+        const uint64_t U = (q ^ s64) - s64 + 0x0080020008002000ull;  // + 8192 sum_{k<4} 16384^k
+        const uint32_t ul = (uint32_t)U, uh = (uint32_t)(U >> 32);
+        l.a[0] = balanced_digit(ul & 16383u);
+        l.a[1] = balanced_digit((ul >> 14) & 16383u);
+        l.a[2] = balanced_digit(__funnelshift_r(ul, uh, 28) & 16383u);
+        l.a[3] = balanced_digit(uh >> 10);
     }
-    const uint64_t q = ((uint64_t)qh << 32) | ql;
-    const uint64_t OFF = 0x0080020008002000ull;  // 8192 * sum_{k<4} 16384^k
-    const uint64_t U = (hi >> 31) ? OFF - q : OFF + q;
-    const uint32_t ul = (uint32_t)U, uh = (uint32_t)(U >> 32);
-    Limbs l;
-    l.a[0] = small_int_to_float((int)(ul & 16383u) - 8192);
-    l.a[1] = small_int_to_float((int)((ul >> 14) & 16383u) - 8192);
-    l.a[2] = small_int_to_float((int)(__funnelshift_r(ul, uh, 28) & 16383u) - 8192);
-    l.a[3] = small_int_to_float((int)(uh >> 10) - 8192);
     return l;
 }
 
 // The balanced residues (|r| <= 90) of two values' integers modulo p_l, one
 // per lane, on packed fp32 pair instructions: each lane performs exactly
 // the scalar sequence y = a0 + a1 c0 + a2 c1 + a3 c2 (three fused
-// multiply-adds, innermost first), q = fl(y fl(1/p) + MAGIC) - MAGIC,
+// multiply-adds, exact), q = fl(y fl(1/p) + MAGIC) - MAGIC,
 // r = fl(y - q p), with round-to-nearest per lane as the scalar forms, at
 // half the issued instructions.
+template <int NL>
 struct Limbs2 {
-    float2 a[4];  // lane x: the first value's limbs, lane y: the second's
+    float2 a[NL];  // lane x: the first value's limbs, lane y: the second's
 };
 
-__device__ __forceinline__ Limbs2 pair_limbs(const Limbs &u, const Limbs &v) {
-    Limbs2 x;
+template <int NL>
+__device__ __forceinline__ Limbs2<NL> pair_limbs(const Limbs<NL> &u, const Limbs<NL> &v) {
+    Limbs2<NL> x;
 #pragma unroll
-    for (int k = 0; k < 4; k++) x.a[k] = make_float2(u.a[k], v.a[k]);
+    for (int k = 0; k < NL; k++) x.a[k] = make_float2(u.a[k], v.a[k]);
     return x;
 }
 
-__device__ __forceinline__ float2 reduce_pair(float2 y, int l) {
-    const float2 q = __fadd2_rn(__ffma2_rn(y, c_crt.invp2[l], make_float2(MAGIC, MAGIC)),
-                                make_float2(-MAGIC, -MAGIC));
-    return __ffma2_rn(q, c_crt.np2[l], y);
+__device__ __forceinline__ float2 reduce_pair(float2 y, float2 invp, float2 np) {
+    const float2 q = __fadd2_rn(__ffma2_rn(y, invp, make_float2(MAGIC, MAGIC)), make_float2(-MAGIC, -MAGIC));
+    return __ffma2_rn(q, np, y);
 }
+__device__ __forceinline__ float2 reduce_pair(float2 y, int l) { return reduce_pair(y, c_crt.invp2[l], c_crt.np2[l]); }
 
-__device__ __forceinline__ float2 residue_pair(const Limbs2 &x, int l) {
+template <int NL>
+__device__ __forceinline__ float2 residue_pair(const Limbs2<NL> &x, int l) {
     const float2 *c = c_crt.c2[l];
-    return reduce_pair(__ffma2_rn(x.a[3], c[2], __ffma2_rn(x.a[2], c[1], __ffma2_rn(x.a[1], c[0], x.a[0]))), l);
+    float2 y = __ffma2_rn(x.a[1], c[0], x.a[0]);
+    if constexpr (NL == 4) y = __ffma2_rn(x.a[3], c[2], __ffma2_rn(x.a[2], c[1], y));
+    return reduce_pair(y, l);
 }
 
 // the same for the integers times y_l (the CRT coefficient of modulus l among
@@ -287,11 +289,15 @@ __device__ __forceinline__ float2 residue_pair(const Limbs2 &x, int l) {
 // y_l A'B' mod p_l, the term the CRT needs.  |y| <= 4 * 8192 * 90 < 2^21.5,
 // so y / p is within 2^-9.3 of y * fl(1/p), still inside the half-integer
 // margin of 2^-8.5.
-__device__ __forceinline__ float2 residue_y_pair(const Limbs2 &x, int L, int l) {
-    const float2 *cy = c_crt.cy2[L - 1][l];
-    return reduce_pair(
-        __ffma2_rn(x.a[3], cy[3], __ffma2_rn(x.a[2], cy[2], __ffma2_rn(x.a[1], cy[1], __fmul2_rn(x.a[0], cy[0])))),
-        l);
+template <int NL>
+__device__ __forceinline__ float2 weigh_pair(const Limbs2<NL> &x, const float2 *c) {
+    const float2 y = __ffma2_rn(x.a[1], c[1], __fmul2_rn(x.a[0], c[0]));
+    if constexpr (NL == 4) return __ffma2_rn(x.a[3], c[3], __ffma2_rn(x.a[2], c[2], y));
+    return y;
+}
+template <int NL>
+__device__ __forceinline__ float2 residue_y_pair(const Limbs2<NL> &x, int L, int l) {
+    return reduce_pair(weigh_pair(x, c_crt.cy2[L - 1][l]), l);
 }
 
 // two residues as packed bf16: |r| <= 90 has at most 7 significant bits, so
@@ -319,25 +325,24 @@ int crt_moduli_needed(int bits, int K) {
 }
 
 // ---------------------------------------------------------------- slice
-// The residues of 4 pairs of values modulo each of the first NL moduli (A
-// side: premultiplied by the CRT coefficients of NL moduli), 8 bf16 per plane.
-template <int NL>
-__device__ __forceinline__ void write_residues_unrolled(const Limbs2 (&x)[4], char *dst, size_t plane_stride,
-                                                        int side) {
+// The residues of 4 pairs of values modulo each of the first L moduli (A
+// side: premultiplied by the CRT coefficients of L moduli), 8 bf16 per plane.
+template <int L, int NL>
+__device__ __forceinline__ void write_residues(const Limbs2<NL> (&x)[4], char *dst, size_t plane_stride, int side) {
     if (side == 0) {
 #pragma unroll
-        for (int l = 0; l < NL; l++) {
+        for (int l = 0; l < L; l++) {
             uint32_t w[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const float2 r = residue_y_pair(x[q], NL, l);
+                const float2 r = residue_y_pair(x[q], L, l);
                 w[q] = pack_bf16x2(r.x, r.y);
             }
             *reinterpret_cast<uint4 *>(dst + (size_t)l * plane_stride) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     } else {
 #pragma unroll
-        for (int l = 0; l < NL; l++) {
+        for (int l = 0; l < L; l++) {
             uint32_t w[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -349,6 +354,38 @@ __device__ __forceinline__ void write_residues_unrolled(const Limbs2 (&x)[4], ch
     }
 }
 
+// The same for a modulus count known at run time, from the constants of one
+// side in shared memory (a few wide loads a modulus, the same for all lanes).
+// Compiled per count as well, the cases' common work was hoisted above the
+// branch and spilled.
+struct __align__(16) SliceConst {
+    float2 c[4];  // A: 2^(14k) y_l mod p_l; B: 2^(14k) mod p_l (the first is 1)
+    float2 invp, np;
+};
+
+template <int NL>
+__device__ __forceinline__ void write_residues_counted(const Limbs2<NL> (&x)[4], int L, const SliceConst *consts,
+                                                       char *dst, size_t plane_stride) {
+#pragma unroll 1
+    for (int l = 0; l < L; l++) {
+        const SliceConst k = consts[l];
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float2 r = reduce_pair(weigh_pair(x[q], k.c), k.invp, k.np);
+            w[q] = pack_bf16x2(r.x, r.y);
+        }
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        dst += plane_stride;
+    }
+}
+
+template <int NL>
+__device__ __forceinline__ void limbs_of(const double (&v)[8], int f, Limbs2<NL> (&x)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) x[q] = pair_limbs(scaled_limbs14<NL>(v[2 * q], f), scaled_limbs14<NL>(v[2 * q + 1], f));
+}
+
 // Residue planes, per modulus l: [l][row tile][ks] for A, [l][column tile][ks]
 // for B, tiles of 128 x 16 (4 KiB), each the UMMA canonical K-major image
 // (8-row x 16-byte core matrices, K halves side by side: K stride 128 B,
@@ -356,7 +393,7 @@ __device__ __forceinline__ void write_residues_unrolled(const Limbs2 (&x)[4], ch
 // block = one tile.
 __device__ __forceinline__ void crt_slice_tile(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
                                                const Geo &g, const SplitHdr *h, int L, int leaf, int64_t tile,
-                                               int side) {
+                                               int side, const SliceConst *consts) {
     const int tiles = side == 0 ? g.mtiles : 2 * g.rtiles;
     if (tile >= (int64_t)tiles * g.nks) return;
     const LeafTask t = tasks[leaf];
@@ -377,42 +414,65 @@ __device__ __forceinline__ void crt_slice_tile(const LeafTask *__restrict__ task
     const bool live = idx < M && ee != 0;
     const int f = tt - (ee - 4096);
     double v[8];
+    if (side == 1 && live && k0 + 8 <= M && ((uintptr_t)src & 15) == 0) {
+        // a column's 8 values lie side by side: 16-byte loads
 #pragma unroll
-    for (int e = 0; e < 8; e++) v[e] = (live && k0 + e < M) ? __ldg(src + e * sk) : 0.0;
-    Limbs2 x[4];
+        for (int e = 0; e < 8; e += 2) {
+            const double2 w = __ldg(reinterpret_cast<const double2 *>(src + e));
+            v[e] = w.x;
+            v[e + 1] = w.y;
+        }
+    } else {
 #pragma unroll
-    for (int q = 0; q < 4; q++) x[q] = pair_limbs(scaled_limbs14(v[2 * q], f), scaled_limbs14(v[2 * q + 1], f));
-    switch (L) {
+        for (int e = 0; e < 8; e++) v[e] = (live && k0 + e < M) ? __ldg(src + e * sk) : 0.0;
+    }
+    if (L >= 15) {
         // float data need 17 moduli at 55 bits, 16 or 15 under an operand-bit
-        // cap: unrolled, the constants' addresses are fixed, with no
-        // per-modulus address arithmetic or loop bookkeeping
-        case 17: write_residues_unrolled<17>(x, dst, plane_stride, side); break;
-        case 16: write_residues_unrolled<16>(x, dst, plane_stride, side); break;
-        case 15: write_residues_unrolled<15>(x, dst, plane_stride, side); break;
-        default:
-#pragma unroll 1
-            for (int l = 0; l < L; l++) {
-                uint32_t w[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float2 r = side == 0 ? residue_y_pair(x[q], L, l) : residue_pair(x[q], l);
-                    w[q] = pack_bf16x2(r.x, r.y);
-                }
-                *reinterpret_cast<uint4 *>(dst + (size_t)l * plane_stride) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
+        // cap or at short K: compiled for these
+        Limbs2<4> x[4];
+        limbs_of(v, f, x);
+        switch (L) {
+            case 17: write_residues<17>(x, dst, plane_stride, side); break;
+            case 16: write_residues<16>(x, dst, plane_stride, side); break;
+            case 15: write_residues<15>(x, dst, plane_stride, side); break;
+        }
+    } else if (tt <= 27) {
+        Limbs2<2> x[4];
+        limbs_of(v, f, x);
+        write_residues_counted(x, L, consts, dst, plane_stride);
+    } else {
+        Limbs2<4> x[4];
+        limbs_of(v, f, x);
+        write_residues_counted(x, L, consts, dst, plane_stride);
     }
 }
 
-// Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).
-__global__ void __launch_bounds__(256) crt_slice_kernel(const LeafTask *__restrict__ tasks,
+// Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).  Bound by HBM at
+// 17 moduli (49 leaves of 2048: 2.73 ms, 0.93 of the copy rate) and by its
+// instructions at few moduli, where the limbs are most of the work: rounding
+// without branches, two limbs for operands of up to 27 bits, 16-byte loads of
+// B and 5 blocks an SM took 49 leaves of 1024 at 6 moduli from 508 to 364 us
+// (0.83 of the copy rate), 7 leaves of 896 at 17 from 86 to 81.
+__global__ void __launch_bounds__(256, 5) crt_slice_kernel(const LeafTask *__restrict__ tasks,
                                                         char *__restrict__ ws, Geo g) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int L = h->moduli;
+    __shared__ SliceConst consts[LMAX];
+    if (threadIdx.x < L) {
+        const int l = threadIdx.x;
+        SliceConst k;
+        for (int i = 0; i < 4; i++)
+            k.c[i] = blockIdx.y == 0 ? c_crt.cy2[L - 1][l][i] : i == 0 ? make_float2(1.f, 1.f) : c_crt.c2[l][i - 1];
+        k.invp = c_crt.invp2[l];
+        k.np = c_crt.np2[l];
+        consts[l] = k;
+    }
+    __syncthreads();
     const int64_t atiles = (int64_t)g.mtiles * g.nks, btiles = (int64_t)g.rtiles * g.nks * 2;
     const int64_t per = atiles > btiles ? atiles : btiles;
     const int64_t total = per * g.count;
     for (int64_t it = blockIdx.x; it < total; it += gridDim.x)
-        crt_slice_tile(tasks, ws, g, h, L, (int)(it / per), it % per, blockIdx.y);
+        crt_slice_tile(tasks, ws, g, h, L, (int)(it / per), it % per, blockIdx.y, consts);
 }
 
 // ---------------------------------------------------------------- CRT reconstruction
