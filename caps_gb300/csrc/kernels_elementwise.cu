@@ -239,9 +239,11 @@ template <int OP>
 static void launch_op(bool vec, const EwTask *tasks, int count, int64_t q, cudaStream_t s) {
     const int threads = 256;
     int64_t work = vec ? (q >> 1) : q;
-    // enough blocks to cover ~4 waves of the 152 SMs across all tasks
+    // a grid stride of up to ~32 waves of the 152 SMs across all tasks: short
+    // blocks even out at the end (n = 16384 integers 'bbdd', ~300 launches:
+    // 94.1 ms at 4 waves, 92.2 at 32; larger multiplies do not change)
     int64_t want = (work + threads - 1) / threads;
-    int64_t cap = (int64_t)152 * 8 * 4 / (count > 0 ? count : 1);
+    int64_t cap = (int64_t)152 * 8 * 32 / (count > 0 ? count : 1);
     if (cap < 1) cap = 1;
     if (want > cap) want = cap;
     if (want < 1) want = 1;
@@ -292,18 +294,47 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
 //
 // A block column is a run of bs consecutive doubles in the CAPS layout and
 // bs consecutive rows of one column of the column-major matrix: the reorder
-// is a copy of n^2 / bs runs.  A warp copies one run (runs of 32 and more:
+// is a copy of n^2 / bs runs.  A warp copies one run (runs of RUN_MIN and more:
 // the leaf columns when bs is 1 or the leaf, which is the workloads' case),
 // with 16-byte accesses when both ends of the run are 16-byte aligned; the
 // run's position is worked out once per run from its index (the quadrant
 // digits of its leaf, its block and column).  Shorter runs take one thread
-// per element.  HBM-bound either way: 16 bytes moved per element.
+// per element, or per pair where bs is even and the matrices are aligned.
+// HBM-bound either way, 16 bytes moved per element, with 8 (runs) or 4 loads
+// issued before their stores and the positions on 32-bit operations (runs: one
+// load in flight; elements: 64-bit divisions, before).  us one way at n = 8192
+// (copy rate: 158), before -> here: bs 1 in leaves of 1024 197 -> 158, n = 8191
+// 340 -> 170, bs 16 573 -> 183, bs 32 570 -> 176, bs 64 299 -> 176; n = 6272 in bs 7
+// 340 -> 152 (93).  Runs of 128 as elements take 172 against 221, of 250 as
+// runs 160 against 174, hence RUN_MIN.
 // ---------------------------------------------------------------------------
+constexpr int RUN_BATCH = 8;  // loads a lane has in flight
+constexpr int RUN_MIN = 160;  // runs from here on take a warp each
+
+// x / d for 0 <= x < 2^31 by a multiplication (Granlund and Montgomery's
+// invariant division): with s = ceil(log2 d), m = floor(2^32 (2^s - d) / d) + 1,
+// x / d = (umulhi(m, x) + x) >> s.
+struct FastDiv {
+    uint32_t d, m, s;
+    __device__ __forceinline__ uint32_t div(uint32_t x) const { return (__umulhi(m, x) + x) >> s; }
+};
+
+static FastDiv fast_div(int64_t d) {
+    FastDiv f;
+    f.d = (uint32_t)d;
+    f.s = 0;
+    while (((int64_t)1 << f.s) < d) f.s++;
+    f.m = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << f.s) - (uint64_t)d)) / (uint64_t)d + 1);
+    return f;
+}
+
 struct ReorderGeom {
     int64_t n, m, mm;   // matrix, leaf, leaf^2
     int nrec;
     int bs;             // effective block size (m when bs == 1 or bs == m)
     int nb;             // blocks per leaf side
+    bool small;         // n^2 < 2^31: the divisions below
+    FastDiv dbs, dnb, druns;  // by bs, nb and the runs of a leaf
 };
 
 // column-major offset of the first element of run `run` (run = leaf * (mm /
@@ -331,6 +362,20 @@ __device__ __forceinline__ int64_t caps_to_colmajor_index(const ReorderGeom &g, 
     return run_colmajor_offset(g, run) + (idx - run * g.bs);
 }
 
+// A run by a warp, in batches of loads issued before their stores.
+template <typename T>
+__device__ __forceinline__ void copy_run(const T *__restrict__ s, T *__restrict__ d, int count, int lane) {
+    for (int k = lane; k < count; k += 32 * RUN_BATCH) {
+        T v[RUN_BATCH];
+#pragma unroll
+        for (int b = 0; b < RUN_BATCH; b++)
+            if (k + 32 * b < count) v[b] = __ldcs(s + k + 32 * b);
+#pragma unroll
+        for (int b = 0; b < RUN_BATCH; b++)
+            if (k + 32 * b < count) __stcs(d + k + 32 * b, v[b]);
+    }
+}
+
 // one warp per run of bs >= 32 doubles
 template <bool TO_CAPS>
 __device__ __forceinline__ void reorder_runs(const double *__restrict__ s, double *__restrict__ d,
@@ -342,11 +387,50 @@ __device__ __forceinline__ void reorder_runs(const double *__restrict__ s, doubl
         const double *src = s + (TO_CAPS ? cm : cp);
         double *dst = d + (TO_CAPS ? cp : cm);
         if (((g.bs & 1) == 0) && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
-            const double2 *s2 = reinterpret_cast<const double2 *>(src);
-            double2 *d2 = reinterpret_cast<double2 *>(dst);
-            for (int64_t k = lane; k < g.bs / 2; k += 32) __stcs(d2 + k, __ldcs(s2 + k));
+            copy_run(reinterpret_cast<const double2 *>(src), reinterpret_cast<double2 *>(dst), g.bs / 2, lane);
         } else {
-            for (int64_t k = lane; k < g.bs; k += 32) __stcs(dst + k, __ldcs(src + k));
+            copy_run(src, dst, g.bs, lane);
+        }
+    }
+}
+
+// the same on 32-bit operations (64-bit divisions are several times the copy)
+__device__ __forceinline__ uint32_t caps_to_colmajor_index32(const ReorderGeom &g, uint32_t idx) {
+    const uint32_t run = g.dbs.div(idx), leaf = g.druns.div(run), rest = run - leaf * g.druns.d;
+    const uint32_t blk = g.dbs.div(rest), cc = rest - blk * g.dbs.d;
+    const uint32_t bi = g.dnb.div(blk), bj = blk - bi * g.dnb.d;  // block column, block row
+    uint32_t r = bj * g.dbs.d + (idx - run * g.dbs.d), c = bi * g.dbs.d + cc;
+    uint32_t h = (uint32_t)g.m;
+    for (uint32_t l = leaf, k = 0; k < (uint32_t)g.nrec; k++, l >>= 2, h *= 2) {
+        r += (l & 1) * h;
+        c += ((l >> 1) & 1) * h;
+    }
+    return r + c * (uint32_t)g.n;
+}
+
+// T: double, or double2 where bs is even and both matrices are 16-byte aligned
+// (then every pair of a run is, on both sides)
+template <bool TO_CAPS, typename T>
+__device__ __forceinline__ void reorder_elements32(const double *__restrict__ s, double *__restrict__ d,
+                                                   const ReorderGeom &g, int64_t t0, int64_t nthreads) {
+    constexpr int W = sizeof(T) / sizeof(double), B = 4;
+    const int64_t total = g.n * g.n / W;
+    // four units a thread and pass, their loads before their stores
+    for (int64_t base = t0; base < total; base += B * nthreads) {
+        T v[B];
+        uint32_t cm[B];
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            const int64_t u = base + b * nthreads;
+            if (u < total) {
+                cm[b] = caps_to_colmajor_index32(g, (uint32_t)u * W);
+                v[b] = __ldcs(reinterpret_cast<const T *>(s + (TO_CAPS ? cm[b] : (uint32_t)u * W)));
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+            const int64_t u = base + b * nthreads;
+            if (u < total) *reinterpret_cast<T *>(d + (TO_CAPS ? (uint32_t)u * W : cm[b])) = v[b];
         }
     }
 }
@@ -355,6 +439,13 @@ template <bool TO_CAPS>
 __device__ __forceinline__ void reorder_elements(const double *__restrict__ s, double *__restrict__ d,
                                                  const ReorderGeom &g, int64_t t0, int64_t nthreads) {
     const int64_t total = g.n * g.n;
+    if (g.small) {
+        if ((g.bs & 1) == 0 && (((uintptr_t)s | (uintptr_t)d) & 15) == 0)
+            reorder_elements32<TO_CAPS, double2>(s, d, g, t0, nthreads);
+        else
+            reorder_elements32<TO_CAPS, double>(s, d, g, t0, nthreads);
+        return;
+    }
     for (int64_t idx = t0; idx < total; idx += nthreads) {
         int64_t cm = caps_to_colmajor_index(g, idx);
         if (TO_CAPS)
@@ -370,7 +461,7 @@ __global__ void __launch_bounds__(256) reorder_kernel(const double *const *__res
                                                       ReorderGeom g) {
     const double *s = src[blockIdx.y];
     double *d = dst[blockIdx.y];
-    if (g.bs >= 32)
+    if (g.bs >= RUN_MIN)
         reorder_runs<TO_CAPS>(s, d, g, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                               ((int64_t)gridDim.x * blockDim.x) >> 5);
     else
@@ -386,15 +477,19 @@ static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
     g.mm = g.m * g.m;
     g.bs = (bs == 1 || bs == g.m) ? (int)g.m : (int)bs;
     g.nb = (int)(g.m / g.bs);
+    g.small = n * n < ((int64_t)1 << 31);
+    g.dbs = fast_div(g.bs);
+    g.dnb = fast_div(g.nb);
+    g.druns = fast_div(g.small ? g.mm / g.bs : 1);
     return g;
 }
 
 // grid: enough blocks for a run (or element) per thread, at most 8 blocks of
 // 256 threads per SM for all matrices together
 static unsigned reorder_blocks(const ReorderGeom &g, int count) {
-    const int64_t items = g.bs >= 32 ? g.n * g.n / g.bs * 32 : g.n * g.n;
+    const int64_t items = g.bs >= RUN_MIN ? g.n * g.n / g.bs * 32 : g.n * g.n;
     int64_t blocks = (items + 255) / 256;
-    int64_t cap = (int64_t)152 * 8 / count;
+    int64_t cap = (int64_t)152 * 32 / count;
     if (cap < 1) cap = 1;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
@@ -417,7 +512,7 @@ cudaError_t launch_reorder(const double *const *src_dev, double *const *dst_dev,
 template <bool TO_CAPS>
 __global__ void __launch_bounds__(256) reorder_one_kernel(const double *__restrict__ s,
                                                           double *__restrict__ d, ReorderGeom g) {
-    if (g.bs >= 32)
+    if (g.bs >= RUN_MIN)
         reorder_runs<TO_CAPS>(s, d, g, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                               ((int64_t)gridDim.x * blockDim.x) >> 5);
     else
