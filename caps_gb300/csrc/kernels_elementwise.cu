@@ -8,7 +8,7 @@
 // All of these are HBM-bound streams: 8 bytes per element per operand.  A
 // block handles one task (blockIdx.y) and a grid-stride range of elements;
 // when every pointer of the launch is 16-byte aligned and q is even, the
-// loop moves double2 vectors.
+// loop moves double2 vectors, otherwise two elements 256 apart.
 #include "common.cuh"
 
 namespace caps {
@@ -83,131 +83,95 @@ __host__ __device__ constexpr bool lean_reads(int k) {
                                 : (k == 0 || k == 1 || k == 2 || k == 3);
 }
 
-template <int OP>
-__device__ __forceinline__ void ew_scalar(const EwTask &t, int64_t i) {
-    if (OP == EW_FORM_ST) {
-        double o[8];
-        form_st(t.src[0][i], t.src[1][i], t.src[2][i], t.src[3][i], t.src[4][i], t.src[5][i],
-                t.src[6][i], t.src[7][i], o);
-#pragma unroll
-        for (int k = 0; k < 8; k++) t.dst[k][i] = o[k];
-    } else if (OP == EW_COPY) {
-        t.dst[0][i] = t.src[0][i];
-    } else if (OP == EW_ADD_DUP) {
-        double v = t.src[0][i] + t.src[1][i];
-        t.dst[0][i] = v;
-        t.dst[1][i] = v;
-    } else if (OP == EW_ADD) {
-        t.dst[0][i] = t.src[0][i] + t.src[1][i];
-    } else if (OP == EW_SUB) {
-        t.dst[0][i] = t.src[0][i] - t.src[1][i];
-    } else if (OP == EW_ADD2) {
-        double q = t.src[2][i];
-        double a = t.src[0][i] + q;
-        double b = t.src[1][i] + q;
-        t.dst[0][i] = a;
-        t.dst[1][i] = b;
-    } else if (OP == EW_CALC_CIJ) {
-        double q[7], c[4];
-#pragma unroll
-        for (int k = 0; k < 7; k++) q[k] = t.src[k][i];
-        calc_cij(q, c);
-#pragma unroll
-        for (int k = 0; k < 4; k++) t.dst[k][i] = c[k];
-    } else if (OP >= EW_FORM_T4S4 && OP <= EW_FORM_T6) {
-        double v[8], o0, o1;
-#pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = lean_reads<OP>(k) ? t.src[k][i] : 0.0;
-        form_lean<OP>(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], o0, o1);
-        t.dst[0][i] = o0;
-        if (OP <= EW_FORM_T3S3) t.dst[1][i] = o1;
-    } else if (OP == EW_U2_Q3) {
-        double u2 = t.src[0][i], u1 = t.src[1][i], q = t.src[2][i];
-        t.dst[0][i] = u2;
-        t.dst[1][i] = u2 + q;
-        t.dst[2][i] = u1 + q;
+// Two elements of a stream: a 16-byte vector (i counts vectors), or, where the
+// launch is not aligned for that, elements i and i + 256 (the second only if
+// `two`) -- either way both loads of every source come before the stores.
+template <bool VEC>
+__device__ __forceinline__ double2 ld2(const double *p, int64_t i, bool two) {
+    if constexpr (VEC) return __ldcs(reinterpret_cast<const double2 *>(p) + i);
+    else return make_double2(__ldcs(p + i), two ? __ldcs(p + i + 256) : 0.0);
+}
+template <bool VEC>
+__device__ __forceinline__ void st2(double *p, int64_t i, bool two, double2 v) {
+    if constexpr (VEC) {
+        __stcs(reinterpret_cast<double2 *>(p) + i, v);
+    } else {
+        __stcs(p + i, v.x);
+        if (two) __stcs(p + i + 256, v.y);
     }
 }
 
-__device__ __forceinline__ double2 ld2(const double *p, int64_t i) {
-    return __ldcs(reinterpret_cast<const double2 *>(p) + i);
-}
-__device__ __forceinline__ void st2(double *p, int64_t i, double2 v) {
-    __stcs(reinterpret_cast<double2 *>(p) + i, v);
-}
-
-template <int OP>
-__device__ __forceinline__ void ew_vec2(const EwTask &t, int64_t i) {
-    // i indexes double2 vectors; the two lanes are independent elements.
+template <int OP, bool VEC>
+__device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
+    // the two lanes are independent elements
     if (OP == EW_FORM_ST) {
         double2 v[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = ld2(t.src[k], i);
+        for (int k = 0; k < 8; k++) v[k] = ld2<VEC>(t.src[k], i, two);
         double o0[8], o1[8];
         form_st(v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, v[5].x, v[6].x, v[7].x, o0);
         form_st(v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y, v[6].y, v[7].y, o1);
 #pragma unroll
-        for (int k = 0; k < 8; k++) st2(t.dst[k], i, make_double2(o0[k], o1[k]));
+        for (int k = 0; k < 8; k++) st2<VEC>(t.dst[k], i, two, make_double2(o0[k], o1[k]));
     } else if (OP == EW_CALC_CIJ) {
         double2 v[7];
 #pragma unroll
-        for (int k = 0; k < 7; k++) v[k] = ld2(t.src[k], i);
+        for (int k = 0; k < 7; k++) v[k] = ld2<VEC>(t.src[k], i, two);
         double q0[7], q1[7], c0[4], c1[4];
 #pragma unroll
         for (int k = 0; k < 7; k++) { q0[k] = v[k].x; q1[k] = v[k].y; }
         calc_cij(q0, c0);
         calc_cij(q1, c1);
 #pragma unroll
-        for (int k = 0; k < 4; k++) st2(t.dst[k], i, make_double2(c0[k], c1[k]));
+        for (int k = 0; k < 4; k++) st2<VEC>(t.dst[k], i, two, make_double2(c0[k], c1[k]));
     } else if (OP == EW_COPY) {
-        st2(t.dst[0], i, ld2(t.src[0], i));
+        st2<VEC>(t.dst[0], i, two, ld2<VEC>(t.src[0], i, two));
     } else if (OP == EW_ADD_DUP) {
-        double2 a = ld2(t.src[0], i), b = ld2(t.src[1], i);
+        double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
         double2 r = make_double2(a.x + b.x, a.y + b.y);
-        st2(t.dst[0], i, r);
-        st2(t.dst[1], i, r);
+        st2<VEC>(t.dst[0], i, two, r);
+        st2<VEC>(t.dst[1], i, two, r);
     } else if (OP == EW_ADD) {
-        double2 a = ld2(t.src[0], i), b = ld2(t.src[1], i);
-        st2(t.dst[0], i, make_double2(a.x + b.x, a.y + b.y));
+        double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
+        st2<VEC>(t.dst[0], i, two, make_double2(a.x + b.x, a.y + b.y));
     } else if (OP == EW_SUB) {
-        double2 a = ld2(t.src[0], i), b = ld2(t.src[1], i);
-        st2(t.dst[0], i, make_double2(a.x - b.x, a.y - b.y));
+        double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
+        st2<VEC>(t.dst[0], i, two, make_double2(a.x - b.x, a.y - b.y));
     } else if (OP == EW_ADD2) {
-        double2 a = ld2(t.src[0], i), b = ld2(t.src[1], i), q = ld2(t.src[2], i);
+        double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two), q = ld2<VEC>(t.src[2], i, two);
         double2 r0 = make_double2(a.x + q.x, a.y + q.y);
         double2 r1 = make_double2(b.x + q.x, b.y + q.y);
-        st2(t.dst[0], i, r0);
-        st2(t.dst[1], i, r1);
+        st2<VEC>(t.dst[0], i, two, r0);
+        st2<VEC>(t.dst[1], i, two, r1);
     } else if (OP >= EW_FORM_T4S4 && OP <= EW_FORM_T6) {
         // only the sources the formula reads are loaded
         double2 v[8];
 #pragma unroll
         for (int k = 0; k < 8; k++)
-            v[k] = lean_reads<OP>(k) ? ld2(t.src[k], i) : make_double2(0.0, 0.0);
+            v[k] = lean_reads<OP>(k) ? ld2<VEC>(t.src[k], i, two) : make_double2(0.0, 0.0);
         double a0, a1, b0, b1;
         form_lean<OP>(v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, v[5].x, v[6].x, v[7].x, a0, a1);
         form_lean<OP>(v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y, v[6].y, v[7].y, b0, b1);
-        st2(t.dst[0], i, make_double2(a0, b0));
-        if (OP <= EW_FORM_T3S3) st2(t.dst[1], i, make_double2(a1, b1));
+        st2<VEC>(t.dst[0], i, two, make_double2(a0, b0));
+        if (OP <= EW_FORM_T3S3) st2<VEC>(t.dst[1], i, two, make_double2(a1, b1));
     } else if (OP == EW_U2_Q3) {
-        double2 u2 = ld2(t.src[0], i), u1 = ld2(t.src[1], i), q = ld2(t.src[2], i);
-        st2(t.dst[0], i, u2);
-        st2(t.dst[1], i, make_double2(u2.x + q.x, u2.y + q.y));
-        st2(t.dst[2], i, make_double2(u1.x + q.x, u1.y + q.y));
+        double2 u2 = ld2<VEC>(t.src[0], i, two), u1 = ld2<VEC>(t.src[1], i, two), q = ld2<VEC>(t.src[2], i, two);
+        st2<VEC>(t.dst[0], i, two, u2);
+        st2<VEC>(t.dst[1], i, two, make_double2(u2.x + q.x, u2.y + q.y));
+        st2<VEC>(t.dst[2], i, two, make_double2(u1.x + q.x, u1.y + q.y));
     }
 }
 
 template <int OP, bool VEC>
 __global__ void __launch_bounds__(256) ew_kernel(const EwTask *__restrict__ tasks, int64_t q) {
     const EwTask t = tasks[blockIdx.y];
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     if (VEC) {
-        const int64_t nv = q >> 1;
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride)
-            ew_vec2<OP>(t, i);
+        const int64_t nv = q >> 1, stride = (int64_t)gridDim.x * 256;
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nv; i += stride) ew_pair<OP, true>(t, i, true);
     } else {
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q; i += stride)
-            ew_scalar<OP>(t, i);
+        const int64_t stride = (int64_t)gridDim.x * 512;
+        for (int64_t i = (int64_t)blockIdx.x * 512 + threadIdx.x; i < q; i += stride)
+            ew_pair<OP, false>(t, i, i + 256 < q);
     }
 }
 
@@ -238,12 +202,13 @@ int ew_dests(int op) { return ew_ndst(op); }
 template <int OP>
 static void launch_op(bool vec, const EwTask *tasks, int count, int64_t q, cudaStream_t s) {
     const int threads = 256;
-    int64_t work = vec ? (q >> 1) : q;
+    const int64_t work = (q + 1) / 2;
     // a grid stride of up to ~32 waves of the 152 SMs across all tasks: short
     // blocks even out at the end (n = 16384 integers 'bbdd', ~300 launches:
-    // 94.1 ms at 4 waves, 92.2 at 32; larger multiplies do not change)
+    // 94.1 ms at 4 waves, 92.2 at 32; larger multiplies do not change).
+    // Unaligned launches stay at 4 (7 products of 2671: 5 us faster than at 32).
     int64_t want = (work + threads - 1) / threads;
-    int64_t cap = (int64_t)152 * 8 * 32 / (count > 0 ? count : 1);
+    int64_t cap = (int64_t)152 * 8 * (vec ? 32 : 4) / (count > 0 ? count : 1);
     if (cap < 1) cap = 1;
     if (want > cap) want = cap;
     if (want < 1) want = 1;

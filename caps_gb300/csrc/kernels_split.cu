@@ -122,6 +122,52 @@ __device__ __forceinline__ void scan_value(double x, int &emax, int &lmin) {
     }
 }
 
+__device__ __forceinline__ void scan_value(double2 v, int &emax, int &lmin) {
+    scan_value(v.x, emax, lmin);
+    scan_value(v.y, emax, lmin);
+}
+
+// Two adjacent rows over n columns, `step` apart.
+template <bool PAIR>
+__device__ __forceinline__ void scan_columns(const double *col, int64_t step, int n, bool two, int &e0, int &l0, int &e1,
+                                             int &l1) {
+    auto load = [&](const double *p) {
+        if constexpr (PAIR) return __ldg(reinterpret_cast<const double2 *>(p));
+        else return make_double2(__ldg(p), two ? __ldg(p + 1) : 0.0);
+    };
+    int k = 0;
+    for (; k + SCAN_BATCH <= n; k += SCAN_BATCH) {
+        double2 v[SCAN_BATCH];
+#pragma unroll
+        for (int b = 0; b < SCAN_BATCH; b++, col += step) v[b] = load(col);
+#pragma unroll
+        for (int b = 0; b < SCAN_BATCH; b++) {
+            scan_value(v[b].x, e0, l0);
+            scan_value(v[b].y, e1, l1);
+        }
+    }
+    for (; k < n; k++, col += step) {
+        const double2 v = load(col);
+        scan_value(v.x, e0, l0);
+        scan_value(v.y, e1, l1);
+    }
+}
+
+// A column's n units, by a warp.
+template <typename T>
+__device__ __forceinline__ void scan_run(const T *col, int n, int lane, int &emax, int &lmin) {
+    const T *p = col + lane;
+    int k = lane;
+    for (; k + 32 * (SCAN_BATCH - 1) < n; k += 32 * SCAN_BATCH, p += 32 * SCAN_BATCH) {
+        T v[SCAN_BATCH];
+#pragma unroll
+        for (int b = 0; b < SCAN_BATCH; b++) v[b] = __ldg(p + 32 * b);
+#pragma unroll
+        for (int b = 0; b < SCAN_BATCH; b++) scan_value(v[b], emax, lmin);
+    }
+    for (; k < n; k += 32, p += 32) scan_value(__ldg(p), emax, lmin);
+}
+
 // The group's header, once every exponent is in (one thread): digits and
 // diagonals, or operand bits and the fewest moduli whose product M_L holds
 // them, K 2^(ta+tb) < M_L / 2.
@@ -209,31 +255,9 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
             const int64_t step = M * sh.kt;
             const double *col = t.A + i0 + k0 * M;
             int e0 = -100000, l0 = 100000, e1 = -100000, l1 = 100000;
-            if ((M & 1) == 0 && ((uintptr_t)t.A & 15) == 0) {  // i0 even, M even: the pair is 16-byte aligned
-                int k = 0;
-                for (; k + SCAN_BATCH <= n; k += SCAN_BATCH) {
-                    double2 v[SCAN_BATCH];
-#pragma unroll
-                    for (int b = 0; b < SCAN_BATCH; b++, col += step) v[b] = __ldg(reinterpret_cast<const double2 *>(col));
-#pragma unroll
-                    for (int b = 0; b < SCAN_BATCH; b++) {
-                        scan_value(v[b].x, e0, l0);
-                        scan_value(v[b].y, e1, l1);
-                    }
-                }
-                for (; k < n; k++, col += step) {
-                    const double2 v = __ldg(reinterpret_cast<const double2 *>(col));
-                    scan_value(v.x, e0, l0);
-                    scan_value(v.y, e1, l1);
-                }
-            } else {
-                const bool two = i0 + 1 < M;
-#pragma unroll 8
-                for (int k = 0; k < n; k++, col += step) {
-                    scan_value(__ldg(col), e0, l0);
-                    if (two) scan_value(__ldg(col + 1), e1, l1);
-                }
-            }
+            // i0 even: where M is even and the base aligned, the pair is 16-byte aligned
+            if ((M & 1) == 0 && ((uintptr_t)t.A & 15) == 0) scan_columns<true>(col, step, n, true, e0, l0, e1, l1);
+            else scan_columns<false>(col, step, n, i0 + 1 < M, e0, l0, e1, l1);
             int *ea = reinterpret_cast<int *>(sc + g.off_ea), *la = reinterpret_cast<int *>(sc + g.off_la);
             if (e0 > -100000) {
                 atomicMax(ea + i0, e0 + 4096);
@@ -252,29 +276,8 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
                 if (j >= M) break;
                 const double *col = t.B + j * M;
                 int emax = -100000, lmin = 100000;
-                if (vec) {
-                    const double2 *p = reinterpret_cast<const double2 *>(col) + lane;
-                    int k = lane;
-                    const int n = (int)(M / 2);
-                    for (; k + 32 * (SCAN_BATCH - 1) < n; k += 32 * SCAN_BATCH, p += 32 * SCAN_BATCH) {
-                        double2 v[SCAN_BATCH];
-#pragma unroll
-                        for (int b = 0; b < SCAN_BATCH; b++) v[b] = __ldg(p + 32 * b);
-#pragma unroll
-                        for (int b = 0; b < SCAN_BATCH; b++) {
-                            scan_value(v[b].x, emax, lmin);
-                            scan_value(v[b].y, emax, lmin);
-                        }
-                    }
-                    for (; k < n; k += 32, p += 32) {
-                        const double2 v = __ldg(p);
-                        scan_value(v.x, emax, lmin);
-                        scan_value(v.y, emax, lmin);
-                    }
-                } else {
-#pragma unroll 8
-                    for (int64_t k = lane; k < M; k += 32) scan_value(__ldg(col + k), emax, lmin);
-                }
+                if (vec) scan_run(reinterpret_cast<const double2 *>(col), (int)(M / 2), lane, emax, lmin);
+                else scan_run(col, (int)M, lane, emax, lmin);
                 emax = __reduce_max_sync(0xffffffffu, emax);
                 lmin = __reduce_min_sync(0xffffffffu, lmin);
                 if (lane == 0 && emax > -100000) {
