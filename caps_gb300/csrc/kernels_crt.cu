@@ -206,43 +206,17 @@ __device__ __forceinline__ float balanced_digit(uint32_t d) {
     return __uint_as_float(0x4B400000u | d) - (MAGIC + 8192.0f);
 }
 
-// The limbs of X = round(x 2^f) (ties to even; scaled_round in
-// split_common.cuh computes the same X), on 32-bit operations and without
-// branches: for the slicer's f (t - E with E the row's exponent bound, t <=
-// 55) the shift of the significand M (M < 2^53, x = +-M 2^e) left by e + f is
-// at most 3, so M 2^3 is shifted right by 3 - e - f >= 0: first by a whole word
-// where that is 32 or more, then by the rest.  What falls out decides the
-// rounding: its top word, with the lowest bit set if any lower bit is.  Shifts
-// of 63 and more leave less than 2^-7 of a unit: 63.  Checked equal to
-// scaled_round on 60 million doubles and shifts, ties, carries, subnormals and
-// zeros included.
+// The limbs of X = round(x 2^f).
 template <int NL>
 __device__ __forceinline__ Limbs<NL> scaled_limbs14(double x, int f) {
-    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    const int field = (int)((hi >> 20) & 0x7FFu);
-    const uint32_t mh = (hi & 0xFFFFFu) | (field ? 0x100000u : 0u);
-    uint32_t vh = __funnelshift_l(lo, mh, 3), vl = lo << 3;  // M 2^3 < 2^56
-    const int r = min(1078 - max(field, 1) - f, 63);
-    const bool word = r >= 32;
-    const uint32_t out = word ? vl : 0u;  // the word shifted out whole
-    vl = word ? vh : vl;
-    vh = word ? 0u : vh;
-    // shift counts are modulo 32
-    const uint32_t rem = __funnelshift_r(out, vl, r) | (__funnelshift_r(0u, out, r) != 0u ? 1u : 0u);
-    uint32_t ql = __funnelshift_r(vl, vh, r), qh = vh >> (r & 31);
-    const uint32_t up = rem > 0x80000000u - (ql & 1u) ? 1u : 0u;
-    ql += up;
-    qh += ql < up ? 1u : 0u;
     Limbs<NL> l;
-    const uint32_t s = (uint32_t)((int)hi >> 31);  // all ones for x < 0
+    uint32_t ul, uh;
     if constexpr (NL == 2) {
-        const uint32_t u = (ql ^ s) - s + 0x08002000u;  // + 8192 (1 + 2^14)
-        l.a[0] = balanced_digit(u & 16383u);
-        l.a[1] = balanced_digit(u >> 14);
+        scaled_offset(x, f, 0x08002000u, 0u, ul, uh);  // 8192 (1 + 2^14); uh unused
+        l.a[0] = balanced_digit(ul & 16383u);
+        l.a[1] = balanced_digit(ul >> 14);
     } else {
-        const uint64_t q = ((uint64_t)qh << 32) | ql, s64 = ((uint64_t)s << 32) | s;
-        const uint64_t U = (q ^ s64) - s64 + 0x0080020008002000ull;  // + 8192 sum_{k<4} 16384^k
-        const uint32_t ul = (uint32_t)U, uh = (uint32_t)(U >> 32);
+        scaled_offset(x, f, 0x08002000u, 0x00800200u, ul, uh);  // 8192 sum_{k<4} 16384^k
         l.a[0] = balanced_digit(ul & 16383u);
         l.a[1] = balanced_digit((ul >> 14) & 16383u);
         l.a[2] = balanced_digit(__funnelshift_r(ul, uh, 28) & 16383u);

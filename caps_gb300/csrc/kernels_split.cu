@@ -303,103 +303,89 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
 }
 
 // ---------------------------------------------------------------- slice
-// balanced base-128 digits of round(x 2^f), most significant first.
-// X + 64 (1 + 128 + ... + 128^7) has ordinary base-128 digits d_k + 64, so
-// each balanced digit is a 7-bit field minus 64; the top field is not masked
-// (it may reach 128: d_1 = 64 when |X| = 2^55).  Same digits as peeling
-// them off one by one with a carry.
-__device__ __forceinline__ void digits8(double x, int f, int (&d)[8]) {
-    const unsigned long long OFF = 0x0081020408102040ull;  // 64 * sum_{k<8} 128^k
-    const unsigned long long U = (unsigned long long)scaled_round(x, f) + OFF;
-    const uint32_t lo = (uint32_t)U, hi = (uint32_t)(U >> 32);
-    d[7] = (int)(lo & 127u) - 64;
-    d[6] = (int)((lo >> 7) & 127u) - 64;
-    d[5] = (int)((lo >> 14) & 127u) - 64;
-    d[4] = (int)((lo >> 21) & 127u) - 64;
-    d[3] = (int)(__funnelshift_r(lo, hi, 28) & 127u) - 64;
-    d[2] = (int)((hi >> 3) & 127u) - 64;
-    d[1] = (int)((hi >> 10) & 127u) - 64;
-    d[0] = (int)(hi >> 17) - 64;
+// Balanced base-128 digits of round(x 2^f), most significant first, each as
+// the float whose top half is its exact bf16 encoding (|d| <= 64 has at most 7
+// significant bits).  X + 64 (1 + 128 + ... + 128^7) has ordinary base-128
+// digits d_k + 64, so each balanced digit is a 7-bit field minus 64; the top
+// field is not masked (it may reach 128: d_1 = 64 when |X| = 2^55).  Same digits
+// as peeling them off one by one with a carry.
+__device__ __forceinline__ void digits8(double x, int f, float (&d)[8]) {
+    uint32_t lo, hi;
+    scaled_offset(x, f, 0x08102040u, 0x00810204u, lo, hi);  // 64 * sum_{k<8} 128^k
+    const uint32_t c[8] = {hi >> 17, (hi >> 10) & 127u, (hi >> 3) & 127u, __funnelshift_r(lo, hi, 28) & 127u,
+                           (lo >> 21) & 127u, (lo >> 14) & 127u, (lo >> 7) & 127u, lo & 127u};
+#pragma unroll
+    for (int k = 0; k < 8; k++) d[k] = __uint_as_float(0x4B400000u | c[k]) - (12582912.0f + 64.0f);
 }
 
-// |d| <= 64 has at most 7 significant bits: 1.5 * 2^23 + d is exact in fp32,
-// and the top half of the fp32 encoding of d is its exact bf16 encoding
-__device__ __forceinline__ uint32_t bf16_of_digit(int d) {
-    return __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f) >> 16;
-}
-
-// A side: one thread = one row x 8 k (16 bytes per plane); 256 threads = one
-// 128 x 16 tile.  B side: one thread = one column x 8 k; 256 threads = two
-// 64 x 16 tiles.
-__device__ __forceinline__ void split_slice_tile(const LeafTask *__restrict__ tasks, int m, char *__restrict__ ws,
+// One thread = one row of A or column of B x 8 k, 16 bytes per plane.  A: 256
+// threads = one 128 x 16 tile; B: 256 threads = two 64 x 16 tiles.  Bound by HBM
+// (8 B read and 2 B a digit written per entry): 7 leaves of 2500, 8 digits,
+// 474 us with a 64-bit rounding and 8-byte loads of B, 346 us (0.89 of the copy
+// rate) now; integers of 11 bits 413 and 248.
+__device__ __forceinline__ void split_slice_tile(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
                                                  const Geo &g, int s, int leaf, int64_t tile, int side) {
     const LeafTask t = tasks[leaf];
     char *sc = leaf_scalars(ws, g, leaf);
     char *dg = leaf_digits(ws, g, leaf);
-    const int64_t M = m;
+    const int64_t M = g.m;
     const int tid = threadIdx.x;
-    const int64_t atiles = (int64_t)g.mtiles * g.nks;
+    int64_t idx, k0;  // row of A / column of B, first k
+    char *dst;
+    size_t plane;     // bytes between planes
     if (side == 0) {
-        if (tile >= atiles) return;
-        int mt = (int)(tile / g.nks), ks = (int)(tile % g.nks);
-        int r = tid & 127, kg = tid >> 7;
-        int64_t i = (int64_t)mt * TM + r;
-        int64_t k0 = (int64_t)ks * TK + kg * 8;
-        int f = i < M ? reinterpret_cast<const int *>(sc + g.off_fa)[i] : 0;
-        uint32_t packed[MAXS][4];
-#pragma unroll
-        for (int pl = 0; pl < MAXS; pl++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) packed[pl][q] = 0;
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            int64_t k = k0 + e;
-            double x = (i < M && k < M) ? t.A[i + k * M] : 0.0;
-            int d[8];
-            digits8(x, f, d);
-#pragma unroll
-            for (int pl = 0; pl < MAXS; pl++) packed[pl][e >> 1] |= bf16_of_digit(d[pl]) << (16 * (e & 1));
-        }
-        char *base = dg + g.off_da + (size_t)(mt * g.nks + ks) * s * A_PLANE_BYTES;
-        size_t off = (size_t)(r >> 3) * 256 + (size_t)kg * 128 + (size_t)(r & 7) * 16;
-        for (int pl = 0; pl < s; pl++)
-            *reinterpret_cast<uint4 *>(base + (size_t)pl * A_PLANE_BYTES + off) =
-                make_uint4(packed[pl][0], packed[pl][1], packed[pl][2], packed[pl][3]);
+        if (tile >= (int64_t)g.mtiles * g.nks) return;
+        const int r = tid & 127, kg = tid >> 7;
+        idx = tile / g.nks * TM + r;
+        k0 = tile % g.nks * TK + kg * 8;
+        dst = dg + g.off_da + (size_t)tile * s * A_PLANE_BYTES + (size_t)(r >> 3) * 256 + (size_t)kg * 128 +
+              (size_t)(r & 7) * 16;
+        plane = A_PLANE_BYTES;
     } else {
-        int64_t btiles = (int64_t)g.ntiles * g.nks;
-        int64_t bt = tile * 2 + (tid >> 7);
-        if (bt >= btiles) return;
-        int nt = (int)(bt / g.nks), ks = (int)(bt % g.nks);
-        int c = tid & 63, kg = (tid >> 6) & 1;
-        int64_t j = (int64_t)nt * TN + c;
-        int64_t k0 = (int64_t)ks * TK + kg * 8;
-        int f = j < M ? reinterpret_cast<const int *>(sc + g.off_fb)[j] : 0;
-        uint32_t packed[MAXS][4];
+        const int64_t bt = tile * 2 + (tid >> 7);
+        if (bt >= (int64_t)g.ntiles * g.nks) return;
+        const int c = tid & 63, kg = (tid >> 6) & 1;
+        idx = bt / g.nks * TN + c;
+        k0 = bt % g.nks * TK + kg * 8;
+        dst = dg + g.off_db + (size_t)bt * s * B_PLANE_BYTES + (size_t)(c >> 3) * 256 + (size_t)kg * 128 +
+              (size_t)(c & 7) * 16;
+        plane = B_PLANE_BYTES;
+    }
+    const int64_t sk = side == 0 ? M : 1;  // stride between k
+    const double *src = side == 0 ? t.A + idx + k0 * M : t.B + k0 + idx * M;
+    const int f = idx < M ? reinterpret_cast<const int *>(sc + (side == 0 ? g.off_fa : g.off_fb))[idx] : 0;
+    double v[8];
+    if (side == 1 && idx < M && k0 + 8 <= M && ((uintptr_t)src & 15) == 0) {
+        // a column's 8 values lie side by side: 16-byte loads
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+            const double2 w = __ldg(reinterpret_cast<const double2 *>(src + e));
+            v[e] = w.x;
+            v[e + 1] = w.y;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = (idx < M && k0 + e < M) ? __ldg(src + e * sk) : 0.0;
+    }
+    uint32_t packed[MAXS][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float a[8], b[8];
+        digits8(v[2 * q], f, a);
+        digits8(v[2 * q + 1], f, b);
 #pragma unroll
         for (int pl = 0; pl < MAXS; pl++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) packed[pl][q] = 0;
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            int64_t k = k0 + e;
-            double x = (j < M && k < M) ? t.B[k + j * M] : 0.0;
-            int d[8];
-            digits8(x, f, d);
-#pragma unroll
-            for (int pl = 0; pl < MAXS; pl++) packed[pl][e >> 1] |= bf16_of_digit(d[pl]) << (16 * (e & 1));
-        }
-        char *base = dg + g.off_db + (size_t)(nt * g.nks + ks) * s * B_PLANE_BYTES;
-        for (int pl = 0; pl < s; pl++) {
-            size_t off = (size_t)pl * B_PLANE_BYTES + (size_t)(c >> 3) * 256 + (size_t)kg * 128 +
-                         (size_t)(c & 7) * 16;
-            *reinterpret_cast<uint4 *>(base + off) =
-                make_uint4(packed[pl][0], packed[pl][1], packed[pl][2], packed[pl][3]);
-        }
+            packed[pl][q] = __byte_perm(__float_as_uint(a[pl]), __float_as_uint(b[pl]), 0x7632);
     }
+#pragma unroll
+    for (int pl = 0; pl < MAXS; pl++)
+        if (pl < s)
+            *reinterpret_cast<uint4 *>(dst + (size_t)pl * plane) =
+                make_uint4(packed[pl][0], packed[pl][1], packed[pl][2], packed[pl][3]);
 }
 
 // Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).
-__global__ void __launch_bounds__(256) split_slice_kernel(const LeafTask *__restrict__ tasks, int m,
+__global__ void __launch_bounds__(256) split_slice_kernel(const LeafTask *__restrict__ tasks,
                                                           char *__restrict__ ws, Geo g, SplitParams p) {
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     int s, nd;
@@ -408,7 +394,7 @@ __global__ void __launch_bounds__(256) split_slice_kernel(const LeafTask *__rest
     const int64_t per = atiles > btiles2 ? atiles : btiles2;
     const int64_t total = per * g.count;
     for (int64_t it = blockIdx.x; it < total; it += gridDim.x)
-        split_slice_tile(tasks, m, ws, g, s, (int)(it / per), it % per, blockIdx.y);
+        split_slice_tile(tasks, ws, g, s, (int)(it / per), it % per, blockIdx.y);
 }
 
 // ---------------------------------------------------------------- gemm
@@ -710,7 +696,7 @@ cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, Split
     int64_t btiles2 = ((int64_t)g.ntiles * g.nks + 1) / 2;
     int64_t items = (atiles > btiles2 ? atiles : btiles2) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-    split_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, m, ws, g, p);
+    split_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, ws, g, p);
     count_launch();
     return cudaGetLastError();
 }

@@ -144,38 +144,38 @@ __device__ __forceinline__ bool nonzero_bits(double x) {
     return (((uint32_t)__double2hiint(x) << 1) | (uint32_t)__double2loint(x)) != 0u;
 }
 
-// round(x 2^f) to nearest, ties to even, for |x 2^f| <= 2^55, by integer
-// operations on the IEEE bits (the FP64 pipe runs at 1/64 of FP32 here).
-// With x = +-M 2^e (M < 2^53) and f = t - E, t <= 55, E >= e + 52 (E = -1022
-// and M < 2^52 for subnormals), the shift e + f is at most 3 and M << 3 stays
-// below 2^56, so a left shift never overflows.
-__device__ __forceinline__ long long scaled_round(double x, int f) {
-    unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    int field = (int)((u >> 52) & 0x7ff);
-    unsigned long long M = u & 0xFFFFFFFFFFFFFull;
-    int e;
-    if (field == 0) {
-        if (M == 0) return 0;
-        e = -1074;
-    } else {
-        M |= 1ull << 52;
-        e = field - 1075;
-    }
-    int sh = e + f;
-    unsigned long long q;
-    if (sh >= 0) {
-        q = M << sh;
-    } else {
-        int r = -sh;
-        if (r > 63) {
-            q = 0;
-        } else {
-            q = M >> r;
-            unsigned long long rem = M & ((1ull << r) - 1), half = 1ull << (r - 1);
-            if (rem > half || (rem == half && (q & 1))) q++;
-        }
-    }
-    return (u >> 63) ? -(long long)q : (long long)q;
+// X + off, X = round(x 2^f) to nearest, ties to even, |X| <= 2^55, as two words,
+// on 32-bit operations and without branches (the FP64 pipe, which also runs
+// 64-bit shifts, has 1/64 of FP32's rate here).  x = +-M 2^e with M < 2^53, and
+// f = t - E with t <= 55 and E >= e + 52 (E = -1022 and M < 2^52 for subnormals),
+// so the shift of M left by e + f is at most 3 and M 2^3 < 2^56 is shifted right
+// by 3 - e - f >= 0: first by a whole word where that is 32 or more, then by
+// the rest.  What falls out decides the rounding: its top word, with the lowest
+// bit set if any lower bit is.  Shifts of 63 and more leave less than 2^-7 of
+// a unit: 63.  Checked equal to the 64-bit formulation (shift, compare the
+// remainder with half) on 60 million doubles and shifts, ties, carries,
+// subnormals and zeros included.
+__device__ __forceinline__ void scaled_offset(double x, int f, uint32_t off_lo, uint32_t off_hi, uint32_t &ul,
+                                              uint32_t &uh) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const int field = (int)((hi >> 20) & 0x7FFu);
+    const uint32_t mh = (hi & 0xFFFFFu) | (field ? 0x100000u : 0u);
+    uint32_t vh = __funnelshift_l(lo, mh, 3), vl = lo << 3;
+    const int r = min(1078 - max(field, 1) - f, 63);
+    const bool word = r >= 32;
+    const uint32_t out = word ? vl : 0u;  // the word shifted out whole
+    vl = word ? vh : vl;
+    vh = word ? 0u : vh;
+    // shift counts are modulo 32
+    const uint32_t rem = __funnelshift_r(out, vl, r) | (__funnelshift_r(0u, out, r) != 0u ? 1u : 0u);
+    uint32_t ql = __funnelshift_r(vl, vh, r), qh = vh >> (r & 31);
+    const uint32_t up = rem > 0x80000000u - (ql & 1u) ? 1u : 0u;
+    ql += up;
+    qh += ql < up ? 1u : 0u;
+    const uint64_t q = ((uint64_t)qh << 32) | ql, s = (uint64_t)(int64_t)((int)hi >> 31);  // all ones for x < 0
+    const uint64_t u = (q ^ s) - s + (((uint64_t)off_hi << 32) | off_lo);
+    ul = (uint32_t)u;
+    uh = (uint32_t)(u >> 32);
 }
 
 // ---------------------------------------------------------------- sm_100+ wrappers

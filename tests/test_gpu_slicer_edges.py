@@ -1,6 +1,6 @@
-"""The residue slicer rounds and cuts operands without branches, two limbs for
-few operand bits and four otherwise: magnitudes on every side of its shifts,
-ties and rounding carries, against the oracle's 128-bit model, bit for bit."""
+"""The slicers round and cut operands without branches (residues: two limbs for
+few operand bits and four otherwise): magnitudes on every side of the shifts,
+ties and rounding carries, against the oracle's models, bit for bit."""
 import numpy as np
 import pytest
 
@@ -39,3 +39,19 @@ def test_subnormal_and_huge_operands(caps, oracle_mod, cuda, scale_a, scale_b):
     A, B = rng.uniform(-1, 1, (m, m)) * scale_a, rng.uniform(-1, 1, (m, m)) * scale_b
     C, _ = leaf(caps, cuda, A, B)
     assert np.array_equal(C, model(oracle_mod, A, B)[0])
+
+
+@pytest.mark.parametrize("m", [96, 131])
+@pytest.mark.parametrize("slices", [0, 3])
+def test_digit_rounding_at_every_shift_bitexact_vs_model(caps, oracle_mod, cuda, m, slices):
+    import torch
+    rng = np.random.default_rng(m)
+    A, B = magnitudes(m, rng), magnitudes(m, rng).T.copy()
+    B[:, 1] *= 2.0 ** -1000  # with the tail of the column subnormal
+    a, b = A.T.copy().reshape(-1), B.T.copy().reshape(-1)
+    C = torch.full((m * m,), float("nan"), dtype=torch.float64, device=cuda)
+    caps.leaf_gemm(torch.from_numpy(a).to(cuda), torch.from_numpy(b).to(cuda), C, m, form="split", scheme="digits",
+                   slices=slices)
+    torch.cuda.synchronize()
+    cnt = caps.counters()
+    assert np.array_equal(C.cpu().numpy(), oracle_mod.split_gemm(a, b, m, cnt["split_slices"], cnt["split_diagonals"]))
