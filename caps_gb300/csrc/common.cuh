@@ -158,9 +158,10 @@ constexpr int RESIDUE_KMAX = 2048;  // residue scheme: largest leaf K (K 90^2 < 
 // dimension K (0 if more than it has).
 int crt_moduli_needed(int bits, int K);
 int crt_product_bits(int L);  // floor(log2) of the product of the first L moduli
-// Per-row / per-column scale exponents, the digit or modulus count.
+// Per-row / per-column scale exponents, the digit or modulus count.  `report`
+// (may be null): digits needed, digits, diagonals and moduli go there too.
 cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
-                             cudaStream_t stream);
+                              int *report, cudaStream_t stream);
 // The operand slices (digit or residue planes).
 cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, SplitParams p,
                               void *workspace, cudaStream_t stream);

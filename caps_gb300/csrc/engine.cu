@@ -90,7 +90,18 @@ static caps_status ensure(DevBuf &b, size_t bytes) {
 
 static DevBuf g_arena;   // workspace + task tables
 static DevBuf g_io;      // device copies for caps_multiply_host
-static DevBuf g_status;  // device status words of split kernels
+
+// Mapped host memory the split kernels write: their status word, and the
+// first fields of the last launch group's header.  The host reads it once the
+// stream is done, with no copies of its own (two of them took 10 us of one
+// leaf of 448's 78).
+struct SplitReport {
+    unsigned status;
+    int counts[4];  // needed, digits, diagonals, moduli
+};
+static SplitReport *g_report = nullptr;      // host address
+static SplitReport *g_report_dev = nullptr;  // the same on the device
+
 static DevBuf g_chol;    // -B^T and the product of caps_chol_mult_dev
 static DevBuf g_rect;    // task table of caps_rect_mm_dev
 
@@ -833,7 +844,7 @@ static caps_status launch_ops(const std::vector<Op> &ops, char *tables, char *ws
                 // scan + prep are timed with the multiply phase but not as GEMM
                 Rec pre{nullptr, nullptr, PH_MUL, false, 0.0};
                 if (timed) ev_begin(pre.e0);
-                err = launch_split_scan(t, o.count, o.m, o.sp, ws, s);
+                err = launch_split_scan(t, o.count, o.m, o.sp, ws, g_report_dev->counts, s);
                 if (err == cudaSuccess) err = launch_split_prep(t, o.count, o.m, o.sp, ws, s);
                 if (timed) {
                     cudaEventCreate(&pre.e1);
@@ -842,7 +853,7 @@ static caps_status launch_ops(const std::vector<Op> &ops, char *tables, char *ws
                 }
                 if (err != cudaSuccess) break;
                 if (timed) ev_begin(r.e0);
-                err = launch_split_gemm(t, o.count, o.m, o.sp, ws, reinterpret_cast<unsigned *>(g_status.ptr), s);
+                err = launch_split_gemm(t, o.count, o.m, o.sp, ws, &g_report_dev->status, s);
                 r.phase = PH_MUL;
                 r.gemm = true;
                 r.m3 = (double)o.count * o.m * (double)o.m * o.m;
@@ -912,31 +923,37 @@ static caps_status run_ops(Planned &pl, cudaStream_t s, double *phase_time, Kern
 }
 
 static caps_status status_buffer() {
-    if (!g_status.ptr) {
-        CAPS_TRY(ensure(g_status, 256));
-        CAPS_CUDA_TRY(cudaMemset(g_status.ptr, 0, 256));
+    if (g_report) return CAPS_OK;
+    void *p = nullptr;
+    CAPS_CUDA_TRY(cudaHostAlloc(&p, sizeof(SplitReport), cudaHostAllocMapped | cudaHostAllocPortable));
+    memset(p, 0, sizeof(SplitReport));
+    void *d = nullptr;
+    cudaError_t e = cudaHostGetDevicePointer(&d, p, 0);
+    if (e != cudaSuccess) {
+        cudaFreeHost(p);
+        note_cuda_error(e, "cudaHostGetDevicePointer");
+        return CAPS_ERR_CUDA;
     }
+    g_report = static_cast<SplitReport *>(p);
+    g_report_dev = static_cast<SplitReport *>(d);
     return CAPS_OK;
 }
 
-// Reads (and clears) the device status word of the split kernels, and the
-// digit / diagonal counts (digit scheme) or the moduli count (residue scheme)
-// the last split launch group used.
-static caps_status check_device_status(cudaStream_t s, const void *last_split_ws) {
-    if (!g_status.ptr) return CAPS_OK;
-    unsigned h = 0;
-    int sd[4] = {0, 0, 0, 0};  // needed, digits, diagonals, moduli (split header)
-    CAPS_CUDA_TRY(cudaMemcpyAsync(&h, g_status.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    if (last_split_ws)
-        CAPS_CUDA_TRY(cudaMemcpyAsync(sd, last_split_ws, sizeof sd, cudaMemcpyDeviceToHost, s));
+// Waits for the stream, reads (and clears) the status word of the split
+// kernels, and with `counts` takes the digit / diagonal counts (digit scheme)
+// or the moduli count (residue scheme) of the last launch group.
+static caps_status check_device_status(cudaStream_t s, bool counts) {
     CAPS_CUDA_TRY(cudaStreamSynchronize(s));
-    g_counters.split_moduli = sd[3];
-    g_counters.split_slices = sd[3] ? 0 : sd[1];
-    g_counters.split_diagonals = sd[3] ? 0 : sd[2];
-    if (h != 0) {
-        CAPS_CUDA_TRY(cudaMemsetAsync(g_status.ptr, 0, sizeof(unsigned), s));
+    if (!g_report) return CAPS_OK;
+    const SplitReport r = *g_report;  // nothing writes it any more
+    const int moduli = counts ? r.counts[3] : 0;
+    g_counters.split_moduli = moduli;
+    g_counters.split_slices = counts && !moduli ? r.counts[1] : 0;
+    g_counters.split_diagonals = counts && !moduli ? r.counts[2] : 0;
+    if (r.status != 0) {
+        g_report->status = 0;
         char buf[96];
-        snprintf(buf, sizeof buf, "device wait gave up (status 0x%x)", h);
+        snprintf(buf, sizeof buf, "device wait gave up (status 0x%x)", r.status);
         g_last_err = buf;
         return CAPS_ERR_TIMEOUT;
     }
@@ -996,10 +1013,7 @@ static caps_status multiply_dev_locked(const double *A, const double *B, double 
     g_counters.workspace_peak_bytes = (long long)pl.ws_bytes;
     g_counters.kernel_launches = g_launches - l0;
     if (o.form == CAPS_FORM_SPLIT && sync_status) {
-        const void *last = nullptr;
-        for (const Op &op : pl.b.ops)
-            if (op.kind == K_LEAF_SPLIT) last = g_arena.ptr + op.split_off;
-        CAPS_TRY(check_device_status(s, last));
+        CAPS_TRY(check_device_status(s, true));
     }
     return CAPS_OK;
 }
@@ -1664,7 +1678,7 @@ static caps_status multiply_batched_locked(const std::vector<BatchItem> &items, 
     g_counters.multiplications = plan->muls;
     g_counters.add_bytes = plan->add_bytes;
     g_counters.kernel_launches = plan->kernels;
-    if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(check_device_status(stream, nullptr));
+    if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(check_device_status(stream, false));
     else CAPS_CUDA_TRY(cudaStreamSynchronize(stream));
     return CAPS_OK;
 }
@@ -1903,7 +1917,7 @@ caps_status caps_multiply_host(const double *A, const double *B, double *C, caps
             CAPS_CUDA_TRY(cudaMemcpyAsync((char *)C + 2 * q + b0, (char *)dC + 2 * q + b0, b1 - b0, cudaMemcpyDeviceToHost, cs));
     }
     if (timeline) CAPS_CUDA_TRY(cudaEventRecord(hs->timing[4], cs));
-    if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(check_device_status(s, nullptr));
+    if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(check_device_status(s, false));
     CAPS_CUDA_TRY(cudaStreamSynchronize(s));
     CAPS_CUDA_TRY(cudaStreamSynchronize(cs));
     if (timeline) {
@@ -2197,10 +2211,12 @@ void caps_release_cache(void) {
     cudaDeviceSynchronize();
     for (BatchPlan *p : g_batch_plans) free_plan(p);
     g_batch_plans.clear();
-    for (DevBuf *b : {&g_arena, &g_io, &g_status, &g_chol, &g_rect}) {
+    for (DevBuf *b : {&g_arena, &g_io, &g_chol, &g_rect}) {
         if (b->ptr) cudaFree(b->ptr);
         *b = DevBuf();
     }
+    if (g_report) cudaFreeHost(g_report);
+    g_report = g_report_dev = nullptr;
     if (g_pinned.ptr) cudaFreeHost(g_pinned.ptr);
     g_pinned.ptr = nullptr;
     g_pinned.size = 0;

@@ -172,7 +172,7 @@ __device__ __forceinline__ void scan_run(const T *col, int n, int lane, int &ema
 // diagonals, or operand bits and the fewest moduli whose product M_L holds
 // them, K 2^(ta+tb) < M_L / 2.
 __device__ __forceinline__ void resolve_group(SplitHdr *h, const Geo &g, SplitParams p, bool residues,
-                                              const ModuliBits &mb) {
+                                              const ModuliBits &mb, int *report) {
     SplitHdr v;
     v.needed = __ldcg(&h->needed);
     int s, nd;
@@ -193,12 +193,18 @@ __device__ __forceinline__ void resolve_group(SplitHdr *h, const Geo &g, SplitPa
     h->ta = ta;
     h->tb = tb;
     h->moduli = L;
+    if (report) {
+        report[0] = v.needed;
+        report[1] = s;
+        report[2] = nd;
+        report[3] = L;
+    }
 }
 
 // One leaf side, by a block: f = 55 - E per row / column (digit scheme),
 // digits needed, and the bits E - lsb + 1; the last side of the group resolves it.
 __device__ __forceinline__ void finish_side(char *__restrict__ ws, const Geo &g, int leaf, int side, SplitParams p,
-                                            bool residues, const ModuliBits &mb) {
+                                            bool residues, const ModuliBits &mb, int *report) {
     SplitHdr *h = reinterpret_cast<SplitHdr *>(ws);
     char *sc = leaf_scalars(ws, g, leaf);
     const int *ev = reinterpret_cast<const int *>(sc + (side ? g.off_eb : g.off_ea));
@@ -226,19 +232,19 @@ __device__ __forceinline__ void finish_side(char *__restrict__ ws, const Geo &g,
         __threadfence();
         const bool all = atomicAdd(&h->finished, 1) == 2 * g.count - 1;
         __threadfence();
-        if (all) resolve_group(h, g, p, residues, mb);
+        if (all) resolve_group(h, g, p, residues, mb, report);
     }
 }
 
 __global__ void __launch_bounds__(256) split_finish_kernel(char *__restrict__ ws, Geo g, SplitParams p, int residues,
-                                                           ModuliBits mb) {
-    finish_side(ws, g, blockIdx.x, blockIdx.y, p, residues != 0, mb);
+                                                           ModuliBits mb, int *report) {
+    finish_side(ws, g, blockIdx.x, blockIdx.y, p, residues != 0, mb, report);
 }
 
 template <bool FINISH>
 __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restrict__ tasks,
                                                          char *__restrict__ ws, Geo g, ScanShape sh, SplitParams p,
-                                                         int residues, ModuliBits mb) {
+                                                         int residues, ModuliBits mb, int *report) {
     const int side = blockIdx.y;
     const int64_t M = g.m, units = side ? sh.bunits : sh.aunits, total = units * g.count;
     __shared__ int last;
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restr
             __threadfence();
         }
         __syncthreads();
-        if (last) finish_side(ws, g, l, side, p, residues != 0, mb);
+        if (last) finish_side(ws, g, l, side, p, residues != 0, mb, report);
     }
 }
 
@@ -665,7 +671,7 @@ void split_gemm_prepare() {
 }
 
 cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
-                              cudaStream_t stream) {
+                              int *report, cudaStream_t stream) {
     const Geo g = make_geo(m, count, p.scheme);
     cudaError_t e = cudaMemsetAsync(workspace, 0, g.dg_base, stream);
     if (e != cudaSuccess) return e;
@@ -677,11 +683,13 @@ cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, Split
     const int residues = runs_residues(g, p);
     // 48 registers a thread: 5 blocks of 256 on each of 152 SMs at once
     if ((sh.aunits + sh.bunits) * count <= 152 * 5) {
-        split_scan_kernel<true><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb);
+        split_scan_kernel<true><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb,
+                                                             report);
         count_launch();
     } else {
-        split_scan_kernel<false><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb);
-        split_finish_kernel<<<dim3((unsigned)count, 2), 256, 0, stream>>>((char *)workspace, g, p, residues, mb);
+        split_scan_kernel<false><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb,
+                                                              report);
+        split_finish_kernel<<<dim3((unsigned)count, 2), 256, 0, stream>>>((char *)workspace, g, p, residues, mb, report);
         count_launch(2);
     }
     return cudaGetLastError();

@@ -110,7 +110,7 @@ extern "C" caps_status caps_leaf_gemm_split_noalloc_dev(const double *A, const d
     caps::count_launch();
     CAPS_CUDA_TRY(cudaGetLastError());
     CAPS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned), s));
-    CAPS_CUDA_TRY(caps::launch_split_scan(task, 1, m, p, ws, s));   // clears header and scales
+    CAPS_CUDA_TRY(caps::launch_split_scan(task, 1, m, p, ws, nullptr, s));   // clears header and scales
     CAPS_CUDA_TRY(caps::launch_split_prep(task, 1, m, p, ws, s));
     CAPS_CUDA_TRY(caps::launch_split_gemm(task, 1, m, p, ws, status, s));
     unsigned h = 0;

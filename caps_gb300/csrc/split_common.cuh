@@ -25,7 +25,6 @@ constexpr uint32_t WAIT_LIMIT_STARVED = 1u << 12;
 enum { SCHEME_AUTO = 0, SCHEME_DIGITS = 1, SCHEME_RESIDUES = 2 };
 
 // First 256 bytes of a launch group's workspace, written by the scan kernel.
-// The host reads the first four fields back after a multiply (counters).
 struct SplitHdr {
     int needed;    // digits needed, max over the group
     int s_used;    // digit scheme: digits and diagonals
