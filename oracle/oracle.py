@@ -39,9 +39,10 @@ def build(force: bool = False) -> str:
 
 
 def reference_dir():
-    """Directory of the reference sources, or None where they are absent: the
-    CAPS_REFERENCE_DIR environment variable, else the directory
-    build_ref.sh built oracle/_ref from (it records it there)."""
+    """Directory of the reference sources: the CAPS_REFERENCE_DIR environment
+    variable, else the directory build_ref.sh built oracle/_ref from (it
+    records it there).  Where they are absent, a directory that does not exist:
+    an empty name joined with "tests" would be this repository's own folder."""
     cands = [os.environ.get("CAPS_REFERENCE_DIR")]
     try:
         with open(os.path.join(HERE, "_ref", "REFERENCE_DIR")) as f:
@@ -51,7 +52,7 @@ def reference_dir():
     for c in cands:
         if c and os.path.isfile(os.path.join(c, "multiply.cpp")):
             return c
-    return None
+    return os.path.join(HERE, "_ref", "no-reference-sources")
 
 
 def openblas_path():
