@@ -429,6 +429,7 @@ __device__ __forceinline__ void crt_slice_tile(const LeafTask *__restrict__ task
 // (0.83 of the copy rate), 7 leaves of 896 at 17 from 86 to 81.
 __global__ void __launch_bounds__(256, 5) crt_slice_kernel(const LeafTask *__restrict__ tasks,
                                                         char *__restrict__ ws, Geo g) {
+    chain_wait();
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int L = h->moduli;
     __shared__ SliceConst consts[LMAX];
@@ -900,8 +901,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     crt_gemm_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws, Geo g,
                     const __grid_constant__ CUtensorMap planes, unsigned *__restrict__ status, int split,
                     int starve) {
-    const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
-    const int L = h->moduli;
     // starve (test hook): no copies are issued, so nothing is ever in flight
     // and every wait may give up after a short spin
     const uint32_t wl = starve ? WAIT_LIMIT_STARVED : WAIT_LIMIT;
@@ -944,6 +943,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RGEMM_THREADS, 1)
     cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
+    const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
+    const int L = h->moduli;
 
     const int64_t tiles = (int64_t)((g.mtiles + 1) / 2) * g.rtiles;
     const int64_t total = tiles * g.count;
@@ -1061,6 +1063,7 @@ __device__ __forceinline__ void combine_step(const Section &t, int step, int64_t
 
 __global__ void __launch_bounds__(128) crt_combine_kernel(const LeafTask *__restrict__ tasks, char *__restrict__ ws,
                                                           Geo g) {
+    chain_wait();
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     const int section = (blockIdx.x >> 3) & 7, step = (blockIdx.x & 7) * 4 + (threadIdx.x >> 5);
     const int64_t tile = blockIdx.x >> 6;
@@ -1118,9 +1121,8 @@ cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitP
     const int64_t atiles = (int64_t)g.mtiles * g.nks, btiles = (int64_t)g.rtiles * g.nks * 2;
     const int64_t items = (atiles > btiles ? atiles : btiles) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-    crt_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g);
     count_launch();
-    return cudaGetLastError();
+    return launch_chained(crt_slice_kernel, grid, 256, 0, stream, tasks_dev, (char *)workspace, g);
 }
 
 cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
@@ -1152,12 +1154,14 @@ cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitPa
     const size_t smem = (size_t)RNSTAGE * RSTAGE_BYTES + 1024 + 1024;
     const int64_t want = split ? units * LMAX : units;
     if (want < pairs) pairs = (int)want;
-    crt_gemm_kernel<<<2 * pairs, RGEMM_THREADS, smem, stream>>>(tasks_dev, (char *)workspace, g, planes, status_dev, split,
-                                                                starve);
+    e = launch_chained(crt_gemm_kernel, 2 * pairs, RGEMM_THREADS, smem, stream, tasks_dev, (char *)workspace, g, planes,
+                       status_dev, split, starve);
     count_launch();
+    if (e != cudaSuccess) return e;
     if (split) {
-        crt_combine_kernel<<<(unsigned)(units * 2 * 64), 128, 0, stream>>>(tasks_dev, (char *)workspace, g);
+        e = launch_chained(crt_combine_kernel, (unsigned)(units * 2 * 64), 128, 0, stream, tasks_dev, (char *)workspace, g);
         count_launch();
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(32 * WM * WN) dmma_gemm_kernel(const DmmaTask 
     constexpr int LDA = BM + 8, LDB = BN + 8;  // padded rows (banks)
     __shared__ double As[BK][LDA];  // As[k][i]
     __shared__ double Bs[BK][LDB];  // Bs[k][j]
+    chain_wait();
     const DmmaTask t = tasks[blockIdx.z];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wr = warp / WN, wc = warp % WN;
@@ -155,7 +156,7 @@ static cudaError_t launch_dmma_shape(const DmmaTask *tasks_dev, int count, int m
     for (int base = 0; base < count; base += 65535) {
         const int c = count - base < 65535 ? count - base : 65535;
         dim3 grid(cols, rows, (unsigned)c);
-        dmma_gemm_kernel<WM, WN, FM, FN><<<grid, 32 * WM * WN, 0, stream>>>(tasks_dev + base, m, n, k);
+        launch_chained(dmma_gemm_kernel<WM, WN, FM, FN>, grid, 32 * WM * WN, 0, stream, tasks_dev + base, m, n, k);
         count_launch();
     }
     return cudaGetLastError();

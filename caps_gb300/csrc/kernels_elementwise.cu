@@ -164,6 +164,7 @@ __device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
 
 template <int OP, bool VEC>
 __global__ void __launch_bounds__(256) ew_kernel(const EwTask *__restrict__ tasks, int64_t q) {
+    chain_wait();
     const EwTask t = tasks[blockIdx.y];
     if (VEC) {
         const int64_t nv = q >> 1, stride = (int64_t)gridDim.x * 256;
@@ -214,9 +215,9 @@ static void launch_op(bool vec, const EwTask *tasks, int count, int64_t q, cudaS
     if (want < 1) want = 1;
     dim3 grid((unsigned)want, (unsigned)count);
     if (vec)
-        ew_kernel<OP, true><<<grid, threads, 0, s>>>(tasks, q);
+        launch_chained(ew_kernel<OP, true>, grid, threads, 0, s, tasks, q);
     else
-        ew_kernel<OP, false><<<grid, threads, 0, s>>>(tasks, q);
+        launch_chained(ew_kernel<OP, false>, grid, threads, 0, s, tasks, q);
 }
 
 cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q,
@@ -424,6 +425,7 @@ template <bool TO_CAPS>
 __global__ void __launch_bounds__(256) reorder_kernel(const double *const *__restrict__ src,
                                                       double *const *__restrict__ dst,
                                                       ReorderGeom g) {
+    chain_wait();
     const double *s = src[blockIdx.y];
     double *d = dst[blockIdx.y];
     if (g.bs >= RUN_MIN)
@@ -467,9 +469,9 @@ cudaError_t launch_reorder(const double *const *src_dev, double *const *dst_dev,
     ReorderGeom g = make_geom(n, nrec, bs);
     dim3 grid(reorder_blocks(g, count), (unsigned)count);
     if (to_caps)
-        reorder_kernel<true><<<grid, 256, 0, stream>>>(src_dev, dst_dev, g);
+        launch_chained(reorder_kernel<true>, grid, 256, 0, stream, src_dev, dst_dev, g);
     else
-        reorder_kernel<false><<<grid, 256, 0, stream>>>(src_dev, dst_dev, g);
+        launch_chained(reorder_kernel<false>, grid, 256, 0, stream, src_dev, dst_dev, g);
     count_launch();
     return cudaGetLastError();
 }

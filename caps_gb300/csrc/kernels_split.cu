@@ -238,6 +238,7 @@ __device__ __forceinline__ void finish_side(char *__restrict__ ws, const Geo &g,
 
 __global__ void __launch_bounds__(256) split_finish_kernel(char *__restrict__ ws, Geo g, SplitParams p, int residues,
                                                            ModuliBits mb, int *report) {
+    chain_wait();
     finish_side(ws, g, blockIdx.x, blockIdx.y, p, residues != 0, mb, report);
 }
 
@@ -245,6 +246,7 @@ template <bool FINISH>
 __global__ void __launch_bounds__(256) split_scan_kernel(const LeafTask *__restrict__ tasks,
                                                          char *__restrict__ ws, Geo g, ScanShape sh, SplitParams p,
                                                          int residues, ModuliBits mb, int *report) {
+    chain_wait();
     const int side = blockIdx.y;
     const int64_t M = g.m, units = side ? sh.bunits : sh.aunits, total = units * g.count;
     __shared__ int last;
@@ -393,6 +395,7 @@ __device__ __forceinline__ void split_slice_tile(const LeafTask *__restrict__ ta
 // Grid-stride over (leaf, tile).  blockIdx.y: A (0) or B (1).
 __global__ void __launch_bounds__(256) split_slice_kernel(const LeafTask *__restrict__ tasks,
                                                           char *__restrict__ ws, Geo g, SplitParams p) {
+    chain_wait();
     const SplitHdr *h = reinterpret_cast<const SplitHdr *>(ws);
     int s, nd;
     resolve_sd(h, p, s, nd);
@@ -463,6 +466,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NSTAGE + 3);
     MmaTable *mtab = reinterpret_cast<MmaTable *>(bars + 16);
 
+    chain_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // starve (test hook): no copies are issued, so nothing is ever in flight
     // and every wait may give up after a short spin
@@ -683,13 +687,14 @@ cudaError_t launch_split_scan(const LeafTask *tasks_dev, int count, int m, Split
     const int residues = runs_residues(g, p);
     // 48 registers a thread: 5 blocks of 256 on each of 152 SMs at once
     if ((sh.aunits + sh.bunits) * count <= 152 * 5) {
-        split_scan_kernel<true><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb,
-                                                             report);
+        launch_chained(split_scan_kernel<true>, grid, 256, 0, stream, tasks_dev, (char *)workspace, g, sh, p, residues, mb,
+                       report);
         count_launch();
     } else {
-        split_scan_kernel<false><<<grid, 256, 0, stream>>>(tasks_dev, (char *)workspace, g, sh, p, residues, mb,
-                                                              report);
-        split_finish_kernel<<<dim3((unsigned)count, 2), 256, 0, stream>>>((char *)workspace, g, p, residues, mb, report);
+        launch_chained(split_scan_kernel<false>, grid, 256, 0, stream, tasks_dev, (char *)workspace, g, sh, p, residues, mb,
+                       report);
+        launch_chained(split_finish_kernel, dim3((unsigned)count, 2), 256, 0, stream, (char *)workspace, g, p, residues, mb,
+                       report);
         count_launch(2);
     }
     return cudaGetLastError();
@@ -704,7 +709,7 @@ cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, Split
     int64_t btiles2 = ((int64_t)g.ntiles * g.nks + 1) / 2;
     int64_t items = (atiles > btiles2 ? atiles : btiles2) * count;
     dim3 grid((unsigned)(items < 4096 ? items : 4096), 2);
-    split_slice_kernel<<<grid, 256, 0, stream>>>(tasks_dev, ws, g, p);
+    launch_chained(split_slice_kernel, grid, 256, 0, stream, tasks_dev, ws, g, p);
     count_launch();
     return cudaGetLastError();
 }
@@ -725,7 +730,7 @@ cudaError_t launch_split_gemm(const LeafTask *tasks_dev, int count, int m, Split
     const size_t smem = (size_t)NSTAGE * STAGE_BYTES + 1024 + 1024;
     int64_t total = (int64_t)g.mtiles * g.ntiles * count;
     int grid = (int)(total < g_num_sms ? total : g_num_sms);
-    split_gemm_kernel<<<grid, GEMM_THREADS, smem, stream>>>(tasks_dev, count, ws, g, p, status_dev, starve);
+    launch_chained(split_gemm_kernel, grid, GEMM_THREADS, smem, stream, tasks_dev, count, ws, g, p, status_dev, starve);
     count_launch();
     return cudaGetLastError();
 }
