@@ -166,14 +166,15 @@ static cudaError_t launch_dmma_shape(const DmmaTask *tasks_dev, int count, int m
 // SM share its one DMMA pipe, so a launch takes as long as the SM with the
 // most tile area: a leaf of 1024 is 256 tiles of 64 on 152 SMs, 2 on the
 // busiest and 1.7 on average; of 32, 1024 tiles, 7 and 6.7.  Smaller tiles read their
-// operands more often and synchronise more per multiply-add, which costs a
-// little where the SM has few of them to overlap.  us a multiply, 64 always ->
-// picked: n = 4096 'dd' (leaves of 1024) 121390 -> 97350 (93100 at the pipe's
-// rate), 4096 x 2048 x 3072 48910 -> 46980, n = 56 'dd' 1471 -> 437 (with the
+// operands more often and synchronise more per multiply-add, which costs next
+// to nothing at this pipe's rate (4096 x 2048 x 3072: 46890 us with 16, 47010
+// with 32).  us a multiply, 64 always -> picked: n = 4096 'dd' (leaves of 1024)
+// 121390 -> 96920 (32 alone: 97100; 93100 at the pipe's rate), leaf of 1500 7040
+// -> 6270, 4096 x 2048 x 3072 48910 -> 46890, n = 56 'dd' 1471 -> 437 (with the
 // skipped padding).
 static int pick_tile(int count, int m, int n) {
     const int sides[3] = {64, 32, 16};
-    const double cost[3] = {1.0, 1.01, 1.04};
+    const double cost[3] = {1.0, 1.01, 1.005};
     int best = 64;
     double best_t = 0.0;
     for (int i = 0; i < 3; i++) {
