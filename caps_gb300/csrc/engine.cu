@@ -995,7 +995,16 @@ static caps_status multiply_dev_locked(const double *A, const double *B, double 
         return CAPS_ERR_BUDGET;
     }
     if (o.form == CAPS_FORM_SPLIT) CAPS_TRY(status_buffer());
-    CAPS_TRY(ensure(g_arena, pl.total));
+    caps_status room = ensure(g_arena, pl.total);
+    if (room == CAPS_ERR_ALLOC && merge) {
+        // a device too full for the merged steps: every step as the pattern
+        // has it, where that takes noticeably less
+        const size_t merged = pl.total;
+        merge = false;
+        CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras, merge));
+        if (pl.total + ((size_t)1 << 20) < merged) room = ensure(g_arena, pl.total);
+    }
+    CAPS_TRY(room);
     CAPS_TRY(plan(A, B, C, d, pat, o, g_arena.ptr, pl, host_overlap, extras, merge));
     double pt[3] = {0, 0, 0};
     long long l0 = g_launches;

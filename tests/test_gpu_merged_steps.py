@@ -47,3 +47,31 @@ def test_host_entry_with_merged_inner_steps(caps, cuda, form):
     caps.multiply(torch.from_numpy(a).to(cuda), torch.from_numpy(b).to(cuda), dC, d, "bbb", form=form)
     torch.cuda.synchronize()
     assert np.array_equal(c, dC.cpu().numpy())
+
+
+def test_full_device_falls_back_to_steps_in_sequence(caps, cuda):
+    """An allocation that fails for the merged steps (host-side injection) is
+    tried again for the steps in sequence, where those take less."""
+    import torch
+    n, r = 1024, 2
+    rng = np.random.default_rng(9)
+    A = torch.from_numpy(rng.uniform(-1, 1, n * n)).to(cuda)
+    B = torch.from_numpy(rng.uniform(-1, 1, n * n)).to(cuda)
+    d = caps.MatDescriptor.make(n, r)
+    want, got = torch.empty_like(A), torch.empty_like(A)
+    caps.multiply(A, B, want, d, "dd", form="split")
+    torch.cuda.synchronize()
+    caps.release_cache()
+    caps.debug_fail_allocations(1)
+    try:
+        caps.multiply(A, B, got, d, "dd", form="split")
+        torch.cuda.synchronize()
+        assert caps.counters()["workspace_peak_bytes"] <= caps.workspace_size(d, "dd", form="split")
+        caps.release_cache()
+        caps.debug_fail_allocations(2)
+        with pytest.raises(caps.CapsError) as e:
+            caps.multiply(A, B, got, d, "dd", form="split")
+        assert e.value.status == 5  # CAPS_ERR_ALLOC
+    finally:
+        caps.debug_fail_allocations(0)
+    assert torch.equal(want, got)
