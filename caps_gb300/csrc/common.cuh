@@ -72,26 +72,21 @@ enum EwOp : int {
     EW_FORM_ST = 0,
     // dst0 = src0 (copy)
     EW_COPY = 1,
-    // dst0 = src0 + src1 ; dst1 = dst0  (U1 = Q1+Q4 stored in two buffers)
-    EW_ADD_DUP = 2,
     // dst0 = src0 + src1
-    EW_ADD = 3,
+    EW_ADD = 2,
     // dst0 = src0 - src1
-    EW_SUB = 4,
+    EW_SUB = 3,
     // dst0 = src0 + src2 ; dst1 = src1 + src2   (C22 = U2+Q3 ; U3 = U3+Q3)
-    EW_ADD2 = 5,
+    EW_ADD2 = 4,
     // calcCij: C11..C22 from Q1..Q7 (7 inputs, 4 outputs)
-    EW_CALC_CIJ = 6,
+    EW_CALC_CIJ = 5,
     // operand pairs of the memory-lean 'd' step, formed just before their
     // subproduct; src = A11 A21 A12 A22 B11 B21 B12 B22
-    EW_FORM_T4S4 = 7,  // dst0 = (A21+A22)-A11, dst1 = B22-(B12-B11)
-    EW_FORM_T5S5 = 8,  // dst0 = A11-A21,       dst1 = B22-B12
-    EW_FORM_T3S3 = 9,  // dst0 = A21+A22,       dst1 = B12-B11
-    EW_FORM_S7 = 10,   // dst0 = (B22-(B12-B11))-B21
-    EW_FORM_T6 = 11,   // dst0 = A12-((A21+A22)-A11)
-    // dst0 = src0 ; dst1 = src0 + src2 ; dst2 = src1 + src2
-    // (C21 = U2 ; C22 = U2 + Q3 ; U3 = U1 + Q3)
-    EW_U2_Q3 = 12,
+    EW_FORM_T4S4 = 6,  // dst0 = (A21+A22)-A11, dst1 = B22-(B12-B11)
+    EW_FORM_T5S5 = 7,  // dst0 = A11-A21,       dst1 = B22-B12
+    EW_FORM_T3S3 = 8,  // dst0 = A21+A22,       dst1 = B12-B11
+    EW_FORM_S7 = 9,    // dst0 = (B22-(B12-B11))-B21
+    EW_FORM_T6 = 10,   // dst0 = A12-((A21+A22)-A11)
 };
 
 struct EwTask {
@@ -136,15 +131,15 @@ struct LeafTask {
 //   FOLD_STORE    C = p
 //   FOLD_ADD      C = s0 + p             (EW_ADD with the product second)
 //   FOLD_SUB      C = s0 - p             (EW_SUB)
-//   FOLD_ADD_DUP  C = d1 = s0 + p        (EW_ADD_DUP: U1 into C22 and C12)
-//   FOLD_U2_Q3    C = s0, d1 = s0 + p, d2 = s1 + p  (EW_U2_Q3; s0 = d1, s1 = d2 may alias)
-enum DmmaFold { FOLD_STORE = 0, FOLD_ADD, FOLD_SUB, FOLD_ADD_DUP, FOLD_U2_Q3 };
+//   FOLD_ADD2     C = s0 + p, d1 = s1 + p  (EW_ADD2)
+// The sums may be in place (s0 = C, s1 = d1).
+enum DmmaFold { FOLD_STORE = 0, FOLD_ADD, FOLD_SUB, FOLD_ADD2 };
 struct DmmaTask {
     const double *A;
     const double *B;
     double *C;
     const double *s0, *s1;
-    double *d1, *d2;
+    double *d1;
     int fold;
     int pad;
 };
@@ -194,7 +189,7 @@ cudaError_t launch_split_prep(const LeafTask *tasks_dev, int count, int m, Split
 void split_gemm_prepare();
 // The tensor-core slice products: the digit-pair GEMM with its exact
 // recombination epilogue, or the per-modulus residue GEMM with its CRT
-// reconstruction warps.
+// reconstruction (in its drain warps, or for small launches a kernel after it).
 cudaError_t launch_split_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p,
                               void *workspace, unsigned int *status_dev, cudaStream_t stream);
 

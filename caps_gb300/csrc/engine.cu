@@ -16,7 +16,8 @@
 // the reference's summation order.  The leaf level runs one batched GEMM
 // launch.  Workspace comes from a stack over one device arena; the plan is
 // built twice (a dry run sizes the arena, then the real one), and all task
-// tables of a call go to the device in one copy.
+// tables of a call go to the device at once (small ones as a launch's
+// arguments).
 #include "common.cuh"
 
 #include <algorithm>
@@ -134,11 +135,11 @@ enum OpKind { K_EW = 0, K_LEAF_DMMA, K_LEAF_SPLIT, K_REORDER, K_WAIT, K_RECORD }
 // Events the host entry point uses to overlap its copies with a top-level
 // 'd' step: the step waits for A11/B11 (0) before Q1, for A12/B21 (1) before
 // Q2 and for the other input quadrants (2) before forming T4/S4; it records
-// when C11 (3), C22 (4) and C21 (5) are final, so their copies back run under
+// when C11 (3), C21 (4) and C22 (5) are final, so their copies back run under
 // the later subproducts, and C12, the last, in four parts (6..9): its final
 // sum runs as four launches, and each part's copy back runs under the next.
 constexpr int C12_PARTS = 4;
-constexpr int EV_C_FIRST = 3;  // events 3..5: C11, C22, C21 final; 6..9: the parts of C12
+constexpr int EV_C_FIRST = 3;  // events 3..5: C11, C21, C22 final; 6..9: the parts of C12
 // With a level below the top step, its first subproduct Q1 = A11 B11 runs as
 // an overlapped lean step too, on the sub-quadrants of A11 and B11: events
 // EV_INNER (A11's and B11's first sub-quadrants), +1 (A11's 12 and B11's 21),
@@ -302,7 +303,7 @@ static void emit_leaf_gemm(Builder &b, const std::vector<Prob> &P, int64_t m) {
         }
     } else {
         std::vector<DmmaTask> t;
-        for (const Prob &p : P) t.push_back(DmmaTask{p.A, p.B, p.C, nullptr, nullptr, nullptr, nullptr, FOLD_STORE, 0});
+        for (const Prob &p : P) t.push_back(DmmaTask{p.A, p.B, p.C, nullptr, nullptr, nullptr, FOLD_STORE, 0});
         emit_dmma(b, t, m);
     }
 }
@@ -438,8 +439,8 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
         // Q, and U1 / U2 / U3 live in C quadrants not yet final -- 3 quarter
         // buffers per node.  Per element the sums, products and their order
         // are the reference's:
-        //   C11=Q1; C22=C12=U1=C11+Q4; C22=U2=C22+Q5;
-        //   C21=U2, C22=U2+Q3, C12=U3=C12+Q3; C21=U2-Q7; C12=U3+Q6; C11+=Q2.
+        //   C11=Q1; C12=U1=C11+Q4; C22=U2=C12+Q5; C21=U2-Q7;
+        //   C22=U2+Q3, C12=U3=C12+Q3; C12=U3+Q6; C11+=Q2.
         struct Nd {
             const double *A11, *A21, *A12, *A22, *B11, *B21, *B12, *B22;
             double *C11, *C21, *C12, *C22, *X, *Y, *Q;
@@ -552,8 +553,9 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             emit_event(b, K_WAIT, ev + 2);  // every input; the lean passes form the sums
         }
         // Plain-form leaves right below a step that is not overlapping host
-        // copies: each fold that consumes a product (C22 = C12 = C11 + Q4,
-        // C22 += Q5, the U2 / Q3 triple, C21 -= Q7, C12 += Q6, C11 += Q2) runs
+        // copies: each fold that consumes a product (C12 = C11 + Q4,
+        // C22 = C12 + Q5, C21 = C22 - Q7, C22 += Q3 with C12 += Q3, C12 += Q6,
+        // C11 += Q2) runs
         // in that product's DMMA epilogue, on the accumulator, instead of as a
         // pass over the stored product: the same FP64 operations in the same
         // order, so the same bits, without the product's round trip to HBM.
@@ -564,7 +566,7 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
         auto folded = [&](int which, int mode) {
             std::vector<DmmaTask> t;
             for (const Nd &d : nd) {
-                DmmaTask k{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, mode, 0};
+                DmmaTask k{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, mode, 0};
                 switch (which) {
                     case 2: k.A = d.A12; k.B = d.B21; break;
                     case 3: case 4: case 5: k.A = d.X; k.B = d.Y; break;
@@ -572,10 +574,10 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
                     case 7: k.A = d.A22; k.B = d.X; break;
                 }
                 switch (which) {
-                    case 4: k.C = d.C22; k.s0 = d.C11; k.d1 = d.C12; break;                     // ADD_DUP
-                    case 5: k.C = d.C22; k.s0 = d.C22; break;                                   // ADD
-                    case 3: k.C = d.C21; k.s0 = d.C22; k.s1 = d.C12; k.d1 = d.C22; k.d2 = d.C12; break;  // U2_Q3
-                    case 7: k.C = d.C21; k.s0 = d.C21; break;                                   // SUB
+                    case 4: k.C = d.C12; k.s0 = d.C11; break;                                   // U1
+                    case 5: k.C = d.C22; k.s0 = d.C12; break;                                   // U2
+                    case 7: k.C = d.C21; k.s0 = d.C22; break;
+                    case 3: k.C = d.C22; k.s0 = d.C22; k.d1 = d.C12; k.s1 = d.C12; break;       // C22, U3
                     case 6: k.C = d.C12; k.s0 = d.C12; break;                                   // ADD
                     case 2: k.C = d.C11; k.s0 = d.C11; break;                                   // ADD
                 }
@@ -586,12 +588,16 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             b.muls += m3;
             emit_dmma(b, t, h);
         };
+        // Q7 before Q3, so that U2 is read out of C22 by both and never copied:
+        // 20 quarter reads and writes for the combination, where U1 stored
+        // twice and U2 moved to C21 took 22 (n = 16384 integers 'bbdd':
+        // 91.0 -> 89.7 ms).
         form(EW_FORM_T4S4);
         if (fold) {
-            folded(4, FOLD_ADD_DUP);
+            folded(4, FOLD_ADD);
         } else {
             sub(4);
-            comb(EW_ADD_DUP, [](const Nd &d, EwTask &t) { t.src[0] = d.C11; t.src[1] = d.Q; t.dst[0] = d.C22; t.dst[1] = d.C12; });
+            comb(EW_ADD, [](const Nd &d, EwTask &t) { t.src[0] = d.C11; t.src[1] = d.Q; t.dst[0] = d.C12; });
         }
         if (lead) {
             comb(EW_ADD, [&](const Nd &d, EwTask &t) { t.src[0] = d.C11; t.src[1] = Q2top; t.dst[0] = d.C11; });
@@ -600,28 +606,26 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
         form(EW_FORM_T5S5);
         if (fold) {
             folded(5, FOLD_ADD);
-        } else if (Q5top) {
-            comb(EW_ADD, [&](const Nd &d, EwTask &t) { t.src[0] = d.C22; t.src[1] = Q5top; t.dst[0] = d.C22; });
         } else {
-            sub(5);
-            comb(EW_ADD, [](const Nd &d, EwTask &t) { t.src[0] = d.C22; t.src[1] = d.Q; t.dst[0] = d.C22; });
+            if (!Q5top) sub(5);
+            comb(EW_ADD, [&](const Nd &d, EwTask &t) { t.src[0] = d.C12; t.src[1] = Q5top ? Q5top : d.Q; t.dst[0] = d.C22; });
         }
-        form(EW_FORM_T3S3);
-        if (fold) {
-            folded(3, FOLD_U2_Q3);
-        } else {
-            sub(3);
-            comb(EW_U2_Q3, [](const Nd &d, EwTask &t) { t.src[0] = d.C22; t.src[1] = d.C12; t.src[2] = d.Q; t.dst[0] = d.C21; t.dst[1] = d.C22; t.dst[2] = d.C12; });
-        }
-        if (top) emit_event(b, K_RECORD, EV_C_FIRST + 1);  // C22 final
         form(EW_FORM_S7);
         if (fold) {
             folded(7, FOLD_SUB);
         } else {
             sub(7);
-            comb(EW_SUB, [](const Nd &d, EwTask &t) { t.src[0] = d.C21; t.src[1] = d.Q; t.dst[0] = d.C21; });
+            comb(EW_SUB, [](const Nd &d, EwTask &t) { t.src[0] = d.C22; t.src[1] = d.Q; t.dst[0] = d.C21; });
         }
-        if (top) emit_event(b, K_RECORD, EV_C_FIRST + 2);  // C21 final
+        if (top) emit_event(b, K_RECORD, EV_C_FIRST + 1);  // C21 final
+        form(EW_FORM_T3S3);
+        if (fold) {
+            folded(3, FOLD_ADD2);
+        } else {
+            sub(3);
+            comb(EW_ADD2, [](const Nd &d, EwTask &t) { t.src[0] = d.C22; t.src[1] = d.C12; t.src[2] = d.Q; t.dst[0] = d.C22; t.dst[1] = d.C12; });
+        }
+        if (top) emit_event(b, K_RECORD, EV_C_FIRST + 2);  // C22 final
         form(EW_FORM_T6);
         if (fold) {
             folded(6, FOLD_ADD);
@@ -1802,7 +1806,7 @@ static caps_status rect_mm_locked(const double *A, const double *B, double *C, i
     std::vector<uint8_t> blob;
     for (size_t i = 0; i < walk.size(); i++) {
         if (last[walk[i].C] != i) continue;
-        const DmmaTask t{walk[i].A, walk[i].B, walk[i].C, nullptr, nullptr, nullptr, nullptr, FOLD_STORE, 0};
+        const DmmaTask t{walk[i].A, walk[i].B, walk[i].C, nullptr, nullptr, nullptr, FOLD_STORE, 0};
         const uint8_t *p = reinterpret_cast<const uint8_t *>(&t);
         blob.insert(blob.end(), p, p + sizeof(DmmaTask));
     }
@@ -1944,9 +1948,9 @@ caps_status caps_multiply_host(const double *A, const double *B, double *C, caps
         return st;
     }
     if (timeline) CAPS_CUDA_TRY(cudaEventRecord(hs->timing[3], s));
-    // C11 (quadrant 0), C22 (3), C21 (1) as they become final, then C12 (2)
+    // C11 (quadrant 0), C21 (1), C22 (3) as they become final, then C12 (2)
     // part by part
-    const int quad_of_event[3] = {0, 3, 1};
+    const int quad_of_event[3] = {0, 1, 3};
     for (int e = EV_C_FIRST; e < EV_C_FIRST + 3; e++) {
         CAPS_CUDA_TRY(cudaStreamWaitEvent(cs, g_host_events[e], 0));
         const int quad = quad_of_event[e - EV_C_FIRST];

@@ -131,17 +131,10 @@ __global__ void __launch_bounds__(32 * WM * WN) dmma_gemm_kernel(const DmmaTask 
                 switch (t.fold) {
                     case FOLD_ADD: t.C[x] = t.s0[x] + p; break;
                     case FOLD_SUB: t.C[x] = t.s0[x] - p; break;
-                    case FOLD_ADD_DUP: {
-                        const double v = t.s0[x] + p;
-                        t.C[x] = v;
-                        t.d1[x] = v;
-                        break;
-                    }
-                    case FOLD_U2_Q3: {
+                    case FOLD_ADD2: {
                         const double u2 = t.s0[x], u1 = t.s1[x];
-                        t.C[x] = u2;
-                        t.d1[x] = u2 + p;
-                        t.d2[x] = u1 + p;
+                        t.C[x] = u2 + p;
+                        t.d1[x] = u1 + p;
                         break;
                     }
                     default: t.C[x] = p;

@@ -126,11 +126,6 @@ __device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
         for (int k = 0; k < 4; k++) st2<VEC>(t.dst[k], i, two, make_double2(c0[k], c1[k]));
     } else if (OP == EW_COPY) {
         st2<VEC>(t.dst[0], i, two, ld2<VEC>(t.src[0], i, two));
-    } else if (OP == EW_ADD_DUP) {
-        double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
-        double2 r = make_double2(a.x + b.x, a.y + b.y);
-        st2<VEC>(t.dst[0], i, two, r);
-        st2<VEC>(t.dst[1], i, two, r);
     } else if (OP == EW_ADD) {
         double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
         st2<VEC>(t.dst[0], i, two, make_double2(a.x + b.x, a.y + b.y));
@@ -154,11 +149,6 @@ __device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
         form_lean<OP>(v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y, v[6].y, v[7].y, b0, b1);
         st2<VEC>(t.dst[0], i, two, make_double2(a0, b0));
         if (OP <= EW_FORM_T3S3) st2<VEC>(t.dst[1], i, two, make_double2(a1, b1));
-    } else if (OP == EW_U2_Q3) {
-        double2 u2 = ld2<VEC>(t.src[0], i, two), u1 = ld2<VEC>(t.src[1], i, two), q = ld2<VEC>(t.src[2], i, two);
-        st2<VEC>(t.dst[0], i, two, u2);
-        st2<VEC>(t.dst[1], i, two, make_double2(u2.x + q.x, u2.y + q.y));
-        st2<VEC>(t.dst[2], i, two, make_double2(u1.x + q.x, u1.y + q.y));
     }
 }
 
@@ -180,9 +170,8 @@ static int ew_nsrc(int op) {
     switch (op) {
         case EW_FORM_ST: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: case EW_FORM_S7:
         case EW_FORM_T6: return 8;
-        case EW_U2_Q3: return 3;
         case EW_COPY: return 1;
-        case EW_ADD_DUP: case EW_ADD: case EW_SUB: return 2;
+        case EW_ADD: case EW_SUB: return 2;
         case EW_ADD2: return 3;
         case EW_CALC_CIJ: return 7;
     }
@@ -191,8 +180,7 @@ static int ew_nsrc(int op) {
 static int ew_ndst(int op) {
     switch (op) {
         case EW_FORM_ST: return 8;
-        case EW_ADD_DUP: case EW_ADD2: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: return 2;
-        case EW_U2_Q3: return 3;
+        case EW_ADD2: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: return 2;
         case EW_CALC_CIJ: return 4;
     }
     return 1;
@@ -229,7 +217,6 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
         switch (op) {
             case EW_FORM_ST: launch_op<EW_FORM_ST>(vec, t, c, q, stream); break;
             case EW_COPY: launch_op<EW_COPY>(vec, t, c, q, stream); break;
-            case EW_ADD_DUP: launch_op<EW_ADD_DUP>(vec, t, c, q, stream); break;
             case EW_ADD: launch_op<EW_ADD>(vec, t, c, q, stream); break;
             case EW_SUB: launch_op<EW_SUB>(vec, t, c, q, stream); break;
             case EW_ADD2: launch_op<EW_ADD2>(vec, t, c, q, stream); break;
@@ -239,7 +226,6 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
             case EW_FORM_T3S3: launch_op<EW_FORM_T3S3>(vec, t, c, q, stream); break;
             case EW_FORM_S7: launch_op<EW_FORM_S7>(vec, t, c, q, stream); break;
             case EW_FORM_T6: launch_op<EW_FORM_T6>(vec, t, c, q, stream); break;
-            case EW_U2_Q3: launch_op<EW_U2_Q3>(vec, t, c, q, stream); break;
             default: return cudaErrorInvalidValue;
         }
         count_launch();
