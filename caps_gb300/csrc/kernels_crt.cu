@@ -701,11 +701,12 @@ __device__ __forceinline__ void reconstruct_step(const Section &t, int step, con
 // stages of K = 64 fit instead of four: that kernel's issuer waited for data a
 // third of the time.  49 leaves of 2048 at 17 moduli: 10.2 -> 8.53 ms (1405 ->
 // 1677 TFLOP/s of modular products); 49 leaves of 1536: 4.53 -> 3.80 ms (ncu;
-// the one-CTA kernel with its own reconstruction warps).  A last odd row tile leaves the second CTA's half unused.
-// The drain reduces each exact sum modulo p
-// (two values per packed fp32 instruction) and stores the balanced residue as
-// a byte, four columns to a word, into its section of the CTA's
-// product-residue tile; two tiles per CTA are used in turn.
+// the one-CTA kernel with its own reconstruction warps).  A last odd row tile
+// leaves the second CTA's half unused.
+// The drain reduces each exact sum modulo p (two values per packed fp32
+// instruction) and stores the balanced residue as a byte, four columns to a
+// word, into its section of the CTA's product-residue tile; two tiles per CTA
+// are used in turn.
 //
 // A drain warp also reconstructs the section it drained for the unit before:
 // ceil(32 / L) steps of 32 rows x 4 columns after each modulus's drain.  The
