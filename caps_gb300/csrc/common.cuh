@@ -87,6 +87,11 @@ enum EwOp : int {
     EW_FORM_T3S3 = 8,  // dst0 = A21+A22,       dst1 = B12-B11
     EW_FORM_S7 = 9,    // dst0 = (B22-(B12-B11))-B21
     EW_FORM_T6 = 10,   // dst0 = A12-((A21+A22)-A11)
+    // the operand sums of a 'd' step in two passes, the second from T4 and S4
+    // and in place: src = A11 A21 A22 B11 B12 B22, dst = T3 S3 T4 S4 T5 S5;
+    // then src = T4 A12 S4 B21, dst0 = T6 = A12-T4, dst1 = S7 = S4-B21
+    EW_FORM_T345 = 11,
+    EW_FORM_T6S7 = 12,
 };
 
 struct EwTask {

@@ -383,6 +383,8 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
     // steps that overlap host copies (below) stay in sequence
     const bool overlaps = b.host_overlap && P.size() == 1 &&
                           ((b.overlap_stage == 0 && b.ops.empty()) || b.overlap_stage == 1);
+    // plain-form leaves right below: the folds run in the products' epilogues
+    const bool fold = !overlaps && nrec == 1 && b.opt.form == CAPS_FORM_PLAIN && (b.bs == 1 || b.bs == h);
     if (c == 'b' || c == 'B' || hyb || (!overlaps && merges(b, P.size(), h))) {
         // strassenBFS (multiply.cpp:212-310) on one GPU: 7 subproducts as one
         // batch.  Q1..Q4 are written straight into the C quadrants (calcCij
@@ -433,11 +435,60 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             }
         }
         emit_ew(b, EW_CALC_CIJ, cij, q);
+    } else if (!overlaps && !fold) {
+        // strassenDFS (multiply.cpp:409-454) with 3 quarter buffers X, Y, Q a
+        // node: with the C quadrants they are seven, which hold the operand
+        // sums first and the seven products in the end, Q1 = A11 B11 and
+        // Q2 = A12 B21 last, as they need no sums; then calcCij, as in a 'b'
+        // step.  29 quarter reads and writes around the products (12 + 6 for
+        // the sums, 11 for C) where each pair formed just before its product
+        // and each product folded into C at once took 50; a 'b' step, with 8
+        // buffers more, takes 27.  n = 16384 integers 'bbdd': 89.6 -> 77.9 ms a
+        // multiply, n = 16384 float, whose top step is a 'd', 96.8 -> 96.0.
+        //   buffer   X       Y      C11      C12      C21      C22     Q
+        //   sums     T3      S3     T4       S4       T5       S5
+        //            Q4 (2)  Q5     T6, Q1   S7, Q2   Q6       Q7      Q3 (1)
+        std::vector<double *> W(P.size());
+        for (double *&w : W) w = b.alloc(3 * q);
+        auto pass = [&](int op, auto fill) {
+            std::vector<EwTask> t(P.size());
+            for (size_t i = 0; i < P.size(); i++) t[i] = fill(P[i], W[i], W[i] + q, W[i] + 2 * q);
+            emit_ew(b, op, t, q);
+        };
+        auto product = [&](auto of) {
+            std::vector<Prob> ch;
+            for (size_t i = 0; i < P.size(); i++) ch.push_back(of(P[i], W[i], W[i] + q, W[i] + 2 * q));
+            build(b, ch, h, nrec - 1, pat + 1);
+        };
+        pass(EW_FORM_T345, [q](const Prob &p, double *X, double *Y, double *) {
+            return EwTask{{p.A, p.A + q, p.A + 3 * q, p.B, p.B + 2 * q, p.B + 3 * q},
+                          {X, Y, p.C, p.C + 2 * q, p.C + q, p.C + 3 * q}};
+        });
+        product([](const Prob &, double *X, double *Y, double *Q) { return Prob{X, Y, Q}; });                   // Q3
+        product([q](const Prob &p, double *X, double *, double *) { return Prob{p.C, p.C + 2 * q, X}; });       // Q4
+        pass(EW_FORM_T6S7, [q](const Prob &p, double *, double *, double *) {
+            return EwTask{{p.C, p.A + 2 * q, p.C + 2 * q, p.B + q}, {p.C, p.C + 2 * q}};
+        });
+        product([q](const Prob &p, double *, double *Y, double *) { return Prob{p.C + q, p.C + 3 * q, Y}; });   // Q5
+        product([q](const Prob &p, double *, double *, double *) { return Prob{p.C, p.B + 3 * q, p.C + q}; });  // Q6
+        product([q](const Prob &p, double *, double *, double *) {                                              // Q7
+            return Prob{p.A + 3 * q, p.C + 2 * q, p.C + 3 * q};
+        });
+        product([](const Prob &p, double *, double *, double *) { return Prob{p.A, p.B, p.C}; });               // Q1
+        product([q](const Prob &p, double *, double *, double *) {                                              // Q2
+            return Prob{p.A + 2 * q, p.B + q, p.C + 2 * q};
+        });
+        pass(EW_CALC_CIJ, [q](const Prob &p, double *X, double *Y, double *Q) {
+            return EwTask{{p.C, p.C + 2 * q, Q, X, Y, p.C + q, p.C + 3 * q},
+                          {p.C, p.C + 2 * q, p.C + q, p.C + 3 * q}};
+        });
     } else {
-        // strassenDFS (multiply.cpp:409-454), memory-lean: each operand pair
-        // is formed just before its subproduct into X, Y, the product goes to
-        // Q, and U1 / U2 / U3 live in C quadrants not yet final -- 3 quarter
-        // buffers per node.  Per element the sums, products and their order
+        // The same step with the products folded into C one by one, where that
+        // runs in the epilogues of plain-form leaves, or lets the copies of a
+        // host call overlap the subproducts.  Each operand pair is formed just
+        // before its subproduct into X, Y, the product goes to Q, and U1 / U2
+        // / U3 live in C quadrants not yet final -- 3 quarter buffers per
+        // node.  Per element the sums, products and their order
         // are the reference's:
         //   C11=Q1; C12=U1=C11+Q4; C22=U2=C12+Q5; C21=U2-Q7;
         //   C22=U2+Q3, C12=U3=C12+Q3; C12=U3+Q6; C11+=Q2.
@@ -484,7 +535,6 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             for (const Nd &d : nd) {
                 switch (which) {
                     case 1: ch.push_back({d.A11, d.B11, d.C11}); break;
-                    case 2: ch.push_back({d.A12, d.B21, d.Q}); break;
                     case 3: case 4: case 5: ch.push_back({d.X, d.Y, d.Q}); break;
                     case 6: ch.push_back({d.X, d.B22, d.Q}); break;
                     case 7: ch.push_back({d.A22, d.X, d.Q}); break;
@@ -555,14 +605,12 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
         // Plain-form leaves right below a step that is not overlapping host
         // copies: each fold that consumes a product (C12 = C11 + Q4,
         // C22 = C12 + Q5, C21 = C22 - Q7, C22 += Q3 with C12 += Q3, C12 += Q6,
-        // C11 += Q2) runs
-        // in that product's DMMA epilogue, on the accumulator, instead of as a
-        // pass over the stored product: the same FP64 operations in the same
-        // order, so the same bits, without the product's round trip to HBM.
-        // (Split-form leaves keep the passes: in the residue GEMM's
-        // reconstruction warps the folds' FP64 adds slowed the GEMM more than
-        // the passes cost.)
-        const bool fold = !lead && nrec == 1 && b.opt.form == CAPS_FORM_PLAIN && (b.bs == 1 || b.bs == h);
+        // C11 += Q2) runs in that product's DMMA epilogue, on the accumulator,
+        // instead of as a pass over the stored product: the same FP64
+        // operations in the same order, so the same bits, without the
+        // product's round trip to HBM.  (Split-form leaves keep the passes: in
+        // the residue GEMM the folds' FP64 adds slowed the GEMM more than the
+        // passes cost.)
         auto folded = [&](int which, int mode) {
             std::vector<DmmaTask> t;
             for (const Nd &d : nd) {
@@ -588,10 +636,7 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             b.muls += m3;
             emit_dmma(b, t, h);
         };
-        // Q7 before Q3, so that U2 is read out of C22 by both and never copied:
-        // 20 quarter reads and writes for the combination, where U1 stored
-        // twice and U2 moved to C21 took 22 (n = 16384 integers 'bbdd':
-        // 91.0 -> 89.7 ms).
+        // Q7 before Q3, so that U2 is read out of C22 by both and never copied
         form(EW_FORM_T4S4);
         if (fold) {
             folded(4, FOLD_ADD);
@@ -642,12 +687,7 @@ static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, c
             sub(6);
             comb(EW_ADD, [](const Nd &d, EwTask &t) { t.src[0] = d.C12; t.src[1] = d.Q; t.dst[0] = d.C12; });
         }
-        if (fold) {
-            folded(2, FOLD_ADD);
-        } else if (!lead) {
-            sub(2);
-            comb(EW_ADD, [](const Nd &d, EwTask &t) { t.src[0] = d.C11; t.src[1] = d.Q; t.dst[0] = d.C11; });
-        }
+        if (fold) folded(2, FOLD_ADD);
     }
     b.release(mk);
 }

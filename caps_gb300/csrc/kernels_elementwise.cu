@@ -44,6 +44,16 @@ __device__ __forceinline__ void calc_cij(const double *q, double *c) {
     c[0] = c11; c[1] = c12; c[2] = c21; c[3] = c22;
 }
 
+// The same sums but T6 and S7, which a 'd' step forms from T4 and S4 later.
+__device__ __forceinline__ void form_t345(double a11, double a21, double a22, double b11, double b12, double b22,
+                                          double *o) {
+    double t3 = a21 + a22;
+    double s3 = b12 - b11;
+    o[0] = t3; o[1] = s3;
+    o[2] = t3 - a11; o[3] = b22 - s3;
+    o[4] = a11 - a21; o[5] = b22 - b12;
+}
+
 // Operand sums of the memory-lean 'd' step: the same formulas, in the same
 // evaluation order, as the reference's (multiply.cpp:421-435).
 template <int OP>
@@ -138,6 +148,20 @@ __device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
         double2 r1 = make_double2(b.x + q.x, b.y + q.y);
         st2<VEC>(t.dst[0], i, two, r0);
         st2<VEC>(t.dst[1], i, two, r1);
+    } else if (OP == EW_FORM_T345) {
+        double2 v[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) v[k] = ld2<VEC>(t.src[k], i, two);
+        double o0[6], o1[6];
+        form_t345(v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, v[5].x, o0);
+        form_t345(v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y, o1);
+#pragma unroll
+        for (int k = 0; k < 6; k++) st2<VEC>(t.dst[k], i, two, make_double2(o0[k], o1[k]));
+    } else if (OP == EW_FORM_T6S7) {
+        double2 t4 = ld2<VEC>(t.src[0], i, two), a12 = ld2<VEC>(t.src[1], i, two);
+        double2 s4 = ld2<VEC>(t.src[2], i, two), b21 = ld2<VEC>(t.src[3], i, two);
+        st2<VEC>(t.dst[0], i, two, make_double2(a12.x - t4.x, a12.y - t4.y));
+        st2<VEC>(t.dst[1], i, two, make_double2(s4.x - b21.x, s4.y - b21.y));
     } else if (OP >= EW_FORM_T4S4 && OP <= EW_FORM_T6) {
         // only the sources the formula reads are loaded
         double2 v[8];
@@ -170,6 +194,8 @@ static int ew_nsrc(int op) {
     switch (op) {
         case EW_FORM_ST: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: case EW_FORM_S7:
         case EW_FORM_T6: return 8;
+        case EW_FORM_T345: return 6;
+        case EW_FORM_T6S7: return 4;
         case EW_COPY: return 1;
         case EW_ADD: case EW_SUB: return 2;
         case EW_ADD2: return 3;
@@ -180,7 +206,8 @@ static int ew_nsrc(int op) {
 static int ew_ndst(int op) {
     switch (op) {
         case EW_FORM_ST: return 8;
-        case EW_ADD2: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: return 2;
+        case EW_FORM_T345: return 6;
+        case EW_FORM_T6S7: case EW_ADD2: case EW_FORM_T4S4: case EW_FORM_T5S5: case EW_FORM_T3S3: return 2;
         case EW_CALC_CIJ: return 4;
     }
     return 1;
@@ -226,6 +253,8 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
             case EW_FORM_T3S3: launch_op<EW_FORM_T3S3>(vec, t, c, q, stream); break;
             case EW_FORM_S7: launch_op<EW_FORM_S7>(vec, t, c, q, stream); break;
             case EW_FORM_T6: launch_op<EW_FORM_T6>(vec, t, c, q, stream); break;
+            case EW_FORM_T345: launch_op<EW_FORM_T345>(vec, t, c, q, stream); break;
+            case EW_FORM_T6S7: launch_op<EW_FORM_T6S7>(vec, t, c, q, stream); break;
             default: return cudaErrorInvalidValue;
         }
         count_launch();
