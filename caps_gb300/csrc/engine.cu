@@ -360,7 +360,7 @@ static void build_leaf(Builder &b, const std::vector<Prob> &P, int64_t m) {
 // element the same operations in the same order): with no budget in the way,
 // steps whose batch takes at most 128 MiB as 'b' steps run as such: one node of
 // quarters up to 1234 (split form, us a call, in sequence -> merged: n = 392
-// 'bd' 377 -> 143, n = 2048 'd' 750 -> 450, n = 2400 'd' 966 -> 735; at n = 4096 a
+// 'bd' 307 -> 131, n = 2048 'd' 590 -> 410, n = 2400 'd' 820 -> 701; at n = 4096 a
 // product of its own takes 85 % of the pairs).  Plain form: quarters up to 154
 // (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger leaves fill the FP64
 // pipe one at a time.
