@@ -358,15 +358,17 @@ static void build_leaf(Builder &b, const std::vector<Prob> &P, int64_t m) {
 // a node instead of 11.  Where those are small the sequence only leaves the
 // GPU idle, launch after launch, and a 'b' step gives the same bits (per
 // element the same operations in the same order): with no budget in the way,
-// steps whose batch takes at most 128 MiB as 'b' steps run as such: one node of
-// quarters up to 1234 (split form, us a call, in sequence -> merged: n = 392
-// 'bd' 307 -> 131, n = 2048 'd' 590 -> 410, n = 2400 'd' 820 -> 701; at n = 4096 a
-// product of its own takes 85 % of the pairs).  Plain form: quarters up to 154
+// steps whose batch takes at most 1 GiB as 'b' steps run as such: one node of
+// quarters up to 3490 (split form, us a call, in sequence -> merged: n = 392
+// 'bd' 307 -> 131, n = 2400 'd' 820 -> 701, n = 4096 'd' 2190 -> 1893, 'dd' 4118 ->
+// 2587, n = 5000 'd' 6265 -> 5362, n = 6144 'd' 9853 -> 9301; beyond, less than 5 %:
+// n = 8192 'bbd', 4.2 GiB, 18370 -> 17680).  With the scratch of the larger launch
+// that is some 6 GiB at the bound.  Plain form: quarters up to 154
 // (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger leaves fill the FP64
 // pipe one at a time.
 static bool merges(const Builder &b, size_t nodes, int64_t h) {
     if (!b.merge_small || (b.opt.form == CAPS_FORM_PLAIN && h > 154)) return false;
-    return (int64_t)nodes * 11 * h * h * (int64_t)sizeof(double) <= (int64_t)128 << 20;
+    return (int64_t)nodes * 11 * h * h * (int64_t)sizeof(double) <= (int64_t)1 << 30;
 }
 
 static void build(Builder &b, const std::vector<Prob> &P, int64_t n, int nrec, const char *pat) {

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("form", ["plain", "split"])
 @pytest.mark.parametrize("n,r,bs,pat,hybrid", [(56, 2, 1, "dd", 1), (56, 2, 7, "dd", 1), (392, 2, 7, "bd", 1),
                                                (112, 3, 1, "hdd", 1), (112, 3, 1, "hdd", 3), (310, 1, 1, "d", 1),
-                                               (1032, 3, 1, "ddd", 1)])
+                                               (1032, 3, 1, "ddd", 1), (2600, 1, 1, "d", 1), (2080, 2, 1, "bd", 1)])
 def test_merged_steps_bit_identical_to_steps_in_sequence(caps, cuda, form, n, r, bs, pat, hybrid):
     import torch
     rng = np.random.default_rng(n + r)
