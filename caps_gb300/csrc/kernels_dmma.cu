@@ -165,14 +165,20 @@ static cudaError_t launch_dmma_shape(const DmmaTask *tasks_dev, int count, int m
 // 121390 -> 96920 (32 alone: 97100; 93100 at the pipe's rate), leaf of 1500 7040
 // -> 6270, 4096 x 2048 x 3072 48910 -> 46890, n = 56 'dd' 1471 -> 437 (with the
 // skipped padding).
+//
+// Row tiles go in grid.y, which holds 65535 of them: a tall, narrow product
+// (the rectangular base case; 1048561 x 8 is 65536 row tiles of 16) takes the
+// best side whose row tiles fit.
 static int pick_tile(int count, int m, int n) {
+    const int64_t max_rows = 65535;
     const int sides[3] = {64, 32, 16};
     const double cost[3] = {1.0, 1.01, 1.005};
     int best = 64;
     double best_t = 0.0;
     for (int i = 0; i < 3; i++) {
-        const int64_t t = sides[i];
-        const int64_t ctas = ((m + t - 1) / t) * ((n + t - 1) / t) * (int64_t)count;
+        const int64_t t = sides[i], rows = (m + t - 1) / t;
+        if (i > 0 && rows > max_rows) continue;
+        const int64_t ctas = rows * ((n + t - 1) / t) * (int64_t)count;
         const double busiest = (double)((ctas + 151) / 152) * (double)(t * t) * cost[i];
         if (i == 0 || busiest < best_t) {
             best = sides[i];
