@@ -288,9 +288,16 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
 // 340 -> 170, bs 16 573 -> 183, bs 32 570 -> 176, bs 64 299 -> 176; n = 6272 in bs 7
 // 340 -> 152 (93).  Runs of 128 as elements take 172 against 221, of 250 as
 // runs 160 against 174, hence RUN_MIN.
+//
+// From n^2 = 2^31 on positions take 64-bit divisions, which cost several times
+// the copy: a run pays them once, so blocks from RUN_MIN_LARGE on go by runs
+// there, and with the shorter ones in kernels of their own (46 registers; the
+// batched loops' 80 leave half the warps to hide the divisions).  ms one way
+// at n = 46592 (copy rate: 5.0), by elements beside the batched loops -> here:
+// bs 64 20.1 -> 7.9, 128 20.1 -> 6.5, 32 20.1 -> 14.7 (elements: 14.8).
 // ---------------------------------------------------------------------------
-constexpr int RUN_BATCH = 8;  // loads a lane has in flight
 constexpr int RUN_MIN = 160;  // runs from here on take a warp each
+constexpr int RUN_MIN_LARGE = 32;  // the same from n^2 = 2^31 on
 
 // x / d for 0 <= x < 2^31 by a multiplication (Granlund and Montgomery's
 // invariant division): with s = ceil(log2 d), m = floor(2^32 (2^s - d) / d) + 1,
@@ -315,6 +322,8 @@ struct ReorderGeom {
     int bs;             // effective block size (m when bs == 1 or bs == m)
     int nb;             // blocks per leaf side
     bool small;         // n^2 < 2^31: the divisions below
+    bool by_runs;       // a warp per run; else a thread per element or pair
+    bool short_large;   // runs below RUN_MIN, n^2 >= 2^31: the kernels for 64-bit positions
     FastDiv dbs, dnb, druns;  // by bs, nb and the runs of a leaf
 };
 
@@ -344,7 +353,7 @@ __device__ __forceinline__ int64_t caps_to_colmajor_index(const ReorderGeom &g, 
 }
 
 // A run by a warp, in batches of loads issued before their stores.
-template <typename T>
+template <int RUN_BATCH, typename T>
 __device__ __forceinline__ void copy_run(const T *__restrict__ s, T *__restrict__ d, int count, int lane) {
     for (int k = lane; k < count; k += 32 * RUN_BATCH) {
         T v[RUN_BATCH];
@@ -357,8 +366,8 @@ __device__ __forceinline__ void copy_run(const T *__restrict__ s, T *__restrict_
     }
 }
 
-// one warp per run of bs >= 32 doubles
-template <bool TO_CAPS>
+// one warp per run of bs doubles
+template <bool TO_CAPS, int RUN_BATCH>
 __device__ __forceinline__ void reorder_runs(const double *__restrict__ s, double *__restrict__ d,
                                              const ReorderGeom &g, int64_t warp0, int64_t nwarps) {
     const int lane = threadIdx.x & 31;
@@ -368,9 +377,9 @@ __device__ __forceinline__ void reorder_runs(const double *__restrict__ s, doubl
         const double *src = s + (TO_CAPS ? cm : cp);
         double *dst = d + (TO_CAPS ? cp : cm);
         if (((g.bs & 1) == 0) && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
-            copy_run(reinterpret_cast<const double2 *>(src), reinterpret_cast<double2 *>(dst), g.bs / 2, lane);
+            copy_run<RUN_BATCH>(reinterpret_cast<const double2 *>(src), reinterpret_cast<double2 *>(dst), g.bs / 2, lane);
         } else {
-            copy_run(src, dst, g.bs, lane);
+            copy_run<RUN_BATCH>(src, dst, g.bs, lane);
         }
     }
 }
@@ -417,16 +426,9 @@ __device__ __forceinline__ void reorder_elements32(const double *__restrict__ s,
 }
 
 template <bool TO_CAPS>
-__device__ __forceinline__ void reorder_elements(const double *__restrict__ s, double *__restrict__ d,
-                                                 const ReorderGeom &g, int64_t t0, int64_t nthreads) {
+__device__ __forceinline__ void reorder_elements64(const double *__restrict__ s, double *__restrict__ d,
+                                                   const ReorderGeom &g, int64_t t0, int64_t nthreads) {
     const int64_t total = g.n * g.n;
-    if (g.small) {
-        if ((g.bs & 1) == 0 && (((uintptr_t)s | (uintptr_t)d) & 15) == 0)
-            reorder_elements32<TO_CAPS, double2>(s, d, g, t0, nthreads);
-        else
-            reorder_elements32<TO_CAPS, double>(s, d, g, t0, nthreads);
-        return;
-    }
     for (int64_t idx = t0; idx < total; idx += nthreads) {
         int64_t cm = caps_to_colmajor_index(g, idx);
         if (TO_CAPS)
@@ -436,19 +438,26 @@ __device__ __forceinline__ void reorder_elements(const double *__restrict__ s, d
     }
 }
 
-template <bool TO_CAPS>
+// SHORT_LARGE: g.short_large (a kernel of its own)
+template <bool TO_CAPS, bool SHORT_LARGE>
+__device__ __forceinline__ void reorder(const double *__restrict__ s, double *__restrict__ d, const ReorderGeom &g) {
+    const int64_t thread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
+    if (g.by_runs)
+        reorder_runs<TO_CAPS, SHORT_LARGE ? 1 : 8>(s, d, g, thread >> 5, nthreads >> 5);
+    else if constexpr (SHORT_LARGE)
+        reorder_elements64<TO_CAPS>(s, d, g, thread, nthreads);
+    else if ((g.bs & 1) == 0 && (((uintptr_t)s | (uintptr_t)d) & 15) == 0)
+        reorder_elements32<TO_CAPS, double2>(s, d, g, thread, nthreads);
+    else
+        reorder_elements32<TO_CAPS, double>(s, d, g, thread, nthreads);
+}
+
+template <bool TO_CAPS, bool SHORT_LARGE>
 __global__ void __launch_bounds__(256) reorder_kernel(const double *const *__restrict__ src,
                                                       double *const *__restrict__ dst,
                                                       ReorderGeom g) {
     chain_wait();
-    const double *s = src[blockIdx.y];
-    double *d = dst[blockIdx.y];
-    if (g.bs >= RUN_MIN)
-        reorder_runs<TO_CAPS>(s, d, g, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                              ((int64_t)gridDim.x * blockDim.x) >> 5);
-    else
-        reorder_elements<TO_CAPS>(s, d, g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
-                                  (int64_t)gridDim.x * blockDim.x);
+    reorder<TO_CAPS, SHORT_LARGE>(src[blockIdx.y], dst[blockIdx.y], g);
 }
 
 static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
@@ -460,6 +469,8 @@ static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
     g.bs = (bs == 1 || bs == g.m) ? (int)g.m : (int)bs;
     g.nb = (int)(g.m / g.bs);
     g.small = n * n < ((int64_t)1 << 31);
+    g.by_runs = g.bs >= (g.small ? RUN_MIN : RUN_MIN_LARGE);
+    g.short_large = !g.small && g.bs < RUN_MIN;
     g.dbs = fast_div(g.bs);
     g.dnb = fast_div(g.nb);
     g.druns = fast_div(g.small ? g.mm / g.bs : 1);
@@ -469,7 +480,7 @@ static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
 // grid: enough blocks for a run (or element) per thread, at most 8 blocks of
 // 256 threads per SM for all matrices together
 static unsigned reorder_blocks(const ReorderGeom &g, int count) {
-    const int64_t items = g.bs >= RUN_MIN ? g.n * g.n / g.bs * 32 : g.n * g.n;
+    const int64_t items = g.by_runs ? g.n * g.n / g.bs * 32 : g.n * g.n;
     int64_t blocks = (items + 255) / 256;
     int64_t cap = (int64_t)152 * 32 / count;
     if (cap < 1) cap = 1;
@@ -483,33 +494,26 @@ cudaError_t launch_reorder(const double *const *src_dev, double *const *dst_dev,
     if (count <= 0) return cudaSuccess;
     ReorderGeom g = make_geom(n, nrec, bs);
     dim3 grid(reorder_blocks(g, count), (unsigned)count);
-    if (to_caps)
-        launch_chained(reorder_kernel<true>, grid, 256, 0, stream, src_dev, dst_dev, g);
-    else
-        launch_chained(reorder_kernel<false>, grid, 256, 0, stream, src_dev, dst_dev, g);
+    auto kernel = to_caps ? (g.short_large ? reorder_kernel<true, true> : reorder_kernel<true, false>)
+                          : (g.short_large ? reorder_kernel<false, true> : reorder_kernel<false, false>);
+    launch_chained(kernel, grid, 256, 0, stream, src_dev, dst_dev, g);
     count_launch();
     return cudaGetLastError();
 }
 
-template <bool TO_CAPS>
+template <bool TO_CAPS, bool SHORT_LARGE>
 __global__ void __launch_bounds__(256) reorder_one_kernel(const double *__restrict__ s,
                                                           double *__restrict__ d, ReorderGeom g) {
-    if (g.bs >= RUN_MIN)
-        reorder_runs<TO_CAPS>(s, d, g, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                              ((int64_t)gridDim.x * blockDim.x) >> 5);
-    else
-        reorder_elements<TO_CAPS>(s, d, g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
-                                  (int64_t)gridDim.x * blockDim.x);
+    reorder<TO_CAPS, SHORT_LARGE>(s, d, g);
 }
 
 cudaError_t launch_reorder_one(const double *src, double *dst, int64_t n, int nrec, int64_t bs,
                                bool to_caps, cudaStream_t stream) {
     ReorderGeom g = make_geom(n, nrec, bs);
     const unsigned blocks = reorder_blocks(g, 1);
-    if (to_caps)
-        reorder_one_kernel<true><<<blocks, 256, 0, stream>>>(src, dst, g);
-    else
-        reorder_one_kernel<false><<<blocks, 256, 0, stream>>>(src, dst, g);
+    auto kernel = to_caps ? (g.short_large ? reorder_one_kernel<true, true> : reorder_one_kernel<true, false>)
+                          : (g.short_large ? reorder_one_kernel<false, true> : reorder_one_kernel<false, false>);
+    kernel<<<blocks, 256, 0, stream>>>(src, dst, g);
     count_launch();
     return cudaGetLastError();
 }
