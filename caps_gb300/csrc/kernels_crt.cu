@@ -1126,21 +1126,22 @@ cudaError_t launch_crt_slice(const LeafTask *tasks_dev, int count, int m, SplitP
     return launch_chained(crt_slice_kernel, grid, 256, 0, stream, tasks_dev, (char *)workspace, g);
 }
 
-cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
-                            unsigned int *status_dev, int num_sms, cudaStream_t stream, int starve) {
-    Geo g = make_geo(m, count, p.scheme);
-    cudaError_t e = crt_prepare();
-    if (e != cudaSuccess) return e;
+// units of a leaf: two row tiles by a column tile
+static int64_t leaf_units(const Geo &g) { return (int64_t)((g.mtiles + 1) / 2) * g.rtiles; }
+
+// One GEMM launch over g.count leaves, and the combine kernel after it for items.
+static cudaError_t launch_crt_gemm_leaves(const LeafTask *tasks_dev, char *ws, const Geo &g, unsigned int *status_dev,
+                                          int num_sms, cudaStream_t stream, int starve) {
     // the leaves' plane blocks as rows of 512 bytes (every plane starts on one)
     CUtensorMap planes;
-    const cuuint64_t dims[2] = {MAP_ROW / 2, (cuuint64_t)((size_t)count * g.dg_per_leaf / MAP_ROW)};
+    const cuuint64_t dims[2] = {MAP_ROW / 2, (cuuint64_t)((size_t)g.count * g.dg_per_leaf / MAP_ROW)};
     const cuuint64_t strides[1] = {MAP_ROW};
     const cuuint32_t box[2] = {MAP_ROW / 2, MAP_BOX}, ones[2] = {1, 1};
-    if (g_encode_tiled(&planes, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (char *)workspace + g.dg_base, dims, strides, box,
-                       ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                       CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    if (g_encode_tiled(&planes, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, ws + g.dg_base, dims, strides, box, ones,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    const int64_t units = (int64_t)((g.mtiles + 1) / 2) * g.rtiles * count;
+    const int64_t units = leaf_units(g) * g.count;
     int pairs = num_sms / 2;
     if (pairs > ZCTA_MAX / 2) pairs = ZCTA_MAX / 2;  // two product-residue tiles per CTA
     // Whole units to a pair, or (unit, modulus) items and the combine kernel:
@@ -1155,16 +1156,44 @@ cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitPa
     const size_t smem = (size_t)RNSTAGE * RSTAGE_BYTES + 1024 + 1024;
     const int64_t want = split ? units * LMAX : units;
     if (want < pairs) pairs = (int)want;
-    e = launch_chained(crt_gemm_kernel, 2 * pairs, RGEMM_THREADS, smem, stream, tasks_dev, (char *)workspace, g, planes,
-                       status_dev, split, starve);
+    cudaError_t e = launch_chained(crt_gemm_kernel, 2 * pairs, RGEMM_THREADS, smem, stream, tasks_dev, ws, g, planes,
+                                   status_dev, split, starve);
     count_launch();
     if (e != cudaSuccess) return e;
     if (split) {
-        e = launch_chained(crt_combine_kernel, (unsigned)(units * 2 * 64), 128, 0, stream, tasks_dev, (char *)workspace, g);
+        e = launch_chained(crt_combine_kernel, (unsigned)(units * 2 * 64), 128, 0, stream, tasks_dev, ws, g);
         count_launch();
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitParams p, void *workspace,
+                            unsigned int *status_dev, int num_sms, cudaStream_t stream, int starve) {
+    const Geo g = make_geo(m, count, p.scheme);
+    cudaError_t e = crt_prepare();
+    if (e != cudaSuccess) return e;
+    // Leaves of one row tile leave a unit's second CTA and half the columns of
+    // the first without work, so of a pair's 16 drain warps 4 at most
+    // reconstruct.  Many of them go as items, in as few equal launches as the
+    // product-residue tiles allow: the combine kernel spreads their
+    // reconstruction over the GPU.  us of the GEMM and combine kernels at 17
+    // moduli, units -> items (with one-CTA MMAs before both): 16807 leaves of 128
+    // 14900 -> 11210 (13600), 2401 of 128 2172 -> 1603 (2000), 2401 of 96 1808 ->
+    // 1428 (1780), 16807 of 40 8480 -> 7340 (9580).  Leaves of up to 32
+    // reconstruct too little for it: integers of 11 bits, 16807 of 16 2870 ->
+    // 3650, of 32 3610 -> 3770, of 40 4080 -> 3870.
+    const bool thin = leaf_units(g) == 1 && m > 32 && m <= TM;
+    const int launches = thin ? (count + ZCTA_MAX - 1) / ZCTA_MAX : 1, per = (count + launches - 1) / launches;
+    for (int first = 0; first < count; first += per) {
+        Geo part = g;
+        part.count = count - first < per ? count - first : per;
+        part.sc_base += (size_t)first * g.sc_per_leaf;
+        part.dg_base += (size_t)first * g.dg_per_leaf;
+        e = launch_crt_gemm_leaves(tasks_dev + first, (char *)workspace, part, status_dev, num_sms, stream, starve);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace caps
