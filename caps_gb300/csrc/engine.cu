@@ -357,15 +357,15 @@ static void build_leaf(Builder &b, const std::vector<Prob> &P, int64_t m) {
 // A 'd' step runs its seven subproducts in sequence to hold 3 quarter buffers
 // a node instead of 11.  Where those are small the sequence only leaves the
 // GPU idle, launch after launch, and a 'b' step gives the same bits (per
-// element the same operations in the same order): with no budget in the way,
-// steps whose batch takes at most 1 GiB as 'b' steps run as such: one node of
-// quarters up to 3490 (split form, us a call, in sequence -> merged: n = 392
-// 'bd' 307 -> 131, n = 2400 'd' 820 -> 701, n = 4096 'd' 2190 -> 1893, 'dd' 4118 ->
-// 2587, n = 5000 'd' 6265 -> 5362, n = 6144 'd' 9853 -> 9301; beyond, less than 5 %:
-// n = 8192 'bbd', 4.2 GiB, 18370 -> 17680).  With the scratch of the larger launch
-// that is some 6 GiB at the bound.  Plain form: quarters up to 154
-// (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger leaves fill the FP64
-// pipe one at a time.
+// element the same operations in the same order): with no budget in the way
+// and memory to spare (room_to_merge), steps whose batch takes at most 1 GiB as
+// 'b' steps run as such: one node of quarters up to 3490 (split form, us a call,
+// in sequence -> merged: n = 392 'bd' 307 -> 131, n = 2400 'd' 820 -> 701, n = 4096
+// 'd' 2190 -> 1893, 'dd' 4118 -> 2587, n = 5000 'd' 6265 -> 5362, n = 6144 'd' 9853
+// -> 9301; beyond, less than 5 %: n = 8192 'bbd', 4.2 GiB, 18370 -> 17680).  With
+// the scratch of the larger launches that is up to some 8 GB.  Plain form:
+// quarters up to 154 (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger
+// leaves fill the FP64 pipe one at a time.
 static bool merges(const Builder &b, size_t nodes, int64_t h) {
     if (!b.merge_small || (b.opt.form == CAPS_FORM_PLAIN && h > 154)) return false;
     return (int64_t)nodes * 11 * h * h * (int64_t)sizeof(double) <= (int64_t)1 << 30;
@@ -1042,6 +1042,28 @@ static caps_status check_device_status(cudaStream_t s, bool counts) {
 
 static caps_status resolve_operand_bits(const caps_desc &d, caps_options &o);
 
+static size_t arena_here() {  // bytes the arena has on the current device
+    int dev = 0;
+    return g_arena.ptr && cudaGetDevice(&dev) == cudaSuccess && g_arena.device == dev ? g_arena.size : 0;
+}
+
+// Whether the arena may grow to `merged` bytes for merged 'd' steps, where the
+// steps in sequence take `lean`, with no limit from the caller: a 'd' is how a
+// caller keeps memory for other uses, so what merging adds stays within a
+// sixteenth of the free device memory (on an empty GPU all merges fit: they
+// add up to some 8 GB), and nothing is allocated under a stream capture.
+static bool room_to_merge(size_t lean, size_t merged, cudaStream_t s) {
+    if (merged <= lean) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+        cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return merged - lean <= (free_bytes + arena_here()) / 16;  // the arena is freed before it grows
+}
+
 static caps_status multiply_dev_locked(const double *A, const double *B, double *C, caps_desc d,
                                        const char *pattern, const caps_options &o_in, cudaStream_t s,
                                        bool sync_status, bool host_overlap = false,
@@ -1065,6 +1087,13 @@ static caps_status multiply_dev_locked(const double *A, const double *B, double 
     if (o.workspace_limit > 0 && (long long)pl.ws_bytes > o.workspace_limit) {
         merge = false;  // every step as the pattern has it
         CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, pl, host_overlap, extras, merge));
+    } else if (o.workspace_limit <= 0 && arena_here() < pl.total) {
+        Planned lean;
+        CAPS_TRY(plan(A, B, C, d, pat, o, nullptr, lean, host_overlap, extras, false));
+        if (!room_to_merge(lean.total, pl.total, s)) {
+            merge = false;
+            pl = lean;
+        }
     }
     if (host_overlap && o.workspace_limit > 0 && (long long)pl.ws_bytes > o.workspace_limit) {
         extras = false;  // the overlapped top step without its extra buffers

@@ -74,7 +74,8 @@ typedef struct caps_options {
     int slices;                /* split form: digits per operand, 0 = automatic, 1..8 */
     int diagonals;             /* split form: digit-pair diagonals kept, 0 = automatic */
     int split_scheme;          /* split form: caps_split_scheme */
-    long long workspace_limit; /* bytes of device workspace allowed (-m); <= 0: no limit */
+    long long workspace_limit; /* bytes of device workspace allowed (-m); <= 0: no limit (then
+                                  small 'd' steps may run as 'b': caps_workspace_size) */
     int plain_tile;            /* plain form: the DMMA base case's CTA tile, caps_plain_tile */
     int operand_bits;          /* split form, residue scheme: cap on the operand bits, 0 = 55
                                   (the data's own need when lower); fewer bits take fewer moduli
@@ -109,7 +110,9 @@ void caps_options_init(caps_options *opt);
  * multiply.h:13, multiply.cpp:9-25, with device pointers and a stream).
  * pattern: one char per level ('b'/'B' = the 7 subproducts run concurrently
  * in one launch, 'd'/'D' = in sequence, 'h'/'H' = 'd' on one GPU), or NULL
- * to let the library choose.  Asynchronous on `stream`. */
+ * to let the library choose.  Where opt sets no workspace limit, small 'd'
+ * steps may run as 'b' steps (the same bits; caps_workspace_size has what
+ * that takes).  Asynchronous on `stream`. */
 caps_status caps_multiply_dev(const double *A, const double *B, double *C, caps_desc desc,
                               const char *pattern, const caps_options *opt, void *stream);
 
@@ -170,7 +173,14 @@ caps_status caps_chol_mult_dev(double *C, const double *A, const double *B, int 
 caps_status caps_chol_mult_host(double *C, const double *A, const double *B, int n, int x, int r,
                                 double alpha, const char *pattern, const caps_options *opt);
 
-/* Workspace bytes caps_multiply_dev needs for (desc, pattern, opt). */
+/* Workspace bytes caps_multiply_dev needs for (desc, pattern, opt), every step
+ * as the pattern has it: the least opt.workspace_limit the call runs with.
+ * Without a limit a call may take more: small 'd' steps then run as 'b' steps,
+ * the same bits in fewer launches (an n = 4096 'dd' multiply in the split form
+ * 4.7 GB for 0.4), as far as that adds no more than a sixteenth of the free
+ * device memory.  The workspace is kept until caps_release_cache();
+ * caps_counters.workspace_peak_bytes is what the last call used.  To keep a
+ * 'd' pattern to this size, pass the size as workspace_limit. */
 caps_status caps_workspace_size(caps_desc desc, const char *pattern, const caps_options *opt,
                                 long long *bytes);
 
