@@ -181,14 +181,14 @@ def _check(status: int) -> None:
 SPLIT_SCHEMES = {"auto": 0, "digits": 1, "residues": 2}
 
 
-PLAIN_TILES = {"64x64": 0, "32x32": 1, "128x64": 2}
+PLAIN_TILES = {"default": 0, "32x32": 1, "128x64": 2, "64x64": 4}
 
 
 def options(form: int | str = CAPS_FORM_PLAIN, slices: int = 0, diagonals: int = 0,
             workspace_limit: int = 0, scheme: int | str = 0, tile: int | str = 0,
             operand_bits: int = 0) -> Options:
-    """caps_options.  tile: the plain form's DMMA tile ("64x64", "32x32",
-    "128x64"); operand_bits: the residue scheme's operand-bit cap (0 = 55; -1:
+    """caps_options.  tile: the plain form's DMMA tile ("default": 64, 32 or 16
+    on a side, picked per launch; or "64x64", "32x32", "128x64"); operand_bits: the residue scheme's operand-bit cap (0 = 55; -1:
     chosen by the library per leaf size under its accuracy gate)."""
     if isinstance(form, str):
         form = {"plain": CAPS_FORM_PLAIN, "split": CAPS_FORM_SPLIT}[form]
@@ -339,7 +339,8 @@ def multiply_batched(As, Bs, Cs, ns, form: int | str = CAPS_FORM_PLAIN, slices: 
 def autotune_table() -> list:
     """The autotuner's choices so far (caps_autotune_info): dicts of n, form,
     nrec, pattern, the split scheme chosen ("residues" / "digits"; None for
-    the plain form), the base-case tile, the residues' operand bits and
+    the plain form), the base-case tile ([64, 64] in the plain form: the
+    default, picked per launch), the residues' operand bits and
     moduli (0 otherwise), the bit caps the accuracy gate turned down, whether
     the entry came from the on-disk cache, and seconds per instance."""
     out = []

@@ -149,16 +149,23 @@ struct DmmaTask {
     int pad;
 };
 
-// FP64 DMMA GEMM (mma.sync f64): C = A * B for every task, in CTA tiles of
-// one of three shapes (an autotuner axis).
-enum DmmaTile { DMMA_TILE_64x64 = 0, DMMA_TILE_32x32 = 1, DMMA_TILE_128x64 = 2, DMMA_TILES = 3 };
+// FP64 DMMA GEMM (mma.sync f64): C = A * B for every task, in CTA tiles picked
+// per launch or of one shape (caps_plain_tile; the autotuner tries the first
+// three, and no choice on disk has another).
+enum DmmaTile {
+    DMMA_TILE_PICK = 0,
+    DMMA_TILE_32x32 = 1,
+    DMMA_TILE_128x64 = 2,
+    DMMA_TUNED_TILES = 3,
+    DMMA_TILE_64x64 = 4
+};
 void dmma_tile_shape(int tile, int *rows, int *cols);
 cudaError_t launch_dmma_gemm(const DmmaTask *tasks_dev, int count, int m, cudaStream_t stream,
-                             int tile = DMMA_TILE_64x64);
+                             int tile = DMMA_TILE_PICK);
 // The same for rectangular leaves: A m x k, B k x n, C m x n (column-major,
 // leading dimensions m, k, m).
 cudaError_t launch_dmma_rect(const DmmaTask *tasks_dev, int count, int m, int n, int k, cudaStream_t stream,
-                             int tile = DMMA_TILE_64x64);
+                             int tile = DMMA_TILE_PICK);
 
 // Split form.  Two schemes share one launch sequence (scan, slice, GEMM); the
 // leaf size and the options choose the scheme, and the data the digits or

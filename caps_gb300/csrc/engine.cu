@@ -732,7 +732,8 @@ static caps_status check_opts(const caps_options &o) {
     if (o.slices < 0 || o.slices > 8) return CAPS_ERR_ARG;
     if (o.diagonals < 0 || o.diagonals > 8) return CAPS_ERR_ARG;
     if (o.split_scheme < CAPS_SPLIT_AUTO || o.split_scheme > CAPS_SPLIT_RESIDUES) return CAPS_ERR_ARG;
-    if (o.plain_tile < CAPS_TILE_64x64 || o.plain_tile > CAPS_TILE_128x64) return CAPS_ERR_ARG;
+    if ((o.plain_tile < CAPS_TILE_DEFAULT || o.plain_tile > CAPS_TILE_128x64) && o.plain_tile != CAPS_TILE_64x64)
+        return CAPS_ERR_ARG;
     if (o.operand_bits < CAPS_OPERAND_BITS_TUNED || o.operand_bits > 55) return CAPS_ERR_ARG;
     return CAPS_OK;
 }
@@ -1364,7 +1365,7 @@ static caps_status run_plan_direct(BatchPlan &p, cudaStream_t s) {
 //   1. recursion depth 0..3 (as the leaves allow) and the b/d pattern of the
 //      top step; for the split form with the scheme left to the library, also
 //      the operand cut (residues where the leaves fit them, digits);
-//   2. plain form: the DMMA CTA tile (64 x 64, 32 x 32, 128 x 64);
+//   2. plain form: the DMMA CTA tile (picked per launch, 32 x 32, 128 x 64);
 //   3. split form, where the residues won: the operand-bit cap, 55 / 52 / 48
 //      bits (17 / 16 / 15 moduli at K <= 2048: fewer modular products and
 //      residue planes).  A smaller cap is kept only if it is faster and, on
@@ -1422,7 +1423,7 @@ static bool parse_tune_line(const char *line, const std::string &dev, int n, con
                &nrec, pat, &chosen, &tile, &bits, &rejected, &sec) != 13)
         return false;
     if (strcmp(ver, kTuneVersion) || dev != dk || fn != n || fform != o.form || fslices != o.slices ||
-        fscheme != o.split_scheme || nrec < 0 || nrec > 3 || tile < 0 || tile >= DMMA_TILES || bits < 0 ||
+        fscheme != o.split_scheme || nrec < 0 || nrec > 3 || tile < 0 || tile >= DMMA_TUNED_TILES || bits < 0 ||
         bits > 55 || chosen < CAPS_SPLIT_AUTO || chosen > CAPS_SPLIT_RESIDUES)
         return false;
     // the tuner writes nrec steps of 'b' or 'd' ("-" for none); anything
@@ -1559,16 +1560,16 @@ struct Tuning {
         oref.slices = oref.diagonals = 0;
         oref.split_scheme = CAPS_SPLIT_AUTO;
         oplain.form = CAPS_FORM_PLAIN;
-        ClassCfg cref{n, 0, {0}, CAPS_SPLIT_AUTO, DMMA_TILE_64x64, 0};
+        ClassCfg cref{n, 0, {0}, CAPS_SPLIT_AUTO, DMMA_TILE_PICK, 0};
         ClassCfg cplain = base;
         cplain.scheme = 0;
         cplain.bits = 0;
-        cplain.tile = DMMA_TILE_64x64;
+        cplain.tile = DMMA_TILE_PICK;
         ClassCfg cand = base;
         cand.bits = bits;
         ok = true;
         caps_status st = CAPS_OK;
-        ClassCfg cabs{n, 0, {0}, 0, DMMA_TILE_64x64, 0};
+        ClassCfg cabs{n, 0, {0}, 0, DMMA_TILE_PICK, 0};
         for (int wide = 0; wide < 2 && ok && st == CAPS_OK; wide++) {
             fill(wide);
             // |A||B| of every instance, the scale of each entry's error
@@ -1629,7 +1630,7 @@ static caps_status tune_size(int n, const caps_options &o_in, ClassCfg &out, boo
     }
     CAPS_CUDA_TRY(cudaEventCreate(&tu.e0));
     CAPS_CUDA_TRY(cudaEventCreate(&tu.e1));
-    ClassCfg best{n, 0, {0}, o.split_scheme, DMMA_TILE_64x64, 0};
+    ClassCfg best{n, 0, {0}, o.split_scheme, DMMA_TILE_PICK, 0};
     double best_t = 1e30;
     caps_status st = CAPS_OK;
     // axis 1: depth, pattern and (split form, scheme left to the library)
@@ -1642,7 +1643,7 @@ static caps_status tune_size(int n, const caps_options &o_in, ClassCfg &out, boo
             const int scheme = both ? (sc == 0 ? CAPS_SPLIT_RESIDUES : CAPS_SPLIT_DIGITS) : o.split_scheme;
             if (both && scheme == CAPS_SPLIT_RESIDUES && (leaf + 15) / 16 * 16 > RESIDUE_KMAX) continue;
             for (int variant = 0; variant < (r >= 2 ? 2 : 1) && st == CAPS_OK; variant++) {
-                ClassCfg c{n, r, {0}, scheme, DMMA_TILE_64x64, 0};
+                ClassCfg c{n, r, {0}, scheme, DMMA_TILE_PICK, 0};
                 for (int k = 0; k < r; k++) c.pat[k] = (variant == 1 && k == 0) ? 'd' : 'b';
                 double t = 1e30;
                 st = tu.run(c, o, &t);

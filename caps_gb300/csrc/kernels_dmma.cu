@@ -188,6 +188,7 @@ static int pick_tile(int count, int m, int n) {
     return best;
 }
 
+// a tuned tile's shape; 64 x 64, the largest it takes, for the pick per launch
 void dmma_tile_shape(int tile, int *rows, int *cols) {
     switch (tile) {
         case DMMA_TILE_32x32: *rows = 32; *cols = 32; break;
@@ -202,6 +203,7 @@ cudaError_t launch_dmma_rect(const DmmaTask *tasks_dev, int count, int m, int n,
     switch (tile) {
         case DMMA_TILE_32x32: return launch_dmma_shape<2, 2, 2, 2>(tasks_dev, count, m, n, k, stream);
         case DMMA_TILE_128x64: return launch_dmma_shape<4, 2, 4, 4>(tasks_dev, count, m, n, k, stream);
+        case DMMA_TILE_64x64: return launch_dmma_shape<2, 2, 4, 4>(tasks_dev, count, m, n, k, stream);
     }
     switch (pick_tile(count, m, n)) {
         case 16: return launch_dmma_shape<2, 2, 1, 1>(tasks_dev, count, m, n, k, stream);

@@ -95,12 +95,13 @@ typedef struct caps_options {
  * such call for a leaf size outside any stream capture. */
 #define CAPS_OPERAND_BITS_TUNED (-1)
 
-/* CTA tiles of the plain form's DMMA base case. */
+/* CTA tiles of the plain form's DMMA base case; all give the same bits. */
 typedef enum caps_plain_tile {
-    CAPS_TILE_64x64 = 0,   /* default: 64 x 64, or 32 x 32 or 16 x 16 for launches whose 64 x 64
-                              tiles spread unevenly over the SMs (the same bits) */
-    CAPS_TILE_32x32 = 1,   /* four warps of 16 x 16: four times the CTAs */
-    CAPS_TILE_128x64 = 2   /* eight warps: half the B traffic per multiply-add */
+    CAPS_TILE_DEFAULT = 0, /* per launch, 64 x 64, 32 x 32 or 16 x 16: the one whose tiles spread
+                              most evenly over the SMs */
+    CAPS_TILE_32x32 = 1,   /* four warps of 16 x 16 */
+    CAPS_TILE_128x64 = 2,  /* eight warps of 32 x 32: half the B traffic per multiply-add */
+    CAPS_TILE_64x64 = 4    /* four warps of 32 x 32 */
 } caps_plain_tile;
 
 /* Fills *opt with defaults (plain form, automatic slices, no limit). */
@@ -282,8 +283,9 @@ typedef struct {
     int nrec;           /* Strassen levels */
     char pattern[8];    /* b/d per level, NUL-terminated */
     int scheme;         /* split form: the scheme chosen (caps_split_scheme); plain form: 0 */
-    int tile_rows;      /* CTA tile of the base-case GEMM: plain form 64 x 64, 32 x 32 or */
-    int tile_cols;      /*   128 x 64 (searched); residues 128 x 256, digits 128 x 64 (fixed) */
+    int tile_rows;      /* CTA tile of the base-case GEMM: plain form 32 x 32 or 128 x 64 where */
+    int tile_cols;      /*   that tile won, 64 x 64 where CAPS_TILE_DEFAULT did (which picks 64, 32
+                             or 16 on a side per launch); residues 128 x 256, digits 128 x 64 (fixed) */
     int operand_bits;   /* residues: operand bits per entry (55, or a smaller cap that won); else 0 */
     int moduli;         /* residues: moduli per leaf product for float data at that cap; else 0 */
     int gate_rejected;  /* residues: smaller bit caps that ran faster but failed the accuracy gate */
@@ -298,7 +300,7 @@ typedef struct {
  *   1. recursion depth (0..3 as the leaves allow) and the top step's b/d
  *      pattern, and for the split form with an automatic scheme, residues
  *      against digits;
- *   2. plain form: the DMMA tile;
+ *   2. plain form: the DMMA tile (picked per launch, 32 x 32 or 128 x 64);
  *   3. split form where the residues won: operand bits 55 / 52 / 48 (17 / 16 /
  *      15 moduli at K <= 2048), a smaller cap kept only if it is faster and
  *      its error against a split reference is no larger than the plain FP64
