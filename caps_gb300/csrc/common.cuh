@@ -70,28 +70,26 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 enum EwOp : int {
     // forms T3,T4,T5,T6 from A and S3,S4,S5,S7 from B (8 outputs)
     EW_FORM_ST = 0,
-    // dst0 = src0 (copy)
-    EW_COPY = 1,
     // dst0 = src0 + src1
-    EW_ADD = 2,
+    EW_ADD = 1,
     // dst0 = src0 - src1
-    EW_SUB = 3,
+    EW_SUB = 2,
     // dst0 = src0 + src2 ; dst1 = src1 + src2   (C22 = U2+Q3 ; U3 = U3+Q3)
-    EW_ADD2 = 4,
+    EW_ADD2 = 3,
     // calcCij: C11..C22 from Q1..Q7 (7 inputs, 4 outputs)
-    EW_CALC_CIJ = 5,
+    EW_CALC_CIJ = 4,
     // operand pairs of the memory-lean 'd' step, formed just before their
     // subproduct; src = A11 A21 A12 A22 B11 B21 B12 B22
-    EW_FORM_T4S4 = 6,  // dst0 = (A21+A22)-A11, dst1 = B22-(B12-B11)
-    EW_FORM_T5S5 = 7,  // dst0 = A11-A21,       dst1 = B22-B12
-    EW_FORM_T3S3 = 8,  // dst0 = A21+A22,       dst1 = B12-B11
-    EW_FORM_S7 = 9,    // dst0 = (B22-(B12-B11))-B21
-    EW_FORM_T6 = 10,   // dst0 = A12-((A21+A22)-A11)
+    EW_FORM_T4S4 = 5,  // dst0 = (A21+A22)-A11, dst1 = B22-(B12-B11)
+    EW_FORM_T5S5 = 6,  // dst0 = A11-A21,       dst1 = B22-B12
+    EW_FORM_T3S3 = 7,  // dst0 = A21+A22,       dst1 = B12-B11
+    EW_FORM_S7 = 8,    // dst0 = (B22-(B12-B11))-B21
+    EW_FORM_T6 = 9,    // dst0 = A12-((A21+A22)-A11)
     // the operand sums of a 'd' step in two passes, the second from T4 and S4
     // and in place: src = A11 A21 A22 B11 B12 B22, dst = T3 S3 T4 S4 T5 S5;
     // then src = T4 A12 S4 B21, dst0 = T6 = A12-T4, dst1 = S7 = S4-B21
-    EW_FORM_T345 = 11,
-    EW_FORM_T6S7 = 12,
+    EW_FORM_T345 = 10,
+    EW_FORM_T6S7 = 11,
 };
 
 struct EwTask {

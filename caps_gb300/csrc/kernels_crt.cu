@@ -62,21 +62,20 @@ constexpr int NTRIPLE = (LMAX + 2) / 3;
 
 struct CrtTables {
     // the slicer's constants, each in both lanes of a float2 for the packed
-    // fp32 pair instructions: -p_l, 1/p_l, c and cy below
-    float2 np2[LMAX], invp2[LMAX];
-    float2 c2[LMAX][3];
-    float2 cy2[LMAX][LMAX][4];
-    float p[LMAX], invp[LMAX];
-    float c[LMAX][3];              // balanced 2^(14k) mod p_l, k = 1..3
-    float cy[LMAX][LMAX][4];       // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
+    // fp32 pair instructions
+    float2 np2[LMAX], invp2[LMAX]; // -p_l, 1/p_l
+    float2 c2[LMAX][3];            // balanced 2^(14k) mod p_l, k = 1..3
+    float2 cy2[LMAX][LMAX][4];     // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
                                    // y_l = (M_L / p_l)^-1 mod p_l
-    // reconstruction (crt_reconstruct4), per modulus count L; triple t is the
-    // moduli 3t..3t+2 among the first L, P_t their product
+    // reconstruction (crt_reconstruct), per modulus count L; triple t is the
+    // moduli 3t..3t+2 among the first L, P_t their product.  Limbs, least
+    // significant first, are read as one 16-byte constant (n = 6144 update at an
+    // offset of 12: 0.5 % slower)
+    alignas(16) uint32_t Mt[LMAX][NTRIPLE][4];  // [L-1][t]: limbs of M_L / P_t
+    alignas(16) uint32_t M[LMAX][4];            // [L-1]: limbs of M_L
+    alignas(16) uint32_t Mn[LMAX][4];           // [L-1]: limbs of 2^(32 W) - M_L, W = crt_words(L)
+    alignas(16) uint32_t Z0[LMAX][4];           // [L-1]: limbs of -ZOFF sum_l M_L / p_l modulo M_L
     uint32_t pc[LMAX][LMAX];       // [L-1][l]: P_t / p_l, t = l / 3
-    uint32_t Mt[LMAX][NTRIPLE][4]; // [L-1][t]: limbs of M_L / P_t, least significant first
-    uint32_t M[LMAX][4];           // [L-1]: limbs of M_L
-    uint32_t Mn[LMAX][4];          // [L-1]: limbs of 2^(32 W) - M_L, W = crt_words(L)
-    uint32_t Z0[LMAX][4];          // [L-1]: limbs of -ZOFF sum_l M_L / p_l modulo M_L
     float m_inv[LMAX];             // [L-1]: 2^(32 (W - 2)) / M_L
 };
 
@@ -128,17 +127,14 @@ int mod_inverse(int a, int p) {
 void build_tables(CrtTables &t) {
     for (int l = 0; l < LMAX; l++) {
         const int p = modulus(l);
-        t.p[l] = (float)p;
-        t.invp[l] = 1.0f / (float)p;
         long long v = 1;
         for (int k = 1; k <= 3; k++) {
             v = (v * 16384) % p;
             long long b = v > p / 2 ? v - p : v;
-            t.c[l][k - 1] = (float)b;
             t.c2[l][k - 1] = make_float2((float)b, (float)b);
         }
         t.np2[l] = make_float2(-(float)p, -(float)p);
-        t.invp2[l] = make_float2(t.invp[l], t.invp[l]);
+        t.invp2[l] = make_float2(1.0f / (float)p, 1.0f / (float)p);
     }
     for (int L = 1; L <= LMAX; L++) {
         u128 M = 1;
@@ -161,18 +157,15 @@ void build_tables(CrtTables &t) {
         for (int l = 0; l < LMAX; l++) {
             if (l >= L) {
                 t.pc[L - 1][l] = 0;
-                for (int k = 0; k < 4; k++) {
-                    t.cy[L - 1][l][k] = 0;
-                    t.cy2[L - 1][l][k] = make_float2(0.f, 0.f);
-                }
+                for (int k = 0; k < 4; k++) t.cy2[L - 1][l][k] = make_float2(0.f, 0.f);
                 continue;
             }
             const u128 Ml = M / (u128)modulus(l);
             const int p = modulus(l), y = mod_inverse((int)(Ml % (u128)p), p);
             long long v = y;
             for (int k = 0; k < 4; k++) {
-                t.cy[L - 1][l][k] = (float)(v > p / 2 ? v - p : v);
-                t.cy2[L - 1][l][k] = make_float2(t.cy[L - 1][l][k], t.cy[L - 1][l][k]);
+                const float b = (float)(v > p / 2 ? v - p : v);
+                t.cy2[L - 1][l][k] = make_float2(b, b);
                 v = (v * 16384) % p;
             }
         }

@@ -134,8 +134,6 @@ __device__ __forceinline__ void ew_pair(const EwTask &t, int64_t i, bool two) {
         calc_cij(q1, c1);
 #pragma unroll
         for (int k = 0; k < 4; k++) st2<VEC>(t.dst[k], i, two, make_double2(c0[k], c1[k]));
-    } else if (OP == EW_COPY) {
-        st2<VEC>(t.dst[0], i, two, ld2<VEC>(t.src[0], i, two));
     } else if (OP == EW_ADD) {
         double2 a = ld2<VEC>(t.src[0], i, two), b = ld2<VEC>(t.src[1], i, two);
         st2<VEC>(t.dst[0], i, two, make_double2(a.x + b.x, a.y + b.y));
@@ -196,7 +194,6 @@ static int ew_nsrc(int op) {
         case EW_FORM_T6: return 8;
         case EW_FORM_T345: return 6;
         case EW_FORM_T6S7: return 4;
-        case EW_COPY: return 1;
         case EW_ADD: case EW_SUB: return 2;
         case EW_ADD2: return 3;
         case EW_CALC_CIJ: return 7;
@@ -243,7 +240,6 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
         const EwTask *t = tasks + base;
         switch (op) {
             case EW_FORM_ST: launch_op<EW_FORM_ST>(vec, t, c, q, stream); break;
-            case EW_COPY: launch_op<EW_COPY>(vec, t, c, q, stream); break;
             case EW_ADD: launch_op<EW_ADD>(vec, t, c, q, stream); break;
             case EW_SUB: launch_op<EW_SUB>(vec, t, c, q, stream); break;
             case EW_ADD2: launch_op<EW_ADD2>(vec, t, c, q, stream); break;
