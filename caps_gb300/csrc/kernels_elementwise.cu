@@ -290,7 +290,9 @@ cudaError_t launch_elementwise(int op, const EwTask *tasks, int count, int64_t q
 // there, and with the shorter ones in kernels of their own (46 registers; the
 // batched loops' 80 leave half the warps to hide the divisions).  ms one way
 // at n = 46592 (copy rate: 5.0), by elements beside the batched loops -> here:
-// bs 64 20.1 -> 7.9, 128 20.1 -> 6.5, 32 20.1 -> 14.7 (elements: 14.8).
+// bs 64 20.1 -> 7.1, 128 20.1 -> 5.9, 32 20.1 -> 13.5 (elements: 14.1).  Which path
+// runs is a comparison of bs, not a flag: with one, 49 leaves of 98 in 7 x 7
+// blocks took 9.6 us instead of 7.8.
 // ---------------------------------------------------------------------------
 constexpr int RUN_MIN = 160;  // runs from here on take a warp each
 constexpr int RUN_MIN_LARGE = 32;  // the same from n^2 = 2^31 on
@@ -318,7 +320,6 @@ struct ReorderGeom {
     int bs;             // effective block size (m when bs == 1 or bs == m)
     int nb;             // blocks per leaf side
     bool small;         // n^2 < 2^31: the divisions below
-    bool by_runs;       // a warp per run; else a thread per element or pair
     bool short_large;   // runs below RUN_MIN, n^2 >= 2^31: the kernels for 64-bit positions
     FastDiv dbs, dnb, druns;  // by bs, nb and the runs of a leaf
 };
@@ -438,7 +439,7 @@ __device__ __forceinline__ void reorder_elements64(const double *__restrict__ s,
 template <bool TO_CAPS, bool SHORT_LARGE>
 __device__ __forceinline__ void reorder(const double *__restrict__ s, double *__restrict__ d, const ReorderGeom &g) {
     const int64_t thread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
-    if (g.by_runs)
+    if (g.bs >= (SHORT_LARGE ? RUN_MIN_LARGE : RUN_MIN))
         reorder_runs<TO_CAPS, SHORT_LARGE ? 1 : 8>(s, d, g, thread >> 5, nthreads >> 5);
     else if constexpr (SHORT_LARGE)
         reorder_elements64<TO_CAPS>(s, d, g, thread, nthreads);
@@ -465,7 +466,6 @@ static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
     g.bs = (bs == 1 || bs == g.m) ? (int)g.m : (int)bs;
     g.nb = (int)(g.m / g.bs);
     g.small = n * n < ((int64_t)1 << 31);
-    g.by_runs = g.bs >= (g.small ? RUN_MIN : RUN_MIN_LARGE);
     g.short_large = !g.small && g.bs < RUN_MIN;
     g.dbs = fast_div(g.bs);
     g.dnb = fast_div(g.nb);
@@ -473,10 +473,11 @@ static ReorderGeom make_geom(int64_t n, int nrec, int64_t bs) {
     return g;
 }
 
-// grid: enough blocks for a run (or element) per thread, at most 8 blocks of
-// 256 threads per SM for all matrices together
+// grid: a warp per run, or a thread per element, in blocks of 256 threads, at
+// most 32 blocks per SM for all matrices together (then each takes several;
+// by elements a thread takes four, or four pairs, a pass)
 static unsigned reorder_blocks(const ReorderGeom &g, int count) {
-    const int64_t items = g.by_runs ? g.n * g.n / g.bs * 32 : g.n * g.n;
+    const int64_t items = g.bs >= (g.short_large ? RUN_MIN_LARGE : RUN_MIN) ? g.n * g.n / g.bs * 32 : g.n * g.n;
     int64_t blocks = (items + 255) / 256;
     int64_t cap = (int64_t)152 * 32 / count;
     if (cap < 1) cap = 1;

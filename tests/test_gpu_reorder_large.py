@@ -54,7 +54,7 @@ def test_large_reorder_is_the_layout(caps, cuda, buffers, r, bs):
 @pytest.mark.parametrize("bs", [64, 128])
 def test_large_reorder_in_blocks_is_no_chain_of_divisions(caps, cuda, buffers, bs):
     """Against the same reorder in whole leaf columns, which runs at the copy
-    rate: blocks of 64 take 1.6 times as long by runs and 4.0 times with
+    rate: blocks of 64 take 1.4 times as long by runs and 4.0 times with
     divisions for every element; the bound lies between."""
     x, y, _ = buffers
     for move in (caps.to_caps_layout, caps.from_caps_layout):
