@@ -68,14 +68,16 @@ struct CrtTables {
     float2 cy2[LMAX][LMAX][4];     // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
                                    // y_l = (M_L / p_l)^-1 mod p_l
     // reconstruction (crt_reconstruct), per modulus count L; triple t is the
-    // moduli 3t..3t+2 among the first L, P_t their product.  Limbs, least
-    // significant first, are read as one 16-byte constant (n = 6144 update at an
-    // offset of 12: 0.5 % slower)
+    // moduli 3t..3t+2 among the first L, P_t their product.  Constants
+    // are read 16 bytes at a time where they are aligned for it, so limbs (least
+    // significant first) and rows of factors are: with limbs at an offset of 12
+    // the n = 6144 update is 0.5 % slower, with factors in rows of 17 words
+    // 49 leaves of 777 at 10 moduli 1.8 %
     alignas(16) uint32_t Mt[LMAX][NTRIPLE][4];  // [L-1][t]: limbs of M_L / P_t
     alignas(16) uint32_t M[LMAX][4];            // [L-1]: limbs of M_L
     alignas(16) uint32_t Mn[LMAX][4];           // [L-1]: limbs of 2^(32 W) - M_L, W = crt_words(L)
     alignas(16) uint32_t Z0[LMAX][4];           // [L-1]: limbs of -ZOFF sum_l M_L / p_l modulo M_L
-    uint32_t pc[LMAX][LMAX];       // [L-1][l]: P_t / p_l, t = l / 3
+    alignas(16) uint32_t pc[LMAX][LMAX + 3];    // [L-1][l]: P_t / p_l, t = l / 3
     float m_inv[LMAX];             // [L-1]: 2^(32 (W - 2)) / M_L
 };
 
@@ -722,8 +724,8 @@ __device__ __forceinline__ void reconstruct_step(const Section &t, int step, con
 // units of a modulus before the next, so that the pairs still share its planes
 // (as runs of one unit's moduli, a leaf of 1792 read every tile's planes from
 // DRAM: 210 us instead of 111).  Each unit then has a residue tile per CTA, and
-// crt_combine_kernel turns the tiles into C with the whole GPU; launch_crt_gemm
-// has the rule.
+// crt_combine_kernel turns the tiles into C with the whole GPU;
+// launch_crt_gemm_leaves and launch_crt_gemm have the rules.
 struct Items {
     uint32_t total, pairs, c, L, count;
     int split;
