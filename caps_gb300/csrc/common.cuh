@@ -35,11 +35,13 @@ void note_cuda_error(cudaError_t e, const char *where);
 // Count of kernels this library launched (for the bench's launch count).
 void count_launch(long long n = 1);
 
-// A launch that may be set up while the kernel before it in the stream still
-// runs (programmatic stream serialisation).  The kernel calls chain_wait()
-// before it touches memory, in every block and also where a block has nothing
-// to do: the wait ends when all earlier kernels are done and their writes
-// visible, and the kernel after it relies on that.  us a call, without ->
+// A launch whose set-up overlaps the end of the kernel before it in the stream
+// (programmatic stream serialisation; no kernel here triggers its successor,
+// so its blocks start once the predecessor's last block has exited, before
+// that kernel's completion and flush).  The kernel calls chain_wait() before it
+// touches memory, in every block and also where a block has nothing to do: the
+// wait ends when all earlier kernels are done and their writes visible, and
+// the kernel after it relies on that.  us a call, without ->
 // with: n = 392 'bd' in 7 x 7 blocks 128 -> 104, one leaf of 448 64 -> 55, n = 1792
 // 366 -> 353, n = 16384 integers 'bbdd' (288 launches) 91900 -> 91200.
 template <typename... K, typename... A>

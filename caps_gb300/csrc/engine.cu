@@ -12,12 +12,14 @@
 // the batch in one launch and recurses on a batch seven times larger (the 7
 // subproducts run concurrently), then forms C in one launch (calcCij).  A 'd'
 // level forms the operand sums once and recurses seven times on a batch of
-// the same size, folding each subproduct into C as soon as it is ready, in
-// the reference's summation order.  The leaf level runs one batched GEMM
-// launch.  Workspace comes from a stack over one device arena; the plan is
-// built twice (a dry run sizes the arena, then the real one), and all task
-// tables of a call go to the device at once (small ones as a launch's
-// arguments).
+// the same size, with the operand sums and products in the C quadrants and
+// three buffers (over plain-form leaves and under a host call's copies, folding
+// each subproduct into C as soon as it is ready), in the reference's summation
+// order; small ones run as 'b' levels where memory allows.  The leaf level
+// runs one batched GEMM launch.  Workspace comes from a stack over one device
+// arena; the plan is built twice (a dry run sizes the arena, then the real
+// one), and all task tables of a call go to the device at once (small ones as
+// a launch's arguments).
 #include "common.cuh"
 
 #include <algorithm>
@@ -364,8 +366,10 @@ static void build_leaf(Builder &b, const std::vector<Prob> &P, int64_t m) {
 // 'd' 2190 -> 1893, 'dd' 4118 -> 2587, n = 5000 'd' 6265 -> 5362, n = 6144 'd' 9853
 // -> 9301; beyond, less than 5 %: n = 8192 'bbd', 4.2 GiB, 18370 -> 17680).  With
 // the scratch of the larger launches that is up to some 8 GB.  Plain form:
-// quarters up to 154 (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48), as larger
-// leaves fill the FP64 pipe one at a time.
+// quarters up to 154 (n = 56 'dd' 471 -> 31, n = 256 'd' 129 -> 48).  That line is
+// not where merging stops to pay (a 'd' step on quarters of 160 133 -> 80, 200
+// 241 -> 137, 300 495 -> 388, 400 1039 -> 850, 500 1805 -> 1738): beyond it a 'd'
+// over plain leaves keeps its memory and its folds in the products' epilogues.
 static bool merges(const Builder &b, size_t nodes, int64_t h) {
     if (!b.merge_small || (b.opt.form == CAPS_FORM_PLAIN && h > 154)) return false;
     return (int64_t)nodes * 11 * h * h * (int64_t)sizeof(double) <= (int64_t)1 << 30;

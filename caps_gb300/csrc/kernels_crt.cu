@@ -68,11 +68,10 @@ struct CrtTables {
     float2 cy2[LMAX][LMAX][4];     // [L-1][l][k]: balanced 2^(14k) y_l mod p_l, k = 0..3,
                                    // y_l = (M_L / p_l)^-1 mod p_l
     // reconstruction (crt_reconstruct), per modulus count L; triple t is the
-    // moduli 3t..3t+2 among the first L, P_t their product.  Constants
-    // are read 16 bytes at a time where they are aligned for it, so limbs (least
-    // significant first) and rows of factors are: with limbs at an offset of 12
-    // the n = 6144 update is 0.5 % slower, with factors in rows of 17 words
-    // 49 leaves of 777 at 10 moduli 1.8 %
+    // moduli 3t..3t+2 among the first L, P_t their product.  Limbs stand least
+    // significant first.  Aligned, several constants come in one read: with
+    // limbs at an offset of 12 the n = 6144 update is 0.5 % slower, with factors
+    // in rows of 17 words 49 leaves of 777 at 10 moduli 1.8 %
     alignas(16) uint32_t Mt[LMAX][NTRIPLE][4];  // [L-1][t]: limbs of M_L / P_t
     alignas(16) uint32_t M[LMAX][4];            // [L-1]: limbs of M_L
     alignas(16) uint32_t Mn[LMAX][4];           // [L-1]: limbs of 2^(32 W) - M_L, W = crt_words(L)
