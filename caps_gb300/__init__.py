@@ -188,8 +188,9 @@ def options(form: int | str = CAPS_FORM_PLAIN, slices: int = 0, diagonals: int =
             workspace_limit: int = 0, scheme: int | str = 0, tile: int | str = 0,
             operand_bits: int = 0) -> Options:
     """caps_options.  tile: the plain form's DMMA tile ("default": 64, 32 or 16
-    on a side, picked per launch; or "64x64", "32x32", "128x64"); operand_bits: the residue scheme's operand-bit cap (0 = 55; -1:
-    chosen by the library per leaf size under its accuracy gate)."""
+    on a side, picked per launch; or "64x64", "32x32", "128x64");
+    operand_bits: the residue scheme's operand-bit cap (0 = 55; -1: chosen by
+    the library per leaf size under its accuracy gate)."""
     if isinstance(form, str):
         form = {"plain": CAPS_FORM_PLAIN, "split": CAPS_FORM_SPLIT}[form]
     if isinstance(scheme, str):

@@ -1177,8 +1177,8 @@ cudaError_t launch_crt_gemm(const LeafTask *tasks_dev, int count, int m, SplitPa
     // 1428 (1780), 16807 of 40 8480 -> 7340 (9580).  Leaves of up to 32
     // reconstruct too little for it: integers of 11 bits, 16807 of 16 2870 ->
     // 3650, of 32 3610 -> 3770, of 40 4080 -> 3870.
-    const bool thin = leaf_units(g) == 1 && m > 32 && m <= TM;
-    const int launches = thin ? (count + ZCTA_MAX - 1) / ZCTA_MAX : 1, per = (count + launches - 1) / launches;
+    const bool parts = count > ZCTA_MAX && m > 32 && m <= TM;
+    const int launches = parts ? (count + ZCTA_MAX - 1) / ZCTA_MAX : 1, per = (count + launches - 1) / launches;
     for (int first = 0; first < count; first += per) {
         Geo part = g;
         part.count = count - first < per ? count - first : per;

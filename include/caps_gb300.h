@@ -175,7 +175,7 @@ caps_status caps_chol_mult_host(double *C, const double *A, const double *B, int
                                 double alpha, const char *pattern, const caps_options *opt);
 
 /* Workspace bytes caps_multiply_dev needs for (desc, pattern, opt), every step
- * as the pattern has it: the least opt.workspace_limit the call runs with.
+ * as the pattern has it: the least opt.workspace_limit the pattern runs with.
  * Without a limit a call may take more: small 'd' steps then run as 'b' steps,
  * the same bits in fewer launches (an n = 4096 'dd' multiply in the split form
  * 4.7 GB for 0.4), as far as that adds no more than a sixteenth of the free
